@@ -22,11 +22,20 @@
 // must start at zero, and calls that overlap on the GPU (different streams,
 // or different host threads) race on it.
 //
-// The sweep structure is one launch per phase (clear, triangles, hinges,
-// vertex update) with float atomics into the accumulator, so results match
+// The frame is one cooperative launch.  Its sweeps alternate two phases with a
+// grid barrier after each: the elements (one thread per triangle or hinge)
+// add their corner forces to the accumulator, the vertices take their update
+// and clear it.  What bounds it is latency, not bytes: a 129x129 cloth moves
+// about 5 MB per sweep through L2.  The former form issued five launches per
+// sweep (control, clear, triangles, hinges, update; three scalar atomics per
+// corner).  A frame of 32 sweeps at 129x129 took 875 us in that form, 355 us
+// as one launch with one 16-byte reduction per corner, and takes 220 us with
+// what a frame does not change kept in registers and one arrival per block
+// and barrier.  The float reductions add in any order, so results match
 // pdg_solver_step to rounding, not bitwise.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <mutex>
 
@@ -43,6 +52,8 @@ constexpr int kMaxIters = PDG_NOALLOC_MAX_ITERS;
 struct NaCtl {
     int active, used, status, pad;
     double res_y2, res0_2, resf_2;
+    unsigned bar;      // grid barrier: arrivals so far (cleared before each frame)
+    int err;           // a barrier wait gave up (cleared with them)
 };
 
 constexpr size_t kOffY = 0;
@@ -71,174 +82,271 @@ Scratch carve(unsigned char* base)
     return s;
 }
 
-inline int nb(int n, int b) { return (n + b - 1) / b; }
+constexpr int kNaThreads = 512;
+constexpr long long kNaWaitCycles = 4000000000LL;   // about 2 s: bound of a barrier wait
 
-__global__ void k_na_setup(Scratch s, int nacc)
+struct NaArgs {
+    Scratch s;
+    int N, T, E, P;
+    float *pos, *vel;
+    const float *mass, *diag;
+    const int* tris;
+    const float *Dm_inv, *area, *ks;
+    const int* quads;
+    const float *w4, *nrest, *kb;
+    const int* pin_idx;
+    const float* pin_target;
+    float h, ax, ay, az, damping, gamma, tol, rho2;
+    int cap, have_final, use_cheb, cheb_delay;
+};
+
+// Barrier `phase` (1, 2, ...) of the frame over the grid: one arrival per
+// block on a count that only grows, polled until all blocks of the phase are
+// in.  False on every thread of a block once a wait, here or in another
+// block, gave up.
+__device__ __forceinline__ bool na_barrier(NaCtl* c, unsigned& phase)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < nacc) s.acc[i] = 0.0;
-    if (i == 0) {
-        NaCtl c;
-        c.active = 1; c.used = 0; c.status = 0; c.pad = 0;
-        c.res_y2 = 0.0; c.res0_2 = 0.0; c.resf_2 = -1.0;
-        *s.ctl = c;
+    __shared__ int ok;
+    __syncthreads();
+    ++phase;
+    if (threadIdx.x == 0) {
+        const unsigned want = phase * gridDim.x;
+        __threadfence();
+        atomicAdd(&c->bar, 1u);
+        unsigned v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(__cvta_generic_to_global(&c->bar)) : "memory");
+        if (v < want) {
+            const long long t0 = clock64();
+            do {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(__cvta_generic_to_global(&c->bar)) : "memory");
+                if (clock64() - t0 > kNaWaitCycles) { atomicCAS(&c->err, 0, 1); break; }
+            } while (v < want);
+        }
+        ok = v >= want;
+    }
+    __syncthreads();
+    return ok != 0;
+}
+
+__device__ __forceinline__ void na_add(float4* F, int v, float x, float y, float z)
+{
+    atomicAdd(&F[v], make_float4(x, y, z, 0.f));   // one 16-byte reduction
+}
+
+// A triangle (quad i3 < 0) or hinge with what does not change over the
+// sweeps of a frame: its corners, constants and the prediction's edge vectors.
+struct NaElem {
+    int i0, i1, i2, i3;
+    float4 c;             // Dm_inv, or the hinge's weights
+    float s, nrest;       // h^2 k area, or h^2 k and the rest norm
+    float3 e1, e2, e3;    // y_1 - y_0, y_2 - y_0, y_3 - y_0
+    float3 y0;
+};
+
+__device__ __forceinline__ float3 na_sub(float4 p, float4 q)
+{
+    return make_float3(fsub(p.x, q.x), fsub(p.y, q.y), fsub(p.z, q.z));
+}
+
+__device__ __forceinline__ NaElem na_element(const NaArgs& a, long long q)
+{
+    NaElem m;
+    const float h2 = fmul(a.h, a.h);
+    if (q < a.T) {
+        const int t = (int)q;
+        m.i0 = a.tris[3 * t]; m.i1 = a.tris[3 * t + 1]; m.i2 = a.tris[3 * t + 2]; m.i3 = -1;
+        m.c = make_float4(a.Dm_inv[4 * t], a.Dm_inv[4 * t + 1], a.Dm_inv[4 * t + 2], a.Dm_inv[4 * t + 3]);
+        m.s = h2 * (a.ks[t] * a.area[t]);
+        m.nrest = 0.f;
+    } else {
+        const int e = (int)(q - a.T);
+        m.i0 = a.quads[4 * e]; m.i1 = a.quads[4 * e + 1]; m.i2 = a.quads[4 * e + 2]; m.i3 = a.quads[4 * e + 3];
+        m.c = make_float4(a.w4[4 * e], a.w4[4 * e + 1], a.w4[4 * e + 2], a.w4[4 * e + 3]);
+        m.s = h2 * a.kb[e];
+        m.nrest = a.nrest[e];
+    }
+    const float4 y0 = __ldcg(&a.s.Y[m.i0]), y1 = __ldcg(&a.s.Y[m.i1]), y2 = __ldcg(&a.s.Y[m.i2]);
+    const float4 y3 = m.i3 >= 0 ? __ldcg(&a.s.Y[m.i3]) : y0;
+    m.e1 = na_sub(y1, y0); m.e2 = na_sub(y2, y0); m.e3 = na_sub(y3, y0);
+    m.y0 = f3(y0);
+    return m;
+}
+
+// Adds the element's corner forces at offsets D to F.
+__device__ __forceinline__ void na_apply(const NaElem& m, const float4* D, float4* F)
+{
+    const float4 d0 = __ldcg(&D[m.i0]), d1 = __ldcg(&D[m.i1]), d2 = __ldcg(&D[m.i2]);
+    const float4 d3 = m.i3 >= 0 ? __ldcg(&D[m.i3]) : d0;
+    const float3 e1 = fadd3(m.e1, na_sub(d1, d0)), e2 = fadd3(m.e2, na_sub(d2, d0));
+    if (m.i3 < 0) {
+        float3 c0, c1, c2;
+        tri_force<kModeConsistent>(e1, e2, m.c, m.s, c0, c1, c2);
+        na_add(F, m.i0, c0.x, c0.y, c0.z);
+        na_add(F, m.i1, c1.x, c1.y, c1.z);
+        na_add(F, m.i2, c2.x, c2.y, c2.z);
+    } else {
+        const float3 e3 = fadd3(m.e3, na_sub(d3, d0));
+        const float3 x0 = make_float3(fadd(m.y0.x, d0.x), fadd(m.y0.y, d0.y), fadd(m.y0.z, d0.z));
+        const float3 f = hinge_force<kModeConsistent>(e1, e2, e3, x0, m.c, m.s, m.nrest);
+        na_add(F, m.i0, fmul(f.x, m.c.x), fmul(f.y, m.c.x), fmul(f.z, m.c.x));
+        na_add(F, m.i1, fmul(f.x, m.c.y), fmul(f.y, m.c.y), fmul(f.z, m.c.y));
+        na_add(F, m.i2, fmul(f.x, m.c.z), fmul(f.y, m.c.z), fmul(f.z, m.c.z));
+        na_add(F, m.i3, fmul(f.x, m.c.w), fmul(f.y, m.c.w), fmul(f.z, m.c.w));
     }
 }
 
-__global__ void k_na_predict(Scratch s, int N, const float* __restrict__ pos, const float* __restrict__ vel,
-                             const float* __restrict__ mass, const float* __restrict__ diag, float h, float ax,
-                             float ay, float az)
+// Two 512-thread blocks per SM at 64 registers: a 129x129 cloth's 80,000
+// elements are then one per thread on all 152 SMs.
+// ONE: no thread has more than one element; its element's constants and rest
+// of the prediction then stay in registers for the frame, so that a sweep's
+// only loads are the offsets of its corners (one trip to L2).  Likewise each
+// thread keeps its first vertex's mass, prediction and last two offsets.
+template <bool ONE>
+__global__ void __launch_bounds__(kNaThreads, 2) k_na_frame(NaArgs a)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N) return;
-    const float h2 = fmul(h, h);
-    float4 y;
-    y.x = ffma(h2, ax, ffma(h, vel[3 * i], pos[3 * i]));
-    y.y = ffma(h2, ay, ffma(h, vel[3 * i + 1], pos[3 * i + 1]));
-    y.z = ffma(h2, az, ffma(h, vel[3 * i + 2], pos[3 * i + 2]));
-    y.w = mass[i];
-    s.Y[i] = y;
-    const float dg = diag[i];
-    const float4 d0 = make_float4(0.f, 0.f, 0.f, dg > 1e-10f ? 1.0f / dg : 0.f);   // inertial start
-    s.A[i] = d0;
-    s.B[i] = d0;
-}
+    __shared__ float red[kNaThreads / 32];
+    __shared__ int done_s;
+    const Scratch s = a.s;
+    NaCtl* ctl = s.ctl;
+    const int gtid = blockIdx.x * kNaThreads + threadIdx.x, gstride = gridDim.x * kNaThreads;
+    const float h = a.h, h2 = fmul(h, h);
+    const int nsweep = a.cap + a.have_final;
+    unsigned phase = 0;
 
-__global__ void k_na_pins(Scratch s, int P, const int* __restrict__ idx, const float* __restrict__ target)
-{
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= P) return;
-    const int i = idx[q];
-    const float4 y = s.Y[i];
-    const float4 d = make_float4(fsub(target[3 * q], y.x), fsub(target[3 * q + 1], y.y), fsub(target[3 * q + 2], y.z), -1.f);
-    s.A[i] = d;
-    s.B[i] = d;
-}
+    // prediction, start offsets, cleared sums
+    for (int i = gtid; i < a.cap + 2; i += gstride) s.acc[i] = 0.0;
+    for (int i = gtid; i < a.N; i += gstride) {
+        float4 y;
+        y.x = ffma(h2, a.ax, ffma(h, a.vel[3 * i], a.pos[3 * i]));
+        y.y = ffma(h2, a.ay, ffma(h, a.vel[3 * i + 1], a.pos[3 * i + 1]));
+        y.z = ffma(h2, a.az, ffma(h, a.vel[3 * i + 2], a.pos[3 * i + 2]));
+        y.w = a.mass[i];
+        s.Y[i] = y;
+        const float dg = a.diag[i];
+        const float4 d0 = make_float4(0.f, 0.f, 0.f, dg > 1e-10f ? 1.0f / dg : 0.f);   // inertial start
+        s.A[i] = d0;
+        s.B[i] = d0;
+        s.F[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    if (!na_barrier(ctl, phase)) return;
+    if (a.P > 0) {
+        for (int q = gtid; q < a.P; q += gstride) {
+            const int i = a.pin_idx[q];
+            const float4 y = __ldcg(&s.Y[i]);
+            const float4 d = make_float4(fsub(a.pin_target[3 * q], y.x), fsub(a.pin_target[3 * q + 1], y.y),
+                                         fsub(a.pin_target[3 * q + 2], y.z), -1.f);
+            s.A[i] = d;
+            s.B[i] = d;
+        }
+        if (!na_barrier(ctl, phase)) return;
+    }
 
-// Decision at the start of sweep k (same rules as the solver's per-cloth
-// decision): converged, failed or capped frames become inactive.
-__global__ void k_na_control(Scratch s, int k, int cap, float tol, int have_final)
-{
-    NaCtl& c = *s.ctl;
-    if (!c.active) return;
-    if (k >= 1) {
-        const double acc0 = s.acc[0], rk2 = s.acc[k - 1];
-        if (k == 1) { c.res0_2 = acc0; c.res_y2 = acc0; }
-        if (!isfinite(rk2)) { c.status = -6; c.used = k - 1; c.resf_2 = rk2; c.active = 0; return; }
-        if (tol > 0.f && rk2 <= (double)tol * (double)tol * c.res_y2) {
-            c.used = k - 1; c.resf_2 = rk2; c.active = 0; return;
+    NaElem el;
+    if (ONE && gtid < a.T + a.E) el = na_element(a, gtid);
+    float4 vd = make_float4(0.f, 0.f, 0.f, 0.f), vp = vd, vy = vd;   // vertex gtid: d^k, d^(k-1), y
+    if (gtid < a.N) { vd = __ldcg(&s.A[gtid]); vp = vd; vy = __ldcg(&s.Y[gtid]); }
+
+    bool active = true;
+    float om = 1.f;
+    for (int k = 0; k < nsweep; ++k) {
+        const bool res_only = k >= a.cap;
+        if (!res_only) {   // Chebyshev weight of sweep k (the solver's recurrence)
+            if (!a.use_cheb || k < a.cheb_delay) om = 1.f;
+            else if (k == a.cheb_delay) om = fdiv(2.f, fsub(2.f, a.rho2));
+            else om = fdiv(4.f, fsub(4.f, fmul(a.rho2, om)));
+        }
+        // the decision at the start of sweep k, the same in every block:
+        // converged or failed frames end here
+        if (k >= 1) {
+            if (threadIdx.x == 0) {
+                const double acc0 = __ldcg(&s.acc[0]), rk2 = __ldcg(&s.acc[k - 1]);
+                const bool bad = !isfinite(rk2);
+                const bool conv = a.tol > 0.f && rk2 <= (double)a.tol * (double)a.tol * acc0;
+                done_s = bad || conv;
+                if (blockIdx.x == 0) {
+                    if (k == 1) { ctl->res0_2 = acc0; ctl->res_y2 = acc0; }
+                    if (done_s) { ctl->status = bad ? -6 : 0; ctl->used = k - 1; ctl->resf_2 = rk2; ctl->active = 0; }
+                }
+            }
+            __syncthreads();
+            if (done_s) { active = false; break; }
+        }
+        const float4* D = (k & 1) ? s.B : s.A;
+        float4* Dn = (k & 1) ? s.A : s.B;
+        // elements
+        if (ONE) {
+            if (gtid < a.T + a.E) na_apply(el, D, s.F);
+        } else {
+            for (long long q = gtid; q < (long long)a.T + a.E; q += gstride) na_apply(na_element(a, q), D, s.F);
+        }
+        if (!na_barrier(ctl, phase)) return;
+        // vertices; the accumulator is left clear for the next sweep
+        float r2 = 0.f;
+        for (int i = gtid; i < a.N; i += gstride) {
+            const bool first = i == gtid;
+            const float4 f4 = __ldcg(&s.F[i]);
+            const float4 d = first ? vd : __ldcg(&D[i]), y = first ? vy : __ldcg(&s.Y[i]);
+            const float4 dp = res_only ? d : (first ? vp : __ldcg(&Dn[i]));
+            float rv;
+            const float4 o = update_consistent(d, y, make_float3(f4.x, f4.y, f4.z), dp, a.gamma, res_only ? 1.f : om, rv);
+            r2 += rv;
+            if (!res_only) Dn[i] = o;
+            s.F[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (first && !res_only) { vp = d; vd = o; }
+        }
+        block_residual<kNaThreads>(r2, red, s.acc + k);
+        if (!na_barrier(ctl, phase)) return;
+    }
+
+    // the frame's record (block 0, a warp looks through the sums), known to
+    // the other blocks after one more barrier
+    if (blockIdx.x == 0 && threadIdx.x < 32) {
+        if (a.cap <= 1 && threadIdx.x == 0) { ctl->res0_2 = __ldcg(&s.acc[0]); ctl->res_y2 = __ldcg(&s.acc[0]); }
+        if (active) {
+            bool finite = true;
+            for (int k = threadIdx.x; k <= a.cap; k += 32) {
+                const double v = __ldcg(&s.acc[k]);
+                finite = finite && isfinite(v);
+            }
+            finite = __all_sync(0xffffffffu, finite) != 0;
+            if (threadIdx.x == 0) {
+                ctl->used = a.cap;
+                ctl->resf_2 = a.have_final ? __ldcg(&s.acc[a.cap]) : -1.0;
+                ctl->status = finite ? 0 : -6;
+                ctl->active = 0;
+            }
         }
     }
-    if (k >= cap && !have_final) { c.used = cap; c.resf_2 = -1.0; c.active = 0; }
-}
-
-__global__ void k_na_clear(Scratch s, int N)
-{
-    if (!s.ctl->active) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < N) s.F[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-}
-
-__device__ __forceinline__ void add3(float4* F, int v, float3 c)
-{
-    atomicAdd(&F[v].x, c.x); atomicAdd(&F[v].y, c.y); atomicAdd(&F[v].z, c.z);
-}
-
-__global__ void k_na_tri(Scratch s, int T, const int* __restrict__ tris, const float* __restrict__ Dm_inv,
-                         const float* __restrict__ area, const float* __restrict__ ks, float h2, int k)
-{
-    if (!s.ctl->active) return;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= T) return;
-    const float4* D = (k & 1) ? s.B : s.A;
-    const int i0 = tris[3 * t], i1 = tris[3 * t + 1], i2 = tris[3 * t + 2];
-    const float4 G = make_float4(Dm_inv[4 * t], Dm_inv[4 * t + 1], Dm_inv[4 * t + 2], Dm_inv[4 * t + 3]);
-    float3 c0, c1, c2;
-    tri_force<kModeConsistent>(edge(s.Y, D, i0, i1), edge(s.Y, D, i0, i2), G, h2 * (ks[t] * area[t]), c0, c1, c2);
-    add3(s.F, i0, c0); add3(s.F, i1, c1); add3(s.F, i2, c2);
-}
-
-__global__ void k_na_hinge(Scratch s, int E, const int* __restrict__ quads, const float* __restrict__ w4,
-                           const float* __restrict__ nrest, const float* __restrict__ kb, float h2, int k)
-{
-    if (!s.ctl->active) return;
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= E) return;
-    const float4* D = (k & 1) ? s.B : s.A;
-    const int i0 = quads[4 * e], i1 = quads[4 * e + 1], i2 = quads[4 * e + 2], i3 = quads[4 * e + 3];
-    const float4 w = make_float4(w4[4 * e], w4[4 * e + 1], w4[4 * e + 2], w4[4 * e + 3]);
-    const float4 y0 = s.Y[i0], d0 = D[i0];
-    const float3 x0 = make_float3(fadd(y0.x, d0.x), fadd(y0.y, d0.y), fadd(y0.z, d0.z));
-    const float3 q = hinge_force<kModeConsistent>(edge(s.Y, D, i0, i1), edge(s.Y, D, i0, i2), edge(s.Y, D, i0, i3),
-                                                  x0, w, h2 * kb[e], nrest[e]);
-    add3(s.F, i0, scale3(q, w.x)); add3(s.F, i1, scale3(q, w.y));
-    add3(s.F, i2, scale3(q, w.z)); add3(s.F, i3, scale3(q, w.w));
-}
-
-__global__ void __launch_bounds__(256) k_na_update(Scratch s, int N, int k, int res_only, float omega, float gamma)
-{
-    __shared__ float red[8];
-    if (!s.ctl->active) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const float4* Dk = (k & 1) ? s.B : s.A;
-    float4* Dn = (k & 1) ? s.A : s.B;
-    float r2 = 0.f;
-    if (i < N) {
-        const float4 d = Dk[i], y = s.Y[i], f4 = s.F[i];
-        const float4 dp = res_only ? d : Dn[i];
-        const float4 o = update_consistent(d, y, make_float3(f4.x, f4.y, f4.z), dp, gamma, omega, r2);
-        if (!res_only) Dn[i] = o;
+    if (!na_barrier(ctl, phase)) return;
+    const int status = __ldcg(&ctl->status), used = __ldcg(&ctl->used);
+    const float4* D = (used & 1) ? s.B : s.A;
+    const float sc = 1.f - a.damping, ih = fdiv(1.f, h);
+    for (int i = gtid; i < a.N; i += gstride) {
+        const float4 d = __ldcg(&D[i]);
+        if (d.w < 0.f) continue;   // pinned: written below
+        if (status != 0) {         // failed frame: keep x_n, stop the cloth
+            a.vel[3 * i] = 0.f; a.vel[3 * i + 1] = 0.f; a.vel[3 * i + 2] = 0.f;
+            continue;
+        }
+        const float4 y = __ldcg(&s.Y[i]);
+        a.vel[3 * i] = fmul(sc, ffma(d.x, ih, ffma(h, a.ax, a.vel[3 * i])));
+        a.vel[3 * i + 1] = fmul(sc, ffma(d.y, ih, ffma(h, a.ay, a.vel[3 * i + 1])));
+        a.vel[3 * i + 2] = fmul(sc, ffma(d.z, ih, ffma(h, a.az, a.vel[3 * i + 2])));
+        a.pos[3 * i] = fadd(y.x, d.x); a.pos[3 * i + 1] = fadd(y.y, d.y); a.pos[3 * i + 2] = fadd(y.z, d.z);
     }
-    block_residual<256>(r2, red, s.acc + k);
-}
-
-__global__ void k_na_end(Scratch s, int cap, int have_final)
-{
-    NaCtl& c = *s.ctl;
-    if (cap <= 1) { c.res0_2 = s.acc[0]; c.res_y2 = s.acc[0]; }
-    if (!c.active) return;
-    c.used = cap;
-    bool finite = true;
-    for (int k = 0; k <= cap; ++k) finite = finite && isfinite(s.acc[k]);
-    c.resf_2 = have_final ? s.acc[cap] : -1.0;
-    if (!finite) c.status = -6;
-    c.active = 0;
-}
-
-__global__ void k_na_finalize(Scratch s, int N, float* __restrict__ pos, float* __restrict__ vel, float h,
-                              float damping, float ax, float ay, float az)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N) return;
-    const NaCtl c = *s.ctl;
-    if (c.status != 0) {   // failed frame: keep x_n, stop the cloth
-        vel[3 * i] = 0.f; vel[3 * i + 1] = 0.f; vel[3 * i + 2] = 0.f;
-        return;
+    for (int q = gtid; q < a.P; q += gstride) {
+        const int i = a.pin_idx[q];
+        a.pos[3 * i] = a.pin_target[3 * q]; a.pos[3 * i + 1] = a.pin_target[3 * q + 1]; a.pos[3 * i + 2] = a.pin_target[3 * q + 2];
+        a.vel[3 * i] = 0.f; a.vel[3 * i + 1] = 0.f; a.vel[3 * i + 2] = 0.f;
     }
-    const float4 d = (c.used & 1) ? s.B[i] : s.A[i];
-    const float4 y = s.Y[i];
-    const float sc = 1.f - damping, ih = fdiv(1.f, h);
-    vel[3 * i] = fmul(sc, ffma(d.x, ih, ffma(h, ax, vel[3 * i])));
-    vel[3 * i + 1] = fmul(sc, ffma(d.y, ih, ffma(h, ay, vel[3 * i + 1])));
-    vel[3 * i + 2] = fmul(sc, ffma(d.z, ih, ffma(h, az, vel[3 * i + 2])));
-    pos[3 * i] = fadd(y.x, d.x); pos[3 * i + 1] = fadd(y.y, d.y); pos[3 * i + 2] = fadd(y.z, d.z);
-}
-
-__global__ void k_na_pins_final(int P, const int* __restrict__ idx, const float* __restrict__ target,
-                                float* __restrict__ pos, float* __restrict__ vel)
-{
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= P) return;
-    const int i = idx[q];
-    pos[3 * i] = target[3 * q]; pos[3 * i + 1] = target[3 * q + 1]; pos[3 * i + 2] = target[3 * q + 2];
-    vel[3 * i] = 0.f; vel[3 * i + 1] = 0.f; vel[3 * i + 2] = 0.f;
 }
 
 // Device address of the scratch array, looked up once per device.
 std::mutex g_mu;
 unsigned char* g_addr[64] = {};
+int g_blocks[64] = {};   // blocks of k_na_frame resident at once
 
-int scratch_of(int dev, unsigned char** out)
+int scratch_of(int dev, unsigned char** out, int* blocks)
 {
     if (dev < 0 || dev >= 64) return set_error(PDG_ERR_ARG, "pdg_step_noalloc: device %d out of range", dev);
     std::lock_guard<std::mutex> lock(g_mu);
@@ -247,9 +355,17 @@ int scratch_of(int dev, unsigned char** out)
         const cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
         if (e != cudaSuccess || !p)
             return set_error(PDG_ERR_CUDA, "pdg_step_noalloc: cudaGetSymbolAddress failed: %s", cudaGetErrorString(e));
+        int nsm = 0, per = 0, per2 = 0;
+        if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_na_frame<true>, kNaThreads, 0) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per2, k_na_frame<false>, kNaThreads, 0) != cudaSuccess ||
+            std::min(per, per2) <= 0)
+            return set_error(PDG_ERR_CUDA, "pdg_step_noalloc: occupancy query failed");
+        g_blocks[dev] = nsm * std::min(per, per2);
         g_addr[dev] = static_cast<unsigned char*>(p);
     }
     *out = g_addr[dev];
+    *blocks = g_blocks[dev];
     return PDG_OK;
 }
 
@@ -297,44 +413,37 @@ extern "C" int pdg_step_noalloc(const pdg_config* cfg, int N, float* d_pos, floa
                              sdev, dev);
     }
     unsigned char* base = nullptr;
-    const int rc = scratch_of(dev, &base);
+    int max_blocks = 0;
+    const int rc = scratch_of(dev, &base, &max_blocks);
     if (rc) return rc;
-    const Scratch s = carve(base);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
 
-    const int cap = cfg->max_iterations;
-    const int have_final = (cfg->compute_final_residual || cfg->tolerance > 0.f) ? 1 : 0;
-    const float h = cfg->dt, h2 = h * h;
-    const float ax = cfg->wind[0], ay = cfg->gravity + cfg->wind[1], az = cfg->wind[2];
-
-    k_na_setup<<<nb(cap + 2, 256), 256, 0, st>>>(s, cap + 2);
-    k_na_predict<<<nb(N, 256), 256, 0, st>>>(s, N, d_pos, d_vel, d_mass, d_jacobi_diag, h, ax, ay, az);
-    if (P) k_na_pins<<<nb(P, 128), 128, 0, st>>>(s, P, d_pin_idx, d_pin_target);
-    float om = 1.f;
-    const float r2 = cfg->rho * cfg->rho;
-    const int nsweep = cap + have_final;
-    for (int k = 0; k < nsweep; ++k) {
-        const bool res_only = k >= cap;
-        if (!res_only) {   // Chebyshev weight of sweep k (same recurrence as the solver)
-            if (!cfg->use_chebyshev || k < cfg->cheb_delay) om = 1.f;
-            else if (k == cfg->cheb_delay) om = 2.f / (2.f - r2);
-            else om = 4.f / (4.f - r2 * om);
-        }
-        k_na_control<<<1, 1, 0, st>>>(s, k, cap, cfg->tolerance, have_final);
-        k_na_clear<<<nb(N, 256), 256, 0, st>>>(s, N);
-        if (T) k_na_tri<<<nb(T, 256), 256, 0, st>>>(s, T, d_tris, d_Dm_inv, d_rest_area, d_stretch_k, h2, k);
-        if (E) k_na_hinge<<<nb(E, 256), 256, 0, st>>>(s, E, d_bend_quads, d_bend_w, d_bend_n, d_bend_k, h2, k);
-        k_na_update<<<nb(N, 256), 256, 0, st>>>(s, N, k, res_only ? 1 : 0, res_only ? 1.f : om, cfg->gamma);
-    }
-    k_na_end<<<1, 1, 0, st>>>(s, cap, have_final);
-    k_na_finalize<<<nb(N, 256), 256, 0, st>>>(s, N, d_pos, d_vel, h, cfg->damping, ax, ay, az);
-    if (P) k_na_pins_final<<<nb(P, 128), 128, 0, st>>>(P, d_pin_idx, d_pin_target, d_pos, d_vel);
-    NA_CK(cudaGetLastError());
+    NaArgs a{};
+    a.s = carve(base);
+    a.N = N; a.T = T; a.E = E; a.P = P;
+    a.pos = d_pos; a.vel = d_vel; a.mass = d_mass; a.diag = d_jacobi_diag;
+    a.tris = d_tris; a.Dm_inv = d_Dm_inv; a.area = d_rest_area; a.ks = d_stretch_k;
+    a.quads = d_bend_quads; a.w4 = d_bend_w; a.nrest = d_bend_n; a.kb = d_bend_k;
+    a.pin_idx = d_pin_idx; a.pin_target = d_pin_target;
+    a.h = cfg->dt; a.ax = cfg->wind[0]; a.ay = cfg->gravity + cfg->wind[1]; a.az = cfg->wind[2];
+    a.damping = cfg->damping; a.gamma = cfg->gamma; a.tol = cfg->tolerance; a.rho2 = cfg->rho * cfg->rho;
+    a.cap = cfg->max_iterations;
+    a.have_final = (cfg->compute_final_residual || cfg->tolerance > 0.f) ? 1 : 0;
+    a.use_cheb = cfg->use_chebyshev; a.cheb_delay = cfg->cheb_delay;
+    // one element per thread as far as the resident blocks go
+    const long long work = std::max((long long)T + E, (long long)N);
+    const int grid = (int)std::max(1LL, std::min((long long)max_blocks, (work + kNaThreads - 1) / kNaThreads));
+    NA_CK(cudaMemsetAsync(a.s.ctl, 0, sizeof(NaCtl), st));
+    void* args[] = {&a};
+    const void* kernel = (long long)T + E <= (long long)grid * kNaThreads ? (const void*)k_na_frame<true>
+                                                                          : (const void*)k_na_frame<false>;
+    NA_CK(cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(kNaThreads), args, 0, st));
 
     if (stats) {
         NaCtl c;
-        NA_CK(cudaMemcpyAsync(&c, s.ctl, sizeof(NaCtl), cudaMemcpyDeviceToHost, st));
+        NA_CK(cudaMemcpyAsync(&c, a.s.ctl, sizeof(NaCtl), cudaMemcpyDeviceToHost, st));
         NA_CK(cudaStreamSynchronize(st));
+        if (c.err) return set_error(PDG_ERR_TIMEOUT, "pdg_step_noalloc: bounded wait ran out (grid barrier)");
         stats->iterations = c.used;
         stats->warm_start_used = 0;
         stats->status = c.status;

@@ -419,7 +419,10 @@ void pdg_warmstart_destroy(pdg_warmstart* w);
  * NULL or one host struct (filling it synchronises the stream).  A frame
  * whose solve produced NaN/Inf keeps x, zeroes v and re-applies the pins;
  * it is reported only through stats->status (PDG_ERR_NUMERIC): the call
- * itself returns PDG_OK, since without stats it does not wait for the GPU. */
+ * itself returns PDG_OK, since without stats it does not wait for the GPU.
+ * The frame is one cooperative launch whose grid barriers are bounded (about
+ * 2 s); a wait that runs out is reported as PDG_ERR_TIMEOUT when stats are
+ * asked for, and x and v are then undefined. */
 #define PDG_NOALLOC_MAX_VERTS 131072
 #define PDG_NOALLOC_MAX_ITERS 4096
 int  pdg_step_noalloc(const pdg_config* cfg, int N, float* d_pos, float* d_vel, const float* d_mass,
