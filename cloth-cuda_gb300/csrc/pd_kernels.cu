@@ -194,7 +194,7 @@ __global__ void k_reset_rt(ClothRT* crt, double* acc, int acc_stride)
 
 __global__ void k_frame_stats(IterArgs a)
 {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;   // one warp per cloth
     if (c < a.ncloth) frame_stats_cloth(a, c);
 }
 
@@ -356,7 +356,7 @@ cudaError_t launch_predict(const IterArgs& a, const float4* X, const float4* V, 
 cudaError_t launch_finalize(const IterArgs& a, float4* X, float4* V, const float4* aux, const int* vcloth, int n,
                             cudaStream_t s)
 {
-    k_frame_stats<<<nblk(a.ncloth, 128), 128, 0, s>>>(a);
+    k_frame_stats<<<nblk(a.ncloth, 4), 128, 0, s>>>(a);
     k_finalize<<<nblk(n, 256), 256, 0, s>>>(X, V, a.Y, a.buf[0], a.buf[1], aux, vcloth, a.cinfo, a.crt, n);
     return cudaGetLastError();
 }

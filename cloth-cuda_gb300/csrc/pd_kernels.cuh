@@ -800,21 +800,33 @@ __device__ __forceinline__ void predict_vertex(int i, const float4* X, const flo
 
 // Cloths still active after the last sweep keep x^max_iter.  A non-finite
 // per-sweep sum marks the cloth as failed (sweeps that ran with neighbour
-// synchronisation skip the per-sweep check).
+// synchronisation skip the per-sweep check).  One warp per cloth: its lanes
+// look through the sums together.  (One thread reading them one after another
+// took 0.3 us per sweep of the cap: 61 us of a 200-sweep frame.)
 __device__ __forceinline__ void frame_stats_cloth(const IterArgs& a, int c)
 {
     ClothRT* rt = a.crt + c;
     const ClothInfo& ci = a.cinfo[c];
     const double* acc = a.acc + (size_t)c * a.acc_stride;
-    if (ci.mode == kModeConsistent) {
-        rt->res0_2 = __ldcg(&acc[0]);
-        if (!(ci.init >= 2 && a.warm_active)) rt->res_y2 = rt->res0_2;
+    const int lane = threadIdx.x & 31;
+    const bool consistent = ci.mode == kModeConsistent;
+    const int active = __ldcg(&rt->active);
+    bool finite = true;
+    if (consistent && active)
+        for (int k = lane; k <= ci.max_iter && k < a.acc_stride; k += 32) {
+            const double v = __ldcg(&acc[k]);
+            finite = finite && isfinite(v);
+        }
+    finite = __all_sync(0xffffffffu, finite) != 0;
+    if (lane != 0) return;
+    if (consistent) {
+        const double r0 = __ldcg(&acc[0]);
+        rt->res0_2 = r0;
+        if (!(ci.init >= 2 && a.warm_active)) rt->res_y2 = r0;
     }
-    if (__ldcg(&rt->active)) {
+    if (active) {
         rt->used = ci.max_iter;
-        if (ci.mode == kModeConsistent) {
-            bool finite = true;
-            for (int k = 0; k <= ci.max_iter && k < a.acc_stride; ++k) finite = finite && isfinite(__ldcg(&acc[k]));
+        if (consistent) {
             const double rf = __ldcg(&acc[ci.max_iter]);
             rt->resf_2 = a.have_final ? rf : -1.0;
             if (!finite) rt->status = -6;

@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(NT) k_persistent(PersistArgs p)
         if (!grid_barrier(p.bar, p.err, p.spin_budget)) return;
     }
 
-    for (int c = gtid; c < a.ncloth; c += gstride) frame_stats_cloth(a, c);
+    for (int c = gtid >> 5; c < a.ncloth; c += gstride >> 5) frame_stats_cloth(a, c);
     if (!grid_barrier(p.bar, p.err, p.spin_budget)) return;
     for (int i = gtid; i < p.n; i += gstride)
         finalize_vertex(i, p.Xw, p.V, p.Y, a.buf[0], a.buf[1], p.aux, p.vcloth, a.cinfo, a.crt);

@@ -351,6 +351,10 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
         // tag the top of the next sweep needs no round trip (257x257 sweep
         // 4.72 -> 4.60 us; read before phase B instead: 4.76 us)
         unsigned long long pw0 = 0, pw1 = 0, pw2 = 0;
+        // A patch whose records all fit one round of the threads computes them
+        // together: one local step and barrier less on the sweep's chain.
+        const bool one_phase = ncell + nhin <= NT;
+        const int na = one_phase ? ncell : ph.ncell_a, nha = one_phase ? nhin : ph.nhin_a;
         for (int k = 0; k < nsweep; ++k) {
             if (k > 0 && k <= ci.max_iter) {
                 // the neighbours' d^k (written in their sweep k - 1, which
@@ -387,7 +391,7 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
             // each list), then the boundary vertices, which the neighbouring
             // patches read: their tagged words go out before phase B runs.
             if (!skip_k)
-                local_records<MODE, NT>(rc, rh, hvs, sy, sd, ncell, nhin, 0, ph.ncell_a, 0, ph.nhin_a, cxy, cz);
+                local_records<MODE, NT>(rc, rh, hvs, sy, sd, ncell, nhin, 0, na, 0, nha, cxy, cz);
             named_sync(1, NT);
             // The boundary vertices' sums are on the neighbours' critical path:
             // one thread per vertex, every slot load issued before the
@@ -407,10 +411,12 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
             // phase B stays on the first threads, which reach it after the
             // boundary offsets are out, so that it does not compete with the
             // boundary sums the neighbouring patches wait for.
-            if (!skip_k)
-                local_records<MODE, NT>(rc, rh, hvs, sy, sd, ncell, nhin, ph.ncell_a, ncell, ph.nhin_a, nhin, cxy,
-                                        cz, (ncell - ph.ncell_a) + (nhin - ph.nhin_a) <= 32);
-            named_sync(1, NT);
+            if (!one_phase) {
+                if (!skip_k)
+                    local_records<MODE, NT>(rc, rh, hvs, sy, sd, ncell, nhin, ph.ncell_a, ncell, ph.nhin_a, nhin, cxy,
+                                            cz, (ncell - ph.ncell_a) + (nhin - ph.nhin_a) <= 32);
+                named_sync(1, NT);
+            }
             if (k + 1 < nsweep && k + 1 <= ci.max_iter && hl0 < nlocal)
                 ld_words(p.xch + ((size_t)((k + 1) & 1) * (size_t)p.n + hg0) * 4, pw0, pw1, pw2);
             if (!skip_k && own && tid >= ph.nbnd) {
@@ -461,7 +467,7 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
     }
     // every per-sweep sum is complete after this barrier
     if (nbr && !grid_barrier_r(p.bar, p.err, p.spin_budget)) return;
-    if (first && tid == 0) frame_stats_cloth(a, c);
+    if (first && tid < 32) frame_stats_cloth(a, c);
     if (!grid_barrier_r(p.bar, p.err, p.spin_budget)) return;
     if (caller_out) {
         for (int o = o0; comp && o < p.n; o += (int)gridDim.x * NT) {
