@@ -11,10 +11,14 @@
 // and the sweep; a reader polls the words of its halo vertices until all
 // three carry the tag it expects, so the data itself is the completion flag
 // (one write and one read per exchange, no separate mark and no fence).
-// With a residual tolerance every sweep ends in a grid barrier, because the
-// convergence decision needs the complete per-cloth residual.  Every wait is
-// bounded by a clock64 budget; on expiry the block records an error code and
-// leaves, and so do all others at their next wait.
+// With a residual tolerance (the TOL instance) the sweeps run the same way, and
+// the convergence decision lags: a spare warp adds the block's residual of
+// sweep k while the others go on, and before sweep k + 2 the block reads the
+// complete sum of sweep k.  If the cloth stops there, its vertices step back to
+// d^k, which each thread still holds.  (A grid barrier per sweep, which the
+// complete sum of the last sweep would need, made a 129x129 sweep 5.7 us.)
+// Every wait is bounded by a clock64 budget; on expiry the block records an
+// error code and leaves, and so do all others at their next wait.
 //
 // Used when every patch fits one block (nown <= NT) and all patches are
 // co-resident.
@@ -29,28 +33,28 @@
 
 namespace pdg {
 
-__device__ __forceinline__ bool grid_barrier_r(unsigned* bar, int* err, long long budget)
+// Barrier `phase` (1, 2, ...) of the frame: one arrival per block on a count
+// that only grows (cleared before the frame), polled until every block of the
+// phase is in.  False once a wait, here or in another block, gave up.
+__device__ __forceinline__ bool grid_barrier_r(unsigned* bar, int* err, long long budget, unsigned& phase)
 {
     __shared__ int ok;
     __syncthreads();
+    ++phase;
     if (threadIdx.x == 0) {
-        volatile unsigned* vgen = bar + 1;
-        const unsigned gen = *vgen;
+        const unsigned want = phase * gridDim.x;
         __threadfence();
-        const unsigned arrived = atomicAdd(bar, 1u);
-        if (arrived == gridDim.x - 1) {
-            atomicExch(bar, 0u);
-            __threadfence();
-            atomicAdd(bar + 1, 1u);
-        } else {
+        atomicAdd(bar, 1u);
+        unsigned v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(__cvta_generic_to_global(bar)) : "memory");
+        if (v < want) {
             const long long t0 = clock64();
-            while (*vgen == gen) {
-                if (clock64() - t0 > budget || *(volatile int*)err != 0) { atomicCAS(err, 0, 2); break; }
-                __nanosleep(32);
-            }
+            do {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(__cvta_generic_to_global(bar)) : "memory");
+                if (v < want && (clock64() - t0 > budget || *(volatile int*)err != 0)) { atomicCAS(err, 0, 2); break; }
+            } while (v < want);
         }
-        __threadfence();
-        ok = (*(volatile int*)err == 0);
+        ok = (v >= want && *(volatile int*)err == 0);
     }
     __syncthreads();
     return ok != 0;
@@ -93,6 +97,12 @@ __device__ __forceinline__ void store_frame_state(const PersistArgs& p, int o, i
 __device__ __forceinline__ void named_sync(int id, int count)
 {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
+
+// Arrival without waiting (the waiting side uses named_sync).
+__device__ __forceinline__ void named_arrive(int id, int count)
+{
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
 
 // named_sync that also returns whether `v` held on every taking part thread.
@@ -213,31 +223,36 @@ __device__ __forceinline__ void compute_residual(float r2, float* red, double* a
 }
 
 // Block layout: NT compute threads (thread l < nown owns local vertex l;
-// the patch's records in shared memory) and 32 more threads that help stage
-// the records at the start of the frame and otherwise only take part in the
-// block-wide barriers.  (They were the signal warp of a completion-mark
+// the patch's records in shared memory) and one more warp that helps stage
+// the records at the start of the frame.  In the TOL instance that warp adds
+// the residuals and takes the decisions; otherwise it only takes part in the
+// block-wide barriers.  (It was the signal warp of a completion-mark
 // protocol, which the tagged exchange replaced: 257x257 sweep 5.5 -> 4.7 us,
 // 33x33 4.8 -> 4.3 us, bitwise equal.)
 //
-// Fixed sweep counts (neighbour synchronisation), one sweep of the compute
-// threads:
+// One sweep of the compute threads:
 //   [k > 0: poll the halo's tagged d^k words into shared memory] -> bar 1
 //   (a vote: a failed poll makes every compute thread leave the sweep loop)
 //   -> phase A records -> bar 1 -> update of the boundary vertices (d^(k+1)
 //   to global memory and as tagged words) -> phase B records -> bar 1 ->
 //   [first read of the next sweep's halo words] -> interior update.
-// Barrier 1 counts the NT compute threads.  With a tolerance every sweep ends
-// in a grid barrier instead.
+// Barrier 1 counts the NT compute threads.  TOL: before the vote of sweep
+// k >= 2 the compute threads take the spare warp's decision about sweep k - 2
+// (barrier 4 + (k & 1)), after sweep k they hand it their partial sums
+// (barrier 2 + (k & 1)).  Two of each, so that neither side can arrive twice
+// at a barrier that the other has not left.
 // IO: the instance that also moves the caller's state (p.in_x ... p.out_v);
 // the other one compiles without that code.
-template <int MODE, int NT, bool IO>
+template <int MODE, int NT, bool IO, bool TOL>
 __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistArgs p)
 {
     constexpr int NTT = NT + 32;   // a multiple of 128: 4 warps per SM sub-partition
     extern __shared__ float4 smem[];
     __shared__ PatchHdr ph;
-    __shared__ float red[NTT / 32];
-    __shared__ int skip;
+    __shared__ float red[TOL ? 2 : 1][NTT / 32];
+    __shared__ int dec[2];             // TOL: decision, 0 go on, 1 stop, 2 leave (a wait ran out)
+    __shared__ int gone;               // TOL: the compute threads left early
+    unsigned phase = 0;                // grid barriers so far
     __shared__ float som[kResOmega];   // Chebyshev weights of this cloth
     const IterArgs& a = p.it;
     const int tid = threadIdx.x;
@@ -300,7 +315,12 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
     const bool first = (int)blockIdx.x == ci.patch_begin;
     const int g = ph.vbegin + tid;
     float4 dprev = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (first) reset_rt(a.crt, a.acc, a.acc_stride, c, tid, NTT);
+    if (first) {
+        reset_rt(a.crt, a.acc, a.acc_stride, c, tid, NTT);
+        if (TOL)
+            for (int k = tid; k < a.acc_stride; k += NTT) p.cnt[(size_t)c * a.acc_stride + k] = 0;
+    }
+    if (TOL && tid == 0) gone = 0;
     if (caller_in) {
         if (comp && o0 < p.n) predict_caller_vertex(p, gi0, xi0, vi0);
         for (int o = o0 + (int)gridDim.x * NT; comp && o < p.n; o += (int)gridDim.x * NT)
@@ -327,7 +347,7 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
             }
         }
     }
-    if (!grid_barrier_r(p.bar, p.err, p.spin_budget)) return;
+    if (!grid_barrier_r(p.bar, p.err, p.spin_budget, phase)) return;
     // every block has read the word: the next frame's base
     if (p.xch_tag && blockIdx.x == 0 && tid == 0) *p.xch_tag = tag0 + (unsigned)nsweep;
     if (caller_in && own) dprev = __ldcg(&a.buf[0][g]);
@@ -342,10 +362,12 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
     __syncthreads();
 
     const float gamma = ci.gamma;
-    const bool nbr = p.nbr_sync != 0;
     double* acc = a.acc + (size_t)c * a.acc_stride;
-    if (nbr && comp) {
-        // ---- compute threads, neighbour synchronisation ----
+    const int kend = min(nsweep, ci.max_iter + 1);   // TOL: this cloth's sweeps
+    if (comp) {
+        // ---- compute threads ----
+        float4 dpp = make_float4(0.f, 0.f, 0.f, 0.f);   // TOL: own d^(k-2)
+        bool left = false;
         // the words of this thread's first halo vertex for the next sweep, read
         // ahead while the interior is updated: when they already carry the
         // tag the top of the next sweep needs no round trip (257x257 sweep
@@ -355,7 +377,17 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
         // together: one local step and barrier less on the sweep's chain.
         const bool one_phase = ncell + nhin <= NT;
         const int na = one_phase ? ncell : ph.ncell_a, nha = one_phase ? nhin : ph.nhin_a;
-        for (int k = 0; k < nsweep; ++k) {
+        for (int k = 0; k < (TOL ? kend : nsweep); ++k) {
+            if (TOL && k >= 2) {
+                named_sync(4 + (k & 1), NTT);
+                const int go = dec[k & 1];
+                if (go) {
+                    // the cloth stops at d^(k-2), or a wait ran out
+                    if (go == 1 && own) ((k & 1) ? a.buf[1] : a.buf[0])[g] = dpp;
+                    left = true;
+                    break;
+                }
+            }
             if (k > 0 && k <= ci.max_iter) {
                 // the neighbours' d^k (written in their sweep k - 1, which
                 // every sweep up to the cloth's cap has): poll the tagged
@@ -376,7 +408,14 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
                     }
                     sd[l] = v;
                 }
-                if (!named_and(1, NT, ok)) break;   // the grid barrier below reports the error
+                if (!named_and(1, NT, ok)) {   // the grid barrier below reports the error
+                    if (TOL) {
+                        if (tid == 0) gone = 1;
+                        named_arrive(2 + (k & 1), NTT);
+                        left = true;
+                    }
+                    break;
+                }
             } else {
                 named_sync(1, NT);
             }
@@ -426,49 +465,90 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
             // every record has read d^k: the owned offsets move on
             if (!skip_k && own && !res_only) {
                 sd[tid] = o;
+                if (TOL) dpp = dprev;
                 dprev = d;
             }
-            // fixed sweep counts read only the residual of the start and of
-            // the last sweeps
-            if (MODE == kModeConsistent && !skip_k && (k == 0 || k >= ci.max_iter - 1))
-                compute_residual<NT>(r2, red, acc + k);
+            if (TOL) {
+                // the block's residual is added by the spare warp
+                r2 = warp_sum(r2);
+                if ((tid & 31) == 0) red[k & 1][tid >> 5] = r2;
+                named_arrive(2 + (k & 1), NTT);
+            } else if (MODE == kModeConsistent && !skip_k && (k == 0 || k >= ci.max_iter - 1)) {
+                // fixed sweep counts read only the residual of the start and
+                // of the last sweeps
+                compute_residual<NT>(r2, red[0], acc + k);
+            }
         }
-    } else if (!nbr) {
-        // ---- tolerance: every sweep ends in a grid barrier ----
-        for (int k = 0; k < nsweep; ++k) {
-            if (tid == 0) skip = cloth_done(a, c, k, first, true) ? 1 : 0;
-            if (k > 0 && comp) {
-                const float4* Dk = (k & 1) ? a.buf[1] : a.buf[0];
-                if (hl0 < nlocal) sd[hl0] = __ldcg(&Dk[hg0]);
-                for (int l = hl0 + NT; l < nlocal; l += NT) sd[l] = __ldcg(&Dk[__ldg(&a.halo[ph.halo_off + l - nown])]);
-            }
-            __syncthreads();
-            const bool skip_k = skip != 0;
-            const float omega_k =
-                k < a.omega_stride ? (k < kResOmega ? som[k] : a.omega[c * a.omega_stride + k]) : 1.f;
-            const bool res_only = k >= ci.max_iter;
-            float4 o = make_float4(0.f, 0.f, 0.f, 0.f), d = o;
-            float r2 = 0.f;
-            if (!skip_k) {
-                if (comp) local_records<MODE, NT>(rc, rh, hvs, sy, sd, ncell, nhin, 0, ncell, 0, nhin, cxy, cz);
-                __syncthreads();
-                if (own) {
-                    vertex_update<MODE>(npad, sptr, tid, sy, sd, cxy, cz, dprev, gamma, omega_k, o, d, r2);
-                    if (!res_only) {
-                        ((k & 1) ? a.buf[0] : a.buf[1])[g] = o;
-                        sd[tid] = o;
-                        dprev = d;
+        if (TOL && !left && kend >= 2) {
+            // the last decision, about sweep kend - 2; the last sweep may have
+            // only evaluated the residual
+            named_sync(4 + (kend & 1), NTT);
+            if (dec[kend & 1] == 1 && own && kend - 1 < ci.max_iter) ((kend & 1) ? a.buf[1] : a.buf[0])[g] = dpp;
+        }
+    } else if (TOL) {
+        // ---- the spare warp: residual sums and decisions ----
+        int* cnt = p.cnt + (size_t)c * a.acc_stride;
+        const int npc = ci.patch_end - ci.patch_begin;
+        const int lane = tid & 31;
+        for (int k = 0; k < kend; ++k) {
+            if (k >= 1) {
+                // the decision about sweep k - 1, taken at the top of sweep
+                // k + 1: every patch of the cloth has added its part of the
+                // sum by now or is about to
+                const int j = k - 1;
+                int go = 0;
+                if (lane == 0) {
+                    int n;
+                    const long long t0 = clock64();
+                    do {
+                        asm volatile("ld.acquire.gpu.global.s32 %0, [%1];"
+                                     : "=r"(n) : "l"(__cvta_generic_to_global(cnt + j)) : "memory");
+                        if (n < npc && (clock64() - t0 > p.spin_budget || *(volatile int*)p.err != 0)) {
+                            atomicCAS(p.err, 0, 3);
+                            go = 2;
+                            break;
+                        }
+                    } while (n < npc);
+                    if (go == 0) {
+                        const double ry2 = ld_cg_f64(acc), rk2 = ld_cg_f64(acc + j);
+                        const float tol = ci.tol;
+                        const bool bad = !isfinite(rk2);
+                        if (bad || (tol > 0.f && rk2 <= (double)tol * (double)tol * ry2)) {
+                            go = 1;
+                            if (first) {
+                                ClothRT* rt = a.crt + c;
+                                rt->used = j; rt->resf_2 = rk2; rt->active = 0;
+                                if (bad) rt->status = -6;
+                            }
+                        }
                     }
+                    dec[(k + 1) & 1] = go;
                 }
-                if (MODE == kModeConsistent) block_residual<NTT>(r2, red, acc + k);
+                go = __shfl_sync(0xffffffffu, go, 0);
+                __syncwarp();
+                named_arrive(4 + ((k + 1) & 1), NTT);
+                if (go) {
+                    // the compute threads finish sweep k and stop at the top
+                    // of the next one: their partial sums are not needed
+                    named_sync(2 + (k & 1), NTT);
+                    break;
+                }
             }
-            if (!grid_barrier_r(p.bar, p.err, p.spin_budget)) return;
+            named_sync(2 + (k & 1), NTT);
+            if (*(volatile int*)&gone) break;
+            float v = lane < NT / 32 ? red[k & 1][lane] : 0.f;
+            v = warp_sum(v);
+            if (lane == 0) {
+                atomicAdd(acc + k, (double)v);
+                __threadfence();
+                atomicAdd(cnt + k, 1);
+            }
         }
     }
     // every per-sweep sum is complete after this barrier
-    if (nbr && !grid_barrier_r(p.bar, p.err, p.spin_budget)) return;
+    if (!grid_barrier_r(p.bar, p.err, p.spin_budget, phase)) return;
     if (first && tid < 32) frame_stats_cloth(a, c);
-    if (!grid_barrier_r(p.bar, p.err, p.spin_budget)) return;
+    if (!grid_barrier_r(p.bar, p.err, p.spin_budget, phase)) return;
     if (caller_out) {
         for (int o = o0; comp && o < p.n; o += (int)gridDim.x * NT) {
             const int gv = __ldg(&p.io_inv[o]);
@@ -481,18 +561,21 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
 }
 
 // NT compute threads plus one warp: 480 + 32 threads, one block (one patch)
-// per SM; 224 + 32, two half-size patches per SM.  Instances: the
-// consistent solve, the reference-literal solve, and the consistent solve
-// that moves the caller's state.
-struct ResVariant { int nt; void* f[3]; };
+// per SM; 224 + 32, two half-size patches per SM.  Instances: fixed sweep
+// counts (the consistent solve, the reference-literal solve, the consistent
+// solve that moves the caller's state), then the consistent solve to a
+// tolerance without and with the caller's state.
+struct ResVariant { int nt; void* f[5]; };
 
 static const ResVariant* res_variants(int* n)
 {
     static const ResVariant v[] = {
-        {480, {(void*)k_resident<kModeConsistent, 480, false>, (void*)k_resident<kModeLiteral, 480, false>,
-               (void*)k_resident<kModeConsistent, 480, true>}},
-        {224, {(void*)k_resident<kModeConsistent, 224, false>, (void*)k_resident<kModeLiteral, 224, false>,
-               (void*)k_resident<kModeConsistent, 224, true>}},
+        {480, {(void*)k_resident<kModeConsistent, 480, false, false>, (void*)k_resident<kModeLiteral, 480, false, false>,
+               (void*)k_resident<kModeConsistent, 480, true, false>, (void*)k_resident<kModeConsistent, 480, false, true>,
+               (void*)k_resident<kModeConsistent, 480, true, true>}},
+        {224, {(void*)k_resident<kModeConsistent, 224, false, false>, (void*)k_resident<kModeLiteral, 224, false, false>,
+               (void*)k_resident<kModeConsistent, 224, true, false>, (void*)k_resident<kModeConsistent, 224, false, true>,
+               (void*)k_resident<kModeConsistent, 224, true, true>}},
     };
     *n = 2;
     return v;
@@ -507,37 +590,41 @@ int resident_pick(int nt)
     return -1;
 }
 
-static void* variant_fn(int variant, int mode, bool io)
+static void* variant_fn(int variant, int mode, bool io, bool tol)
 {
     int n = 0;
     const ResVariant* v = res_variants(&n);
     if (variant < 0 || variant >= n) return nullptr;
-    if (io) return mode == kModeConsistent ? v[variant].f[2] : nullptr;
-    return v[variant].f[mode == kModeConsistent ? 0 : 1];
+    if (mode != kModeConsistent) return io || tol ? nullptr : v[variant].f[1];
+    return v[variant].f[tol ? (io ? 4 : 3) : (io ? 2 : 0)];
 }
 
 bool resident_moves_state(int mode) { return mode == kModeConsistent; }
 
 int resident_max_blocks(int mode, int variant, size_t smem)
 {
-    void* f = variant_fn(variant, mode, false);
-    if (!f) return 0;
     int n = 0;
+    if (!variant_fn(variant, mode, false, false)) return 0;
     const int nt = res_variants(&n)[variant].nt;
-    for (void* fi : {f, variant_fn(variant, mode, true)})
-        if (fi && cudaFuncSetAttribute(fi, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess)
-            return 0;
-    int dev = 0, nsm = 0, nb = 0;
+    int dev = 0, nsm = 0, nb = 1 << 30;
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
     if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, f, nt + 32, smem) != cudaSuccess) return 0;
+    // the solver may run any instance of its mode (the tolerance can change)
+    for (int i = 0; i < 4; ++i) {
+        void* f = variant_fn(variant, mode, (i & 1) != 0, (i & 2) != 0);
+        int nbi = 0;
+        if (!f) continue;
+        if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess) return 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbi, f, nt + 32, smem) != cudaSuccess) return 0;
+        nb = nbi < nb ? nbi : nb;
+    }
     return nb * nsm;
 }
 
 cudaError_t launch_resident(const PersistArgs& p, int variant, int grid, size_t smem, cudaStream_t s)
 {
     const bool io = p.in_x || p.in_v || p.out_x || p.out_v;
-    void* f = variant_fn(variant, p.mode, io);
+    void* f = variant_fn(variant, p.mode, io, p.nbr_sync == 0);
     if (!f || grid <= 0) return cudaErrorInvalidValue;
     int n = 0;
     const int nt = res_variants(&n)[variant].nt;

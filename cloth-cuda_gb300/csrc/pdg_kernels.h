@@ -76,7 +76,10 @@ struct PersistArgs {
     // which every frame advances by its sweep count (null: no exchange)
     unsigned long long* xch;
     unsigned* xch_tag;
-    int nbr_sync;        // 1: sweeps wait for neighbour patches only
+    int nbr_sync;        // 1: no cloth has a tolerance
+    // resident kernel, with a tolerance: per cloth and sweep (acc_stride
+    // entries each) the patches that have added their part of the residual
+    int* cnt;
     // caller state moved inside the frame launch (resident kernel only): x, v
     // read by the prediction and written by the finalisation, AoS xyz in
     // caller order; any may be null.  Device or page-locked mapped host

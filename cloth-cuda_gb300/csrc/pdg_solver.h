@@ -111,6 +111,7 @@ struct pdg_solver {
     // tag base
     pdg::DevBuf<unsigned long long> xch;
     pdg::DevBuf<unsigned> xch_tag;
+    pdg::DevBuf<int> res_cnt;       // resident kernel: arrivals per cloth and sweep (tolerances)
     int acc_stride = 1;
     int nbr_sync = 0;
     pdg::DevBuf<pdg::PatchHdr> patches;

@@ -86,6 +86,7 @@ int upload_all(pdg_solver* s)
     if (s->kernel == PDG_KERNEL_RESIDENT) {
         CK(s->xch.alloc(8 * (size_t)L.ntot));
         CK(cudaMemsetAsync(s->xch.p, 0, sizeof(unsigned long long) * 8 * (size_t)L.ntot, st));
+        CK(s->res_cnt.alloc((size_t)L.ncloth * s->acc_stride));
         CK(s->xch_tag.alloc(1));
         CK(cudaMemsetAsync(s->xch_tag.p, 0, sizeof(unsigned), st));
     }
@@ -135,6 +136,7 @@ PersistArgs persist_args(pdg_solver* s)
     p.xch = s->xch.p;
     p.xch_tag = s->xch_tag.p;
     p.nbr_sync = s->nbr_sync;
+    p.cnt = s->res_cnt.p;
     p.in_x = p.in_v = nullptr;
     p.out_x = p.out_v = nullptr;
     p.io_inv = s->inv_global.p;
@@ -342,7 +344,7 @@ int pdg::create_solver(int n, const pdg_config* cfgs, const pdg_mesh* const* mes
             s->nt = rnt + 32;
             s->res_variant = variant;
             s->persist_grid = s->L.npatch;
-            // fixed sweep counts: neighbour-only synchronisation between sweeps
+            // fixed sweep counts need no decisions
             s->nbr_sync = 1;
             for (const auto& c : s->cloths)
                 if (c.cfg.tolerance > 0.f) s->nbr_sync = 0;
