@@ -147,17 +147,17 @@ int forward(pdg_warmstart* w, cudaStream_t st)
     return PDG_OK;
 }
 
-int wgrad_grid(int M) { return std::max(1, std::min(kWgradBlocks, nb(M, 32))); }
+int wgrad_grid(int M) { return std::max(1, std::min(kWgradBlocks, nb(M, kWgradRows))); }
 
 // dW (nout x K) and db (nout, may be null) of dY^T X over M rows: block
 // partial sums, then their sum in a fixed order
-template <typename TY, typename TX>
-void wgrad(pdg_warmstart* w, const TY* dY, int ldy, int nout, const TX* X, int ldx, int K, int M, float* dW,
+template <int NP, int KP>
+void wgrad(pdg_warmstart* w, const float* dY, int ldy, int nout, const bf16* X, int ldx, int K, int M, float* dW,
            float* db, cudaStream_t st)
 {
     const int gw = wgrad_grid(M);
-    k_wgrad<TY, TX><<<gw, 256, 0, st>>>(dY, ldy, nout, X, ldx, K, M, w->part.p);
-    k_sum_parts<<<nb(nout * K + nout, 256), 256, 0, st>>>(w->part.p, gw, nout * K, nout, dW, db);
+    k_wgrad<NP, KP><<<gw, 256, 0, st>>>(dY, ldy, nout, X, ldx, K, M, w->part.p);
+    k_sum_parts<<<nb(nout * K + nout, 32), 256, 0, st>>>(w->part.p, gw, nout * K, nout, dW, db);
 }
 
 // gradients of the loss w.r.t. all parameters into w->g (zeroed here);
@@ -173,25 +173,25 @@ int backward(pdg_warmstart* w, float inv_cnt, const float* ew, cudaStream_t st)
     GK(cudaMemsetAsync(w->loss.p, 0, sizeof(double), st));
     k_loss<<<nb(N, 256), 256, 0, st>>>(N, w->out.p, w->target.p, w->freew.p, w->ptr.p, w->adj.p, ew, w->smooth,
                                        inv_cnt, w->dout.p, w->loss.p);
-    wgrad<float, bf16>(w, w->dout.p, 16, NO, w->hfin.p, H, H, N, g + y.Wd, g + y.bd, st);
+    wgrad<16, H>(w, w->dout.p, 16, NO, w->hfin.p, H, H, N, g + y.Wd, g + y.bd, st);
     gemm<float, 16, H, EPI_STOREF>(st, w->dout.p, 16, N, w->W.Wdt, nullptr, nullptr, 0, nullptr, 0, nullptr, 0, w->dh.p,
                                    H);
     for (int l = L - 1; l >= 0; --l) {
         k_relu_bwd<<<nb((long long)N * H, 256), 256, 0, st>>>(N, H, w->dh.p, H, w->uo[l].p, H, w->dtmp.p, H);
-        wgrad<float, bf16>(w, w->dtmp.p, H, H, w->cat[l].p, 2 * H, 2 * H, N, g + y.U[l], g + y.u[l], st);
+        wgrad<H, 2 * H>(w, w->dtmp.p, H, H, w->cat[l].p, 2 * H, 2 * H, N, g + y.U[l], g + y.u[l], st);
         gemm<float, H, 2 * H, EPI_STOREF>(st, w->dtmp.p, H, N, w->W.Ut[l], nullptr, nullptr, 0, nullptr, 0, nullptr, 0,
                                           w->dcat.p, 2 * H);
         k_add<<<nb((long long)N * H, 256), 256, 0, st>>>(N, H, w->dcat.p, 2 * H, w->dh.p, H);
         const int gm = std::max(1, std::min(kMsgBwdBlocks, nb(N, 8)));
         k_msg_bwd<<<gm, 256, 0, st>>>(N, w->ptr.p, w->adj.p, w->rev.p, w->ef.p, w->deg_inv.p, w->pq[l].p, p + y.C[l],
                                       p + y.c[l], w->dcat.p, w->dpq.p, w->part.p);
-        k_sum_parts<<<nb(H * (EF + 1), 256), 256, 0, st>>>(w->part.p, gm, H * EF, H, g + y.C[l], g + y.c[l]);
-        wgrad<float, bf16>(w, w->dpq.p, 2 * H, 2 * H, w->cat[l].p, 2 * H, H, N, g + y.A[l], nullptr, st);
+        k_sum_parts<<<nb(H * (EF + 1), 32), 256, 0, st>>>(w->part.p, gm, H * EF, H, g + y.C[l], g + y.c[l]);
+        wgrad<2 * H, H>(w, w->dpq.p, 2 * H, 2 * H, w->cat[l].p, 2 * H, H, N, g + y.A[l], nullptr, st);
         gemm<float, 2 * H, H, EPI_ACCF>(st, w->dpq.p, 2 * H, N, w->W.ABt[l], nullptr, nullptr, 0, nullptr, 0, nullptr, 0,
                                         w->dh.p, H);
     }
     k_relu_bwd<<<nb((long long)N * H, 256), 256, 0, st>>>(N, H, w->dh.p, H, w->cat[0].p, 2 * H, w->dtmp.p, H);
-    wgrad<float, bf16>(w, w->dtmp.p, H, H, w->xin.p, NFP, NF, N, g + y.We, g + y.be, st);
+    wgrad<H, NFP>(w, w->dtmp.p, H, H, w->xin.p, NFP, NF, N, g + y.We, g + y.be, st);
     GK(cudaGetLastError());
     return PDG_OK;
 }
