@@ -279,9 +279,9 @@ int warm_infer_enqueue(pdg_warmstart* w, pdg_solver* s)
 // messages and the fused update
 int warm_kernel_count() { return 3 + 2 * L; }
 
-void warm_detach(pdg_warmstart* w)
+void warm_detach(pdg_warmstart* w, const pdg_solver* s)
 {
-    if (w) w->solver = nullptr;
+    if (w && w->solver == s) w->solver = nullptr;
 }
 
 int warm_judge_sweeps(const pdg_warmstart* w) { return w ? w->judge : 0; }
@@ -409,6 +409,20 @@ int pdg_warmstart_attach(pdg_warmstart* w, pdg_solver* s)
     if (!w || !s) return set_error(PDG_ERR_ARG, "pdg_warmstart_attach: null argument");
     if (s->kernel != PDG_KERNEL_GRAPH && s->kernel != PDG_KERNEL_STREAM)
         return set_error(PDG_ERR_STATE, "pdg_warmstart_attach: the solver must use the per-sweep (graph) kernels");
+    // a network serves one solver and a solver has one network: either's former
+    // partner lets go (its frames then start from the inertial prediction)
+    if (w->solver && w->solver != s) {
+        pdg_solver* old = w->solver;
+        GK(cudaStreamSynchronize(old->stream));
+        old->ws = nullptr;
+        if (old->graph) { cudaGraphExecDestroy(old->graph); old->graph = nullptr; }
+        w->solver = nullptr;
+    }
+    if (s->ws && s->ws != w) {
+        GK(cudaStreamSynchronize(s->stream));
+        warm_detach(s->ws, s);
+        s->ws = nullptr;
+    }
     const HostLayout& Lh = s->L;
     const int N = Lh.ntot;
     // mesh adjacency in the solver's (reordered) numbering, both directions

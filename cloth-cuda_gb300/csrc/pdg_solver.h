@@ -146,5 +146,5 @@ int warm_kernel_count();
 // sweeps each start runs before the judge compares them (0: compare the
 // start residuals)
 int warm_judge_sweeps(const pdg_warmstart* w);
-void warm_detach(pdg_warmstart* w);
+void warm_detach(pdg_warmstart* w, const pdg_solver* s);
 }  // namespace pdg

@@ -18,7 +18,7 @@ using namespace pdg;
 
 pdg_solver::~pdg_solver()
 {
-    if (ws) warm_detach(ws);
+    if (ws) warm_detach(ws, this);
     if (graph) cudaGraphExecDestroy(graph);
     if (own_stream && stream) cudaStreamDestroy(stream);
 }

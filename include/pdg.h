@@ -359,7 +359,9 @@ int  pdg_warmstart_eval(pdg_warmstart* w, int N, const float* x, const int* ptr,
 /* One Adam step (beta 0.9/0.999) with the gradients of the last eval/train. */
 int  pdg_warmstart_adam_step(pdg_warmstart* w, float lr);
 /* Bind to a solver (per-sweep kernels); its frames then use the prediction
- * for cloths with cfg.init == PDG_INIT_WARMSTART or _KEEP. */
+ * for cloths with cfg.init == PDG_INIT_WARMSTART or _KEEP.  A network serves
+ * one solver and a solver has one network: attaching releases the former
+ * partner of either. */
 int  pdg_warmstart_attach(pdg_warmstart* w, pdg_solver* s);
 /* Training on data the solver generates: one frame of `s` from its current
  * state, then one Adam step (lr > 0) on (x_n, v_n, y, d_prev) ->
