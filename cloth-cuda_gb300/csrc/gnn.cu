@@ -38,6 +38,7 @@ struct pdg_warmstart {
     DevBuf<bf16> xin, cat[L], pq[L], uo[L], hfin;
     DevBuf<float> out, target, freew, dout, dh, dtmp, dcat, dpq;
     DevBuf<double> loss;
+    DevBuf<int> bad;      // the graph failed its checks
     float smooth = 0.f;   // weight of the neighbour-difference term of the loss
     int energy = 0;       // 1: that term weighted by the PD system's stiffness per edge
     // sweeps each start runs before the judge compares them; 1: the starts'
@@ -100,21 +101,23 @@ int alloc_params(pdg_warmstart* w)
     return PDG_OK;
 }
 
-// activation buffers for N nodes and E directed edges
+// Buffers for N nodes and E directed edges.  They are kept for the network's
+// lifetime and only grow: a call of pdg_warmstart_eval allocated and freed
+// about 35 of them, more than half of its time on a 97x97 graph.
 int alloc_graph(pdg_warmstart* w, int N, int E)
 {
     w->N = N; w->E = E;
-    GK(w->ptr.alloc(N + 1)); GK(w->adj.alloc(E)); GK(w->rev.alloc(E));
-    GK(w->rest.alloc(E)); GK(w->deg_inv.alloc(N)); GK(w->ef.alloc(E)); GK(w->stat.alloc(N));
-    GK(w->Xn.alloc(N)); GK(w->Vn.alloc(N)); GK(w->Dn.alloc(N)); GK(w->ew.alloc(E));
-    GK(w->xin.alloc((size_t)N * NFP));
+    GK(w->ptr.reserve(N + 1)); GK(w->adj.reserve(E)); GK(w->rev.reserve(E));
+    GK(w->rest.reserve(E)); GK(w->deg_inv.reserve(N)); GK(w->ef.reserve(E)); GK(w->stat.reserve(N));
+    GK(w->Xn.reserve(N)); GK(w->Vn.reserve(N)); GK(w->Dn.reserve(N)); GK(w->ew.reserve(E));
+    GK(w->xin.reserve((size_t)N * NFP));
     for (int l = 0; l < L; ++l) {
-        GK(w->cat[l].alloc((size_t)N * 2 * H)); GK(w->pq[l].alloc((size_t)N * 2 * H)); GK(w->uo[l].alloc((size_t)N * H));
+        GK(w->cat[l].reserve((size_t)N * 2 * H)); GK(w->pq[l].reserve((size_t)N * 2 * H)); GK(w->uo[l].reserve((size_t)N * H));
     }
-    GK(w->hfin.alloc((size_t)N * H));
-    GK(w->out.alloc((size_t)N * 16)); GK(w->target.alloc((size_t)N * 3)); GK(w->freew.alloc(N));
-    GK(w->dout.alloc((size_t)N * 16)); GK(w->dh.alloc((size_t)N * H)); GK(w->dtmp.alloc((size_t)N * H));
-    GK(w->dcat.alloc((size_t)N * 2 * H)); GK(w->dpq.alloc((size_t)N * 2 * H)); GK(w->loss.alloc(1));
+    GK(w->hfin.reserve((size_t)N * H));
+    GK(w->out.reserve((size_t)N * 16)); GK(w->target.reserve((size_t)N * 3)); GK(w->freew.reserve(N));
+    GK(w->dout.reserve((size_t)N * 16)); GK(w->dh.reserve((size_t)N * H)); GK(w->dtmp.reserve((size_t)N * H));
+    GK(w->dcat.reserve((size_t)N * 2 * H)); GK(w->dpq.reserve((size_t)N * 2 * H)); GK(w->loss.reserve(1)); GK(w->bad.reserve(1));
     return PDG_OK;
 }
 
@@ -208,38 +211,31 @@ int adam_step(pdg_warmstart* w, float lr, cudaStream_t st)
     return refresh_bf16(w, st);
 }
 
-// reverse-edge index of a symmetric CSR; false if some edge has no reverse
-bool reverse_edges(int N, const std::vector<int>& ptr, const std::vector<int>& adj, std::vector<int>& rev)
+// Room for the graph, and its arrays on `st`: the reverse-edge index and the
+// inverse degrees are formed on the device, where graph_ok finds whether the
+// adjacency was symmetric.
+int upload_graph(pdg_warmstart* w, int N, const int* ptr, int E, const int* adj, cudaStream_t st)
 {
-    rev.assign(adj.size(), -1);
-    for (int i = 0; i < N; ++i)
-        for (int e = ptr[i]; e < ptr[i + 1]; ++e) {
-            const int j = adj[e];
-            if (j < 0 || j >= N) return false;
-            for (int f = ptr[j]; f < ptr[j + 1]; ++f)
-                if (adj[f] == i) { rev[e] = f; break; }
-            if (rev[e] < 0) return false;
-        }
-    return true;
+    // work that still reads the buffers
+    GK(cudaStreamSynchronize(w->stream));
+    if (w->solver) GK(cudaStreamSynchronize(w->solver->stream));
+    const int rc = alloc_graph(w, N, E);
+    if (rc) return rc;
+    GK(cudaMemcpyAsync(w->ptr.p, ptr, sizeof(int) * ((size_t)N + 1), cudaMemcpyHostToDevice, st));
+    if (E) GK(cudaMemcpyAsync(w->adj.p, adj, sizeof(int) * (size_t)E, cudaMemcpyHostToDevice, st));
+    GK(cudaMemsetAsync(w->bad.p, 0, sizeof(int), st));
+    k_graph<<<nb(N, 256), 256, 0, st>>>(N, E, w->ptr.p, w->adj.p, w->rev.p, w->deg_inv.p, w->bad.p);
+    GK(cudaGetLastError());
+    return PDG_OK;
 }
 
-int upload_graph(pdg_warmstart* w, const std::vector<int>& ptr, const std::vector<int>& adj, cudaStream_t st)
+// Waits for upload_graph's checks; nothing may read the graph before.
+int graph_ok(pdg_warmstart* w, cudaStream_t st)
 {
-    const int N = (int)ptr.size() - 1;
-    std::vector<int> rev;
-    if (!reverse_edges(N, ptr, adj, rev)) return set_error(PDG_ERR_ARG, "warm start: adjacency is not symmetric");
-    std::vector<float> dinv(N);
-    for (int i = 0; i < N; ++i) dinv[i] = ptr[i + 1] > ptr[i] ? 1.f / (float)(ptr[i + 1] - ptr[i]) : 0.f;
-    const int rc = alloc_graph(w, N, (int)adj.size());
-    if (rc) return rc;
-    GK(cudaMemcpyAsync(w->ptr.p, ptr.data(), sizeof(int) * ptr.size(), cudaMemcpyHostToDevice, st));
-    if (!adj.empty()) {
-        GK(cudaMemcpyAsync(w->adj.p, adj.data(), sizeof(int) * adj.size(), cudaMemcpyHostToDevice, st));
-        GK(cudaMemcpyAsync(w->rev.p, rev.data(), sizeof(int) * rev.size(), cudaMemcpyHostToDevice, st));
-    }
-    GK(cudaMemcpyAsync(w->deg_inv.p, dinv.data(), sizeof(float) * N, cudaMemcpyHostToDevice, st));
+    int bad = 0;
+    GK(cudaMemcpyAsync(&bad, w->bad.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     GK(cudaStreamSynchronize(st));
-    return PDG_OK;
+    return bad ? set_error(PDG_ERR_ARG, "warm start: adjacency is not symmetric") : PDG_OK;
 }
 
 }  // namespace
@@ -364,32 +360,32 @@ int pdg_warmstart_eval(pdg_warmstart* w, int N, const float* x, const int* ptr, 
     const int E = ptr[N];
     if (E < 0 || (E > 0 && (!adj || !ef))) return set_error(PDG_ERR_ARG, "pdg_warmstart_eval: bad adjacency");
     cudaStream_t st = w->stream;
-    std::vector<int> hp(ptr, ptr + N + 1), ha(adj, adj + E);
-    int rc = upload_graph(w, hp, ha, st);
+    int rc = upload_graph(w, N, ptr, E, adj, st);
     if (rc) return rc;
-    std::vector<bf16> xb((size_t)N * NFP);
-    for (int i = 0; i < N; ++i)
-        for (int k = 0; k < NFP; ++k) xb[(size_t)i * NFP + k] = __float2bfloat16_rn(k < NF ? x[(size_t)i * NF + k] : 0.f);
-    GK(cudaMemcpyAsync(w->xin.p, xb.data(), sizeof(bf16) * xb.size(), cudaMemcpyHostToDevice, st));
+    // features to bf16 on the device (staged where the backward pass later
+    // keeps dh)
+    GK(cudaMemcpyAsync(w->dh.p, x, sizeof(float) * NF * (size_t)N, cudaMemcpyHostToDevice, st));
+    k_pack_feat<<<nb(N, 256), 256, 0, st>>>(N, w->dh.p, w->xin.p);
     if (E) GK(cudaMemcpyAsync(w->ef.p, ef, sizeof(float4) * E, cudaMemcpyHostToDevice, st));
     GK(cudaMemcpyAsync(w->target.p, target, sizeof(float) * 3 * N, cudaMemcpyHostToDevice, st));
     GK(cudaMemcpyAsync(w->freew.p, freew, sizeof(float) * N, cudaMemcpyHostToDevice, st));
     if (ew && E) GK(cudaMemcpyAsync(w->ew.p, ew, sizeof(float) * E, cudaMemcpyHostToDevice, st));
+    rc = graph_ok(w, st);
+    if (rc) return rc;
     double cnt = 0.0;
     for (int i = 0; i < N; ++i) cnt += freew[i] > 0.f ? 3.0 : 0.0;
     rc = forward(w, st);
     if (rc) return rc;
     rc = backward(w, (float)(1.0 / std::max(cnt, 1.0)), (ew && E) ? w->ew.p : nullptr, st);
     if (rc) return rc;
-    std::vector<float> o((size_t)N * 16);
     double l = 0.0;
-    GK(cudaMemcpyAsync(o.data(), w->out.p, sizeof(float) * o.size(), cudaMemcpyDeviceToHost, st));
+    if (out) {   // N x 3 of the padded outputs, through a buffer the backward pass is done with
+        k_pack_out<<<nb(N, 256), 256, 0, st>>>(N, w->out.p, w->dtmp.p);
+        GK(cudaMemcpyAsync(out, w->dtmp.p, sizeof(float) * NO * (size_t)N, cudaMemcpyDeviceToHost, st));
+    }
     GK(cudaMemcpyAsync(&l, w->loss.p, sizeof(double), cudaMemcpyDeviceToHost, st));
     if (grads) GK(cudaMemcpyAsync(grads, w->g.p, sizeof(float) * w->lay.total, cudaMemcpyDeviceToHost, st));
     GK(cudaStreamSynchronize(st));
-    if (out)
-        for (int i = 0; i < N; ++i)
-            for (int c = 0; c < NO; ++c) out[3 * i + c] = o[(size_t)i * 16 + c];
     if (loss) *loss = (float)l;
     return PDG_OK;
 }
@@ -477,7 +473,9 @@ int pdg_warmstart_attach(pdg_warmstart* w, pdg_solver* s)
     for (int i = 0; i < N; ++i)
         for (int e = ptr[i]; e < ptr[i + 1]; ++e) ew[e] = 0.5f * (sig[i] + sig[adj[e]]);
     cudaStream_t st = s->stream;
-    int rc = upload_graph(w, ptr, adj, st);
+    int rc = upload_graph(w, N, ptr.data(), (int)adj.size(), adj.data(), st);
+    if (rc) return rc;
+    rc = graph_ok(w, st);
     if (rc) return rc;
     if (!rest.empty()) GK(cudaMemcpyAsync(w->rest.p, rest.data(), sizeof(float) * rest.size(), cudaMemcpyHostToDevice, st));
     if (!ew.empty()) GK(cudaMemcpyAsync(w->ew.p, ew.data(), sizeof(float) * ew.size(), cudaMemcpyHostToDevice, st));

@@ -832,6 +832,52 @@ __global__ void k_to_bf16(const float* __restrict__ src, int rows, int cols, bf1
     if (dstT) dstT[(size_t)c * ldT + r] = b;
 }
 
+// ---- caller graphs ---------------------------------------------------------
+// Per node its inverse degree, per directed edge (i <- adj[e]) the index of its
+// reverse.  *bad is set where the lists leave the arrays or an edge has no
+// reverse; the rest of the node's entries are then left unset.
+__global__ void k_graph(int N, int E, const int* __restrict__ ptr, const int* __restrict__ adj, int* __restrict__ rev,
+                        float* __restrict__ deg_inv, int* __restrict__ bad)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= N) return;
+    const int e0 = ptr[i], e1 = ptr[i + 1];
+    if (e0 < 0 || e1 < e0 || e1 > E) { *bad = 1; return; }
+    deg_inv[i] = e1 > e0 ? __fdiv_rn(1.f, (float)(e1 - e0)) : 0.f;
+    for (int e = e0; e < e1; ++e) {
+        const int j = adj[e];
+        if (j < 0 || j >= N) { *bad = 1; return; }
+        const int f0 = ptr[j], f1 = ptr[j + 1];
+        if (f0 < 0 || f1 < f0 || f1 > E) { *bad = 1; return; }
+        int f = f0;
+        while (f < f1 && adj[f] != i) ++f;
+        if (f == f1) { *bad = 1; return; }
+        rev[e] = f;
+    }
+}
+
+// Caller features (N x NF) to the padded bf16 rows of the encoder.
+__global__ void k_pack_feat(int N, const float* __restrict__ x, bf16* __restrict__ xin)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= N) return;
+    float f[NFP];
+    #pragma unroll
+    for (int k = 0; k < NFP; ++k) f[k] = k < NF ? x[(size_t)i * NF + k] : 0.f;
+    #pragma unroll
+    for (int k = 0; k < NFP; k += 2)
+        *reinterpret_cast<__nv_bfloat162*>(xin + (size_t)i * NFP + k) = __floats2bfloat162_rn(f[k], f[k + 1]);
+}
+
+// The first NO of the 16 padded outputs of every node.
+__global__ void k_pack_out(int N, const float* __restrict__ out, float* __restrict__ dst)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= N) return;
+    #pragma unroll
+    for (int c = 0; c < NO; ++c) dst[(size_t)i * NO + c] = out[(size_t)i * 16 + c];
+}
+
 // ---- solver-side feature kernels -----------------------------------------
 // Node features: (y - x)/s, h v / s, pinned, scaled log mass / log stretch k /
 // log bend k, then the previous frame's offset d_prev / s and its validity

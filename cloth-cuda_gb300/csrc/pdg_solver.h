@@ -55,7 +55,7 @@ std::string check_layout(const std::vector<ClothSetup>& cl, const HostLayout& L)
 template <class T>
 struct DevBuf {
     T* p = nullptr;
-    size_t n = 0;
+    size_t n = 0, cap = 0;
     DevBuf() = default;
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
@@ -63,8 +63,18 @@ struct DevBuf {
     cudaError_t alloc(size_t count)
     {
         if (p) { cudaFree(p); p = nullptr; }
+        n = cap = count;
+        const cudaError_t e = cudaMalloc(&p, sizeof(T) * (count ? count : 1));
+        if (e != cudaSuccess) { p = nullptr; n = cap = 0; }
+        return e;
+    }
+    // room for `count` elements, kept when it is already there (contents
+    // undefined; the caller has waited for the work that used them)
+    cudaError_t reserve(size_t count)
+    {
+        if (!p || cap < count) return alloc(count);
         n = count;
-        return cudaMalloc(&p, sizeof(T) * (count ? count : 1));
+        return cudaSuccess;
     }
     cudaError_t upload(const std::vector<T>& h, cudaStream_t s)
     {
