@@ -243,15 +243,21 @@ __device__ __forceinline__ void compute_residual(float r2, float* red, double* a
 // at a barrier that the other has not left.
 // IO: the instance that also moves the caller's state (p.in_x ... p.out_v);
 // the other one compiles without that code.
-template <int MODE, int NT, bool IO, bool TOL>
+// RANGE (with TOL): sweeps p.k0 .. p.k1 - 1 of a frame whose prediction, start
+// and finalisation are other launches: the streaming plan's sweeps where its
+// patches all fit on the chip at once.  At 54,000 vertices in 128-vertex
+// patches a sweep takes 5.3 us, as launches of the streaming kernel 7.3 us.
+template <int MODE, int NT, bool IO, bool TOL, bool RANGE>
 __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistArgs p)
 {
-    constexpr int NTT = NT + 32;   // a multiple of 128: 4 warps per SM sub-partition
+    static_assert(!RANGE || (TOL && !IO), "ranges take decisions and move no caller state");
+    constexpr int NTT = NT + 32;   // 512 and 256: 4 warps per SM sub-partition
     extern __shared__ float4 smem[];
     __shared__ PatchHdr ph;
     __shared__ float red[TOL ? 2 : 1][NTT / 32];
     __shared__ int dec[2];             // TOL: decision, 0 go on, 1 stop, 2 leave (a wait ran out)
     __shared__ int gone;               // TOL: the compute threads left early
+    __shared__ int over;               // RANGE: the cloth is done before the range
     unsigned phase = 0;                // grid barriers so far
     __shared__ float som[kResOmega];   // Chebyshev weights of this cloth
     const IterArgs& a = p.it;
@@ -315,13 +321,19 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
     const bool first = (int)blockIdx.x == ci.patch_begin;
     const int g = ph.vbegin + tid;
     float4 dprev = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int k0 = RANGE ? p.k0 : 0;   // first sweep
     if (first) {
-        reset_rt(a.crt, a.acc, a.acc_stride, c, tid, NTT);
+        if (!RANGE) reset_rt(a.crt, a.acc, a.acc_stride, c, tid, NTT);
         if (TOL)
             for (int k = tid; k < a.acc_stride; k += NTT) p.cnt[(size_t)c * a.acc_stride + k] = 0;
     }
     if (TOL && tid == 0) gone = 0;
-    if (caller_in) {
+    if (RANGE) {
+        // the decision about the sweep before the range, the same in every
+        // block of the cloth; all have taken it when the barrier below opens
+        if (tid == 0) over = cloth_done(a, c, k0, first, true) ? 1 : 0;
+        if (own) dprev = __ldcg(&((k0 & 1) ? a.buf[0] : a.buf[1])[g]);
+    } else if (caller_in) {
         if (comp && o0 < p.n) predict_caller_vertex(p, gi0, xi0, vi0);
         for (int o = o0 + (int)gridDim.x * NT; comp && o < p.n; o += (int)gridDim.x * NT)
             predict_caller_vertex(p, __ldg(&p.io_inv[o]), caller_vec(p.in_x, o), caller_vec(p.in_v, o));
@@ -334,7 +346,7 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
     // Before the 32-bit tags would wrap, every block clears its boundary
     // vertices' words in both buffers and the frame starts again from 0; the
     // grid barrier below orders the clearing before any neighbour's poll.
-    const int nsweep = p.max_iter + (p.have_final ? 1 : 0);
+    const int nsweep = RANGE ? p.k1 : p.max_iter + (p.have_final ? 1 : 0);   // end of the sweeps
     unsigned tag0 = 0;
     if (p.xch_tag) {
         const unsigned t = __ldcg(p.xch_tag);
@@ -354,7 +366,7 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
     for (int l = tid; l < nlocal; l += NTT) {
         const int gg = l < nown ? ph.vbegin + l : __ldg(&a.halo[ph.halo_off + l - nown]);
         sy[l] = __ldcg(&a.Y[gg]);
-        sd[l] = __ldcg(&a.buf[0][gg]);
+        sd[l] = __ldcg(&(RANGE && (k0 & 1) ? a.buf[1] : a.buf[0])[gg]);
     }
     // this compute thread's first halo vertex, re-read every sweep
     const int hl0 = nown + tid;
@@ -363,7 +375,8 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
 
     const float gamma = ci.gamma;
     double* acc = a.acc + (size_t)c * a.acc_stride;
-    const int kend = min(nsweep, ci.max_iter + 1);   // TOL: this cloth's sweeps
+    // TOL: the end of this cloth's sweeps
+    const int kend = RANGE && over ? k0 : min(nsweep, ci.max_iter + 1);
     if (comp) {
         // ---- compute threads ----
         float4 dpp = make_float4(0.f, 0.f, 0.f, 0.f);   // TOL: own d^(k-2)
@@ -377,8 +390,8 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
         // together: one local step and barrier less on the sweep's chain.
         const bool one_phase = ncell + nhin <= NT;
         const int na = one_phase ? ncell : ph.ncell_a, nha = one_phase ? nhin : ph.nhin_a;
-        for (int k = 0; k < (TOL ? kend : nsweep); ++k) {
-            if (TOL && k >= 2) {
+        for (int k = k0; k < (TOL ? kend : nsweep); ++k) {
+            if (TOL && k >= k0 + 2) {
                 named_sync(4 + (k & 1), NTT);
                 const int go = dec[k & 1];
                 if (go) {
@@ -388,7 +401,7 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
                     break;
                 }
             }
-            if (k > 0 && k <= ci.max_iter) {
+            if (k > k0 && k <= ci.max_iter) {
                 // the neighbours' d^k (written in their sweep k - 1, which
                 // every sweep up to the cloth's cap has): poll the tagged
                 // words of this thread's halo vertices
@@ -479,7 +492,7 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
                 compute_residual<NT>(r2, red[0], acc + k);
             }
         }
-        if (TOL && !left && kend >= 2) {
+        if (TOL && !left && kend >= k0 + 2) {
             // the last decision, about sweep kend - 2; the last sweep may have
             // only evaluated the residual
             named_sync(4 + (kend & 1), NTT);
@@ -490,33 +503,44 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
         int* cnt = p.cnt + (size_t)c * a.acc_stride;
         const int npc = ci.patch_end - ci.patch_begin;
         const int lane = tid & 31;
-        for (int k = 0; k < kend; ++k) {
-            if (k >= 1) {
+        // waits for the complete sum of sweep j; false when a wait ran out
+        auto complete = [&](int j) {
+            const long long t0 = clock64();
+            for (;;) {
+                int n;
+                asm volatile("ld.acquire.gpu.global.s32 %0, [%1];"
+                             : "=r"(n) : "l"(__cvta_generic_to_global(cnt + j)) : "memory");
+                if (n >= npc) return true;
+                if (clock64() - t0 > p.spin_budget || *(volatile int*)p.err != 0) {
+                    atomicCAS(p.err, 0, 3);
+                    return false;
+                }
+            }
+        };
+        bool ended = false;
+        for (int k = k0; k < kend; ++k) {
+            if (k > k0) {
                 // the decision about sweep k - 1, taken at the top of sweep
                 // k + 1: every patch of the cloth has added its part of the
                 // sum by now or is about to
                 const int j = k - 1;
                 int go = 0;
                 if (lane == 0) {
-                    int n;
-                    const long long t0 = clock64();
-                    do {
-                        asm volatile("ld.acquire.gpu.global.s32 %0, [%1];"
-                                     : "=r"(n) : "l"(__cvta_generic_to_global(cnt + j)) : "memory");
-                        if (n < npc && (clock64() - t0 > p.spin_budget || *(volatile int*)p.err != 0)) {
-                            atomicCAS(p.err, 0, 3);
-                            go = 2;
-                            break;
-                        }
-                    } while (n < npc);
+                    if (!complete(j)) go = 2;
                     if (go == 0) {
-                        const double ry2 = ld_cg_f64(acc), rk2 = ld_cg_f64(acc + j);
+                        // the normaliser, as in cloth_done
+                        const bool own_start = !(RANGE && ci.init >= 2 && a.warm_active);
+                        const double ry2 = ld_cg_f64(own_start ? acc : &a.crt[c].res_y2), rk2 = ld_cg_f64(acc + j);
                         const float tol = ci.tol;
                         const bool bad = !isfinite(rk2);
                         if (bad || (tol > 0.f && rk2 <= (double)tol * (double)tol * ry2)) {
                             go = 1;
                             if (first) {
                                 ClothRT* rt = a.crt + c;
+                                if (RANGE) {
+                                    rt->res0_2 = ld_cg_f64(acc);
+                                    if (own_start) rt->res_y2 = ry2;
+                                }
                                 rt->used = j; rt->resf_2 = rk2; rt->active = 0;
                                 if (bad) rt->status = -6;
                             }
@@ -531,11 +555,12 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
                     // the compute threads finish sweep k and stop at the top
                     // of the next one: their partial sums are not needed
                     named_sync(2 + (k & 1), NTT);
+                    ended = true;
                     break;
                 }
             }
             named_sync(2 + (k & 1), NTT);
-            if (*(volatile int*)&gone) break;
+            if (*(volatile int*)&gone) { ended = true; break; }
             float v = lane < NT / 32 ? red[k & 1][lane] : 0.f;
             v = warp_sum(v);
             if (lane == 0) {
@@ -544,7 +569,13 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
                 atomicAdd(cnt + k, 1);
             }
         }
+        // a cloth whose cap lies inside the range: its record, as the sweep
+        // after its last one would have left it
+        const int kq = ci.max_iter + (a.have_final ? 1 : 0);
+        if (RANGE && first && lane == 0 && !ended && kend > k0 && kq < nsweep && complete(kend - 1))
+            cloth_done(a, c, kq, true, true);
     }
+    if (RANGE) return;
     // every per-sweep sum is complete after this barrier
     if (!grid_barrier_r(p.bar, p.err, p.spin_budget, phase)) return;
     if (first && tid < 32) frame_stats_cloth(a, c);
@@ -561,23 +592,31 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
 }
 
 // NT compute threads plus one warp: 480 + 32 threads, one block (one patch)
-// per SM; 224 + 32, two half-size patches per SM.  Instances: fixed sweep
-// counts (the consistent solve, the reference-literal solve, the consistent
-// solve that moves the caller's state), then the consistent solve to a
-// tolerance without and with the caller's state.
-struct ResVariant { int nt; void* f[5]; };
+// per SM; 224 + 32, two half-size patches per SM; 128 + 32, three patches per
+// SM (ranges only).  Instances: fixed sweep counts (the consistent solve, the
+// reference-literal solve, the consistent solve that moves the caller's
+// state), the consistent solve to a tolerance without and with the caller's
+// state, and its ranges of sweeps.
+struct ResVariant { int nt; void* f[6]; };
 
 static const ResVariant* res_variants(int* n)
 {
     static const ResVariant v[] = {
-        {480, {(void*)k_resident<kModeConsistent, 480, false, false>, (void*)k_resident<kModeLiteral, 480, false, false>,
-               (void*)k_resident<kModeConsistent, 480, true, false>, (void*)k_resident<kModeConsistent, 480, false, true>,
-               (void*)k_resident<kModeConsistent, 480, true, true>}},
-        {224, {(void*)k_resident<kModeConsistent, 224, false, false>, (void*)k_resident<kModeLiteral, 224, false, false>,
-               (void*)k_resident<kModeConsistent, 224, true, false>, (void*)k_resident<kModeConsistent, 224, false, true>,
-               (void*)k_resident<kModeConsistent, 224, true, true>}},
+        {480, {(void*)k_resident<kModeConsistent, 480, false, false, false>,
+               (void*)k_resident<kModeLiteral, 480, false, false, false>,
+               (void*)k_resident<kModeConsistent, 480, true, false, false>,
+               (void*)k_resident<kModeConsistent, 480, false, true, false>,
+               (void*)k_resident<kModeConsistent, 480, true, true, false>,
+               (void*)k_resident<kModeConsistent, 480, false, true, true>}},
+        {224, {(void*)k_resident<kModeConsistent, 224, false, false, false>,
+               (void*)k_resident<kModeLiteral, 224, false, false, false>,
+               (void*)k_resident<kModeConsistent, 224, true, false, false>,
+               (void*)k_resident<kModeConsistent, 224, false, true, false>,
+               (void*)k_resident<kModeConsistent, 224, true, true, false>,
+               (void*)k_resident<kModeConsistent, 224, false, true, true>}},
+        {128, {nullptr, nullptr, nullptr, nullptr, nullptr, (void*)k_resident<kModeConsistent, 128, false, true, true>}},
     };
-    *n = 2;
+    *n = 3;
     return v;
 }
 
@@ -599,26 +638,54 @@ static void* variant_fn(int variant, int mode, bool io, bool tol)
     return v[variant].f[tol ? (io ? 4 : 3) : (io ? 2 : 0)];
 }
 
+// Blocks of instance f that are resident at once (0: it cannot run).
+static int resident_blocks_of(void* f, int threads, size_t smem)
+{
+    int dev = 0, nsm = 0, nb = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess) return 0;
+    if (smem > 220 * 1024 || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, f, threads, smem) != cudaSuccess) return 0;
+    return nb * nsm;
+}
+
 bool resident_moves_state(int mode) { return mode == kModeConsistent; }
 
 int resident_max_blocks(int mode, int variant, size_t smem)
 {
-    int n = 0;
-    if (!variant_fn(variant, mode, false, false)) return 0;
-    const int nt = res_variants(&n)[variant].nt;
-    int dev = 0, nsm = 0, nb = 1 << 30;
-    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-    if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    int n = 0, nb = 0;
+    const int nt = variant_fn(variant, mode, false, false) ? res_variants(&n)[variant].nt : 0;
     // the solver may run any instance of its mode (the tolerance can change)
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < 4 && nt; ++i) {
         void* f = variant_fn(variant, mode, (i & 1) != 0, (i & 2) != 0);
-        int nbi = 0;
         if (!f) continue;
-        if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess) return 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbi, f, nt + 32, smem) != cudaSuccess) return 0;
-        nb = nbi < nb ? nbi : nb;
+        const int b = resident_blocks_of(f, nt + 32, smem);
+        nb = i == 0 || b < nb ? b : nb;
     }
-    return nb * nsm;
+    return nb;
+}
+
+int resident_range_pick(int max_nown, int npatch, size_t smem)
+{
+    // the smallest blocks that hold the patches: more of them per SM
+    int n = 0;
+    const ResVariant* v = res_variants(&n);
+    for (int i = n - 1; i >= 0; --i)
+        if (max_nown <= v[i].nt && npatch <= resident_blocks_of(v[i].f[5], v[i].nt + 32, smem)) return i;
+    return -1;
+}
+
+cudaError_t launch_resident_range(const PersistArgs& p, int variant, int grid, size_t smem, cudaStream_t s)
+{
+    int n = 0;
+    const ResVariant* v = res_variants(&n);
+    if (variant < 0 || variant >= n || grid <= 0) return cudaErrorInvalidValue;
+    if (p.k1 <= p.k0) return cudaSuccess;
+    cudaError_t e = cudaMemsetAsync(p.bar, 0, 2 * sizeof(unsigned), s);
+    if (e != cudaSuccess) return e;
+    PersistArgs copy = p;
+    void* args[] = {&copy};
+    return cudaLaunchCooperativeKernel(v[variant].f[5], dim3(grid), dim3(v[variant].nt + 32), args, smem, s);
 }
 
 cudaError_t launch_resident(const PersistArgs& p, int variant, int grid, size_t smem, cudaStream_t s)

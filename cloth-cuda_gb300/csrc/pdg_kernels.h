@@ -80,6 +80,7 @@ struct PersistArgs {
     // resident kernel, with a tolerance: per cloth and sweep (acc_stride
     // entries each) the patches that have added their part of the residual
     int* cnt;
+    int k0, k1;          // launch_resident_range: sweeps k0 .. k1 - 1
     // caller state moved inside the frame launch (resident kernel only): x, v
     // read by the prediction and written by the finalisation, AoS xyz in
     // caller order; any may be null.  Device or page-locked mapped host
@@ -104,6 +105,12 @@ int resident_max_blocks(int mode, int variant, size_t smem);
 // in_x ... out_v) for this mode.
 bool resident_moves_state(int mode);
 cudaError_t launch_resident(const PersistArgs& p, int variant, int grid, size_t smem, cudaStream_t s);
+// Sweeps p.k0 .. p.k1 - 1 of a frame of the consistent mode in one cooperative
+// launch, its prediction, start and finalisation in others.  The variant for
+// patches of at most max_nown vertices that are all resident at once with
+// `smem` bytes each (-1: none).
+int resident_range_pick(int max_nown, int npatch, size_t smem);
+cudaError_t launch_resident_range(const PersistArgs& p, int variant, int grid, size_t smem, cudaStream_t s);
 
 // Streaming per-sweep kernel (pd_stream.cu): persistent grid, the vertex
 // data of each block's next patch double-buffered in shared memory by bulk

@@ -98,6 +98,7 @@ struct pdg_solver {
     int have_final = 1;
     int persist_grid = 0;           // persistent / resident / streaming grid
     int res_variant = -1;           // resident kernel instance (record capacity)
+    int range_variant = -1;         // streaming plan: the resident instance that runs its sweeps, -1: none
     int carveout = 0;               // shared/L1 split of the per-sweep kernel (percent, 0 = default)
     pdg::StreamArgs sargs{};        // streaming kernel: stage layout
     size_t stream_smem = 0;
