@@ -18,6 +18,15 @@ __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b)
 __device__ __forceinline__ float fsub(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ float ffma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdiv_rn(a, b); }
+// Reciprocal square root of a normal number: one instruction.  rsqrtf also
+// handles subnormal inputs (four instructions, the same bits for normal ones);
+// every caller's argument is bounded below by 1e-30.
+__device__ __forceinline__ float frsqrt(float a)
+{
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+    return r;
+}
 __device__ __forceinline__ float dot3(float3 a, float3 b) { return ffma(a.x, b.x, ffma(a.y, b.y, fmul(a.z, b.z))); }
 __device__ __forceinline__ float3 scale3(float3 a, float s) { return make_float3(fmul(a.x, s), fmul(a.y, s), fmul(a.z, s)); }
 __device__ __forceinline__ float3 f3(float4 a) { return make_float3(a.x, a.y, a.z); }
@@ -37,24 +46,24 @@ __device__ __forceinline__ float3 fadd3(float3 a, float3 b)
 __device__ __forceinline__ void polar_consistent(float3 F0, float3 F1, float3& R0, float3& R1)
 {
     const float n0sq = dot3(F0, F0);
-    const float3 b0 = n0sq > 1e-20f ? scale3(F0, rsqrtf(n0sq)) : make_float3(1.f, 0.f, 0.f);
+    const float3 b0 = n0sq > 1e-20f ? scale3(F0, frsqrt(n0sq)) : make_float3(1.f, 0.f, 0.f);
     const float a01 = dot3(F1, b0);
     const float3 c1 = make_float3(ffma(-a01, b0.x, F1.x), ffma(-a01, b0.y, F1.y), ffma(-a01, b0.z, F1.z));
     const float n1sq = dot3(c1, c1);
     float3 b1;
     if (n1sq > 1e-20f) {
-        b1 = scale3(c1, rsqrtf(n1sq));
+        b1 = scale3(c1, frsqrt(n1sq));
     } else {   // F1 parallel to F0: any unit vector orthogonal to b0
         float3 q = make_float3(-b0.y, b0.x, 0.f);
         float nq = ffma(q.x, q.x, fmul(q.y, q.y));
         if (nq < 1e-20f) { q = make_float3(0.f, -b0.z, b0.y); nq = ffma(q.y, q.y, fmul(q.z, q.z)); }
-        b1 = scale3(q, rsqrtf(nq));
+        b1 = scale3(q, frsqrt(nq));
     }
     const float a00 = dot3(b0, F0), a10 = dot3(b1, F0), a11 = dot3(b1, F1);
     const float s = fadd(a00, a11), t = fsub(a10, a01);
     const float rr = ffma(s, s, fmul(t, t));
     float c = 1.f, sn = 0.f;
-    if (rr > 1e-30f) { const float r = rsqrtf(rr); c = fmul(s, r); sn = fmul(t, r); }
+    if (rr > 1e-30f) { const float r = frsqrt(rr); c = fmul(s, r); sn = fmul(t, r); }
     R0 = make_float3(ffma(b0.x, c, fmul(b1.x, sn)), ffma(b0.y, c, fmul(b1.y, sn)), ffma(b0.z, c, fmul(b1.z, sn)));
     R1 = make_float3(ffma(b1.x, c, fmul(-b0.x, sn)), ffma(b1.y, c, fmul(-b0.y, sn)), ffma(b1.z, c, fmul(-b0.z, sn)));
 }
@@ -169,7 +178,7 @@ __device__ __forceinline__ float3 hinge_q(float3 e, float h2k, float nrest)
     float3 p = make_float3(0.f, 0.f, 0.f);
     if (MODE == kModeConsistent) {
         const float n2 = dot3(e, e);
-        if (nrest > 1e-10f && n2 > 1e-20f) p = scale3(e, fmul(nrest, rsqrtf(n2)));
+        if (nrest > 1e-10f && n2 > 1e-20f) p = scale3(e, fmul(nrest, frsqrt(n2)));
         return make_float3(fmul(h2k, fsub(p.x, e.x)), fmul(h2k, fsub(p.y, e.y)), fmul(h2k, fsub(p.z, e.z)));
     }
     if (nrest > 1e-10f) {
@@ -289,24 +298,24 @@ __device__ __forceinline__ V3 edge4_p(float4 yi, float4 di, float4 yj, float4 dj
 __device__ __forceinline__ void polar_consistent_p(V3 F0, V3 F1, V3& R0, V3& R1)
 {
     const float n0sq = vdot(F0, F0);
-    const V3 b0 = n0sq > 1e-20f ? vscale(F0, rsqrtf(n0sq)) : V3{make_float2(1.f, 0.f), 0.f};
+    const V3 b0 = n0sq > 1e-20f ? vscale(F0, frsqrt(n0sq)) : V3{make_float2(1.f, 0.f), 0.f};
     const float a01 = vdot(F1, b0);
     const V3 c1 = vfma(b0, -a01, F1);
     const float n1sq = vdot(c1, c1);
     V3 b1;
     if (n1sq > 1e-20f) {
-        b1 = vscale(c1, rsqrtf(n1sq));
+        b1 = vscale(c1, frsqrt(n1sq));
     } else {   // F1 parallel to F0: any unit vector orthogonal to b0
         float3 q = make_float3(-b0.xy.y, b0.xy.x, 0.f);
         float nq = ffma(q.x, q.x, fmul(q.y, q.y));
         if (nq < 1e-20f) { q = make_float3(0.f, -b0.z, b0.xy.y); nq = ffma(q.y, q.y, fmul(q.z, q.z)); }
-        b1 = v3(scale3(q, rsqrtf(nq)));
+        b1 = v3(scale3(q, frsqrt(nq)));
     }
     const float a00 = vdot(b0, F0), a10 = vdot(b1, F0), a11 = vdot(b1, F1);
     const float s = fadd(a00, a11), t = fsub(a10, a01);
     const float rr = ffma(s, s, fmul(t, t));
     float c = 1.f, sn = 0.f;
-    if (rr > 1e-30f) { const float r = rsqrtf(rr); c = fmul(s, r); sn = fmul(t, r); }
+    if (rr > 1e-30f) { const float r = frsqrt(rr); c = fmul(s, r); sn = fmul(t, r); }
     R0 = vfma(b0, c, vscale(b1, sn));
     R1 = vfma(b1, c, vscale(vneg(b0), sn));
 }
@@ -343,7 +352,7 @@ __device__ __forceinline__ V3 hinge_q_p(V3 e, float h2k, float nrest)
     if (MODE == kModeConsistent) {
         const float n2 = vdot(e, e);
         V3 p = V3{make_float2(0.f, 0.f), 0.f};
-        if (nrest > 1e-10f && n2 > 1e-20f) p = vscale(e, fmul(nrest, rsqrtf(n2)));
+        if (nrest > 1e-10f && n2 > 1e-20f) p = vscale(e, fmul(nrest, frsqrt(n2)));
         return vscale(vsub(p, e), h2k);
     }
     return v3(hinge_q<MODE>(f3(e), h2k, nrest));
@@ -532,6 +541,27 @@ __device__ __forceinline__ float3 gather_vm_p(int l, int j0, int j1, int npad, c
     #pragma unroll
     for (int i = 0; i < M; ++i)
         if (j0 + i < j1) { fx = fadd(fx, vxy[i].x); fy = fadd(fy, vxy[i].y); fz = fadd(fz, vz[i]); }
+    return make_float3(fx, fy, fz);
+}
+
+// gather_vm_p with the slot stride as a constant: the loads are at fixed
+// distances from one address (cxy, cz: the first contribution's slot, n of
+// them), so the address arithmetic per slot goes.  Same sums.
+template <int M, int NPAD>
+__device__ __forceinline__ float3 gather_vm_c(int n, const float2* cxy, const float* cz)
+{
+    float2 vxy[M];
+    float vz[M];
+    #pragma unroll
+    for (int i = 0; i < M; ++i) {
+        vxy[i] = make_float2(0.f, 0.f);
+        vz[i] = 0.f;
+        if (i < n) { vxy[i] = cxy[i * NPAD]; vz[i] = cz[i * NPAD]; }
+    }
+    float fx = 0.f, fy = 0.f, fz = 0.f;
+    #pragma unroll
+    for (int i = 0; i < M; ++i)
+        if (i < n) { fx = fadd(fx, vxy[i].x); fy = fadd(fy, vxy[i].y); fz = fadd(fz, vz[i]); }
     return make_float3(fx, fy, fz);
 }
 

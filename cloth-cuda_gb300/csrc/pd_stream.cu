@@ -249,7 +249,15 @@ __device__ __forceinline__ void gather_halo(const IterArgs& a, const StreamArgs&
 // The register cap is set for 6 blocks of 128 threads per SM (80 registers,
 // no spills); measured on 1025x1025 and the 512-cloth batch it is about 1 %
 // faster than the cap for 5 (96 registers).
-template <int MODE, int NT>
+// LD: distance of d from y in a stage, in vertices, or 0 where it is a launch
+// argument; with a constant one address serves both loads of a corner.  NPAD:
+// the slot stride of a full patch (the last patch of a cloth may differ).
+// Measured with both constant: 1,155 warp instructions (x32) per vertex and
+// sweep instead of 1,250; 333x500 at 256/256 13.6 us instead of 14.5, 400x400
+// at 128/128 13.8 instead of 14.5, batches of 32 and 96 cloths 14.2 and 32.0
+// instead of 14.4 and 32.4; 1025x1025 57.1 (57.2): large grids wait for
+// records, not for issue slots.
+template <int MODE, int NT, int LD, int NPAD>
 __global__ void __launch_bounds__(NT, 768 / NT) k_stream(IterArgs a, StreamArgs sa, int k, int res_only)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -343,7 +351,7 @@ __global__ void __launch_bounds__(NT, 768 / NT) k_stream(IterArgs a, StreamArgs 
         if (tid == 32 && q < sa.npatch) decide(a, hring[(it + 1) % 3], q, k, res_only, &dec[s ^ 1]);
         const PatchDecision dp_ = dec[s];
         const float4* sy = reinterpret_cast<const float4*>(st + sa.o_y);
-        const float4* sd = reinterpret_cast<const float4*>(st + sa.o_d);
+        const float4* sd = LD ? sy + LD : reinterpret_cast<const float4*>(st + sa.o_d);
 
         // local step of patch p: records from global memory, contributions
         // to the vertex-major slots.  Odd rounds run in reverse thread order,
@@ -400,9 +408,14 @@ __global__ void __launch_bounds__(NT, 768 / NT) k_stream(IterArgs a, StreamArgs 
             for (int l = tid; l < nown; l += NT) {
                 const int deg = cp[l + 1] - cp[l];
                 const int hh = gather_half(deg);
-                const float3 f =
-                    deg <= 10 ? fadd3(gather_vm_p<5>(l, 0, hh, npad, cxy, cz), gather_vm_p<5>(l, hh, deg, npad, cxy, cz))
-                              : fadd3(gather_vm(l, 0, hh, npad, cxy, cz), gather_vm(l, hh, deg, npad, cxy, cz));
+                float3 f;
+                if (NPAD && deg <= 10 && npad == NPAD)
+                    f = fadd3(gather_vm_c<5, NPAD ? NPAD : 1>(hh, cxy + l, cz + l),
+                              gather_vm_c<5, NPAD ? NPAD : 1>(deg - hh, cxy + l + hh * NPAD, cz + l + hh * NPAD));
+                else if (deg <= 10)
+                    f = fadd3(gather_vm_p<5>(l, 0, hh, npad, cxy, cz), gather_vm_p<5>(l, hh, deg, npad, cxy, cz));
+                else
+                    f = fadd3(gather_vm(l, 0, hh, npad, cxy, cz), gather_vm(l, hh, deg, npad, cxy, cz));
                 const int g = vbegin + l;
                 const float4 d = sd[l];
                 const float4 y = sy[l];
@@ -422,44 +435,59 @@ __global__ void __launch_bounds__(NT, 768 / NT) k_stream(IterArgs a, StreamArgs 
     cp_async_wait_all();
 }
 
+namespace {
+
+// Constant distance of d from y (see k_stream), 0: none.  448 and 256 hold the
+// 390-404 and 235 local vertices of regular grids at 256 and 128 per patch and
+// keep three blocks of 256 threads, six of 128, on an SM.
+constexpr int stage_stride(int nt) { return nt == 256 ? 448 : (nt == 128 ? 256 : 0); }
+
+}  // namespace
+
 // Stage layout: every region starts on a 16-byte boundary.
-bool stream_layout(int max_nown, int max_nhalo, int max_nlocal, int max_vm_nslot, StreamArgs& sa, size_t& smem)
+bool stream_layout(int nt, int max_nown, int max_nhalo, int max_nlocal, int max_vm_nslot, StreamArgs& sa, size_t& smem)
 {
     auto r16 = [](size_t b) { return (b + 15) / 16 * 16; };
-    size_t o = 0;
-    sa.o_hidx = (int)o; o += r16(4 * (size_t)max_nhalo);
-    sa.o_ptr = (int)o;  o += r16(4 * (size_t)(max_nown + 1));
-    sa.o_y = (int)o;    o += 16 * (size_t)max_nlocal;
-    sa.o_d = (int)o;    o += 16 * (size_t)max_nlocal;
-    sa.o_dp = (int)o;   o += 16 * (size_t)max_nown;
-    o = (o + 127) / 128 * 128;
-    sa.stage_bytes = (int)o;
-    sa.slot_off = (int)(2 * o);
-    sa.max_nslot = max_vm_nslot;
-    smem = 2 * o + 12 * (size_t)max_vm_nslot;
-    return smem < (1u << 31);
+    // the constant distance pads y: only where the blocks an SM then holds are
+    // the register cap's (768 / nt) and every patch fits
+    const int ld = stage_stride(nt);
+    const size_t share = 227 * 1024 / (size_t)(768 / nt > 0 ? 768 / nt : 1) - 2048;
+    for (sa.fixed = ld && max_nlocal <= ld && max_nown <= nt ? 1 : 0;; sa.fixed = 0) {
+        size_t o = 0;
+        sa.o_hidx = (int)o; o += r16(4 * (size_t)max_nhalo);
+        sa.o_ptr = (int)o;  o += r16(4 * (size_t)(max_nown + 1));
+        sa.o_y = (int)o;    o += 16 * (size_t)(sa.fixed ? ld : max_nlocal);
+        sa.o_d = (int)o;    o += 16 * (size_t)max_nlocal;
+        sa.o_dp = (int)o;   o += 16 * (size_t)max_nown;
+        o = (o + 127) / 128 * 128;
+        sa.stage_bytes = (int)o;
+        sa.slot_off = (int)(2 * o);
+        sa.max_nslot = max_vm_nslot;
+        smem = 2 * o + 12 * (size_t)max_vm_nslot;
+        if (!sa.fixed || smem <= share) return smem < (1u << 31);
+    }
 }
 
-template <int MODE, int NT>
-static void* stream_ptr() { return (void*)k_stream<MODE, NT>; }
-
-static void* pick_stream(int mode, int nt)
+static void* pick_stream(int mode, int nt, int fixed)
 {
     if (mode == kModeConsistent) {
-        if (nt == 128) return stream_ptr<kModeConsistent, 128>();
-        if (nt == 256) return stream_ptr<kModeConsistent, 256>();
-        if (nt == 512) return stream_ptr<kModeConsistent, 512>();
+        if (nt == 128) return fixed ? (void*)k_stream<kModeConsistent, 128, stage_stride(128), 129>
+                                    : (void*)k_stream<kModeConsistent, 128, 0, 0>;
+        if (nt == 256) return fixed ? (void*)k_stream<kModeConsistent, 256, stage_stride(256), 257>
+                                    : (void*)k_stream<kModeConsistent, 256, 0, 0>;
+        if (nt == 512) return (void*)k_stream<kModeConsistent, 512, 0, 0>;
     } else {
-        if (nt == 128) return stream_ptr<kModeLiteral, 128>();
-        if (nt == 256) return stream_ptr<kModeLiteral, 256>();
-        if (nt == 512) return stream_ptr<kModeLiteral, 512>();
+        // (the reference-literal mode runs the general form: o_d is set either way)
+        if (nt == 128) return (void*)k_stream<kModeLiteral, 128, 0, 0>;
+        if (nt == 256) return (void*)k_stream<kModeLiteral, 256, 0, 0>;
+        if (nt == 512) return (void*)k_stream<kModeLiteral, 512, 0, 0>;
     }
     return nullptr;
 }
 
-int stream_max_blocks(int mode, int nt, size_t smem)
+int stream_max_blocks(int mode, int nt, int fixed, size_t smem)
 {
-    void* f = pick_stream(mode, nt);
+    void* f = pick_stream(mode, nt, fixed);
     if (!f) return 0;
     int dev = 0, nsm = 0, optin = 0, nb = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
@@ -474,7 +502,7 @@ int stream_max_blocks(int mode, int nt, size_t smem)
 cudaError_t launch_stream(const IterArgs& a, const StreamArgs& sa, int mode, int nt, int grid, size_t smem, int k,
                           int res_only, cudaStream_t s, bool after_sweep)
 {
-    void* f = pick_stream(mode, nt);
+    void* f = pick_stream(mode, nt, sa.fixed);
     if (!f || grid <= 0) return cudaErrorInvalidValue;
     IterArgs ac = a;
     StreamArgs sc = sa;

@@ -122,11 +122,12 @@ struct StreamArgs {
     int slot_off;
     int max_nslot;          // vertex-major slots per patch (largest)
     int npatch;
+    int fixed;              // stage with the plan's constant distance of d from y
     int* err;               // set when a copy wait times out
     long long spin_budget;  // clock64 cycles a wait may take
 };
-bool stream_layout(int max_nown, int max_nhalo, int max_nlocal, int max_vm_nslot, StreamArgs& sa, size_t& smem);
-int stream_max_blocks(int mode, int nt, size_t smem);
+bool stream_layout(int nt, int max_nown, int max_nhalo, int max_nlocal, int max_vm_nslot, StreamArgs& sa, size_t& smem);
+int stream_max_blocks(int mode, int nt, int fixed, size_t smem);
 // after_sweep: the previous launch on the stream is a sweep of this kernel;
 // the launch then overlaps its tail (programmatic dependent launch).
 cudaError_t launch_stream(const IterArgs& a, const StreamArgs& sa, int mode, int nt, int grid, size_t smem, int k,
