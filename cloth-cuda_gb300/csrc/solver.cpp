@@ -274,6 +274,33 @@ int launches_per_frame(const pdg_solver* s)
     return 4 + (s->range_variant >= 0 ? 1 : s->L.cap + (s->have_final ? 1 : 0));
 }
 
+// Patches of at most pv vertices over these cloths.
+long long patch_count(const std::vector<ClothSetup>& cl, int pv)
+{
+    long long n = 0;
+    for (const auto& c : cl) n += (c.mesh->N + pv - 1) / pv;
+    return n;
+}
+
+// Patch size of the streaming plan on 256 threads when the caller leaves it
+// open: 256 vertices, or 192 where these fill the last wave of blocks better.
+// A wave holds 3 blocks per SM.  A 256-vertex patch (335 cells, two rounds of
+// the threads) took about 6.1 us, a 192-vertex one (255 cells, one round) 4.85
+// us; a part-filled last wave counts half of what it leaves empty, because the
+// next sweep's blocks start in it.  The rule picks the measured best on
+// 300x300 (256: 8.1 against 9.2 us per sweep), 333x500 (192: 11.8 against
+// 13.6), 400x400 (192: 12.4 against 13.9), 700x700 (256: 29.1 against 31.0),
+// 1025x1025 (256: 57.1 against 59.7) and batches of 32 and 96 cloths (256:
+// 14.2 against 16.5, 32.0 against 35.0); 513x513 keeps 256 (18.1 against 17.4).
+int stream_patch_verts(const std::vector<ClothSetup>& cl, int nsm)
+{
+    auto cost = [&](int pv, double us) {
+        const double w = (double)patch_count(cl, pv) / (3.0 * nsm);
+        return us * (w <= 1.0 ? 1.0 : 0.5 * (std::ceil(w) + w));
+    };
+    return cost(192, 4.85) < cost(256, 6.1) ? 192 : 256;
+}
+
 int build_graph(pdg_solver* s)
 {
     if (s->graph) { cudaGraphExecDestroy(s->graph); s->graph = nullptr; }
@@ -363,7 +390,8 @@ int pdg::create_solver(int n, const pdg_config* cfgs, const pdg_mesh* const* mes
         for (const auto& c : s->cloths) ntot += c.mesh->N;
         int P = c0.patch_verts;
         if (!P) P = std::min(rnt, std::max(32, ((ntot + per_sm * nsm - 1) / (per_sm * nsm) + 31) / 32 * 32));
-        bool ok = P <= rnt && build_layout(s->cloths, P, s->L, err);
+        // (more patches than blocks cannot fit: no layout is built for them)
+        bool ok = P <= rnt && patch_count(s->cloths, P) <= (long long)per_sm * nsm && build_layout(s->cloths, P, s->L, err);
         int variant = -1;
         if (ok) {
             variant = resident_pick(rnt);
@@ -383,9 +411,12 @@ int pdg::create_solver(int n, const pdg_config* cfgs, const pdg_mesh* const* mes
                 if (c.cfg.tolerance > 0.f) s->nbr_sync = 0;
         } else if (c0.kernel == PDG_KERNEL_RESIDENT) {
             return set_error(PDG_ERR_ARG, "resident kernel does not fit this problem (%d patches of %d vertices)",
-                             s->L.npatch, P);
+                             (int)patch_count(s->cloths, P), P);
         }
     }
+    // (a learned start sums its messages in layout order: its plan stays)
+    if (s->kernel == PDG_KERNEL_STREAM && !c0.patch_verts && !c0.block_threads && !s->any_warm)
+        s->patch_verts = stream_patch_verts(s->cloths, nsm);
     for (; s->kernel != PDG_KERNEL_RESIDENT;) {
         if (!build_layout(s->cloths, s->patch_verts, s->L, err)) return set_error(PDG_ERR_ARG, "%s", err.c_str());
         if (s->kernel == PDG_KERNEL_STREAM) {
