@@ -246,6 +246,22 @@ __device__ __forceinline__ void gather_halo(const IterArgs& a, const StreamArgs&
     cp_async_commit();
 }
 
+// One thread: the sum of a patch's NT / 32 warp sums, in the order of a block
+// sum (halves folded onto each other), added to its cloth's accumulator of
+// sweep k (cloth < 0: none).
+template <int NT>
+__device__ __forceinline__ void add_residual(const IterArgs& a, const float* red, int cloth, int k)
+{
+    float v[NT / 32];
+    #pragma unroll
+    for (int i = 0; i < NT / 32; ++i) v[i] = red[i];
+    #pragma unroll
+    for (int o = NT / 64; o > 0; o >>= 1)
+        #pragma unroll
+        for (int i = 0; i < o; ++i) v[i] += v[i + o];
+    if (cloth >= 0) atomicAdd(a.acc + (size_t)cloth * a.acc_stride + k, (double)v[0]);
+}
+
 // The register cap is set for 6 blocks of 128 threads per SM (80 registers,
 // no spills); measured on 1025x1025 and the 512-cloth batch it is about 1 %
 // faster than the cap for 5 (96 registers).
@@ -255,8 +271,11 @@ __device__ __forceinline__ void gather_halo(const IterArgs& a, const StreamArgs&
 // Measured with both constant: 1,155 warp instructions (x32) per vertex and
 // sweep instead of 1,250; 333x500 at 256/256 13.6 us instead of 14.5, 400x400
 // at 128/128 13.8 instead of 14.5, batches of 32 and 96 cloths 14.2 and 32.0
-// instead of 14.4 and 32.4; 1025x1025 57.1 (57.2): large grids wait for
-// records, not for issue slots.
+// instead of 14.4 and 32.4; 1025x1025 57.1 (57.2).
+// A patch takes two block barriers (after its cells, and where the stages
+// change): its residual is added one patch later by a single thread.  With a
+// third barrier in the residual's block sum the 1025x1025 sweep took 57.1 us,
+// now 55.0; 96 cloths 32.2, now 30.7.
 template <int MODE, int NT, int LD, int NPAD>
 __global__ void __launch_bounds__(NT, 768 / NT) k_stream(IterArgs a, StreamArgs sa, int k, int res_only)
 {
@@ -264,7 +283,8 @@ __global__ void __launch_bounds__(NT, 768 / NT) k_stream(IterArgs a, StreamArgs 
     __shared__ __align__(8) uint64_t bar[3];   // the two stages; the first patch's static lists
     __shared__ __align__(16) PatchHdr hring[3];
     __shared__ PatchDecision dec[2];
-    __shared__ float red[NT / 32];
+    __shared__ float red[2][NT / 32];
+    __shared__ int cloth_prev[2];   // whose residual is in red, -1: none
     const int tid = threadIdx.x;
     const int G = gridDim.x;
     const float4* __restrict__ Dk = (k & 1) ? a.buf[1] : a.buf[0];
@@ -338,6 +358,9 @@ __global__ void __launch_bounds__(NT, 768 / NT) k_stream(IterArgs a, StreamArgs 
         // and the slots are free
         cp_async_wait_all();
         __syncthreads();
+        // the residual of the patch before: one thread adds its warps' sums
+        // while the others go on (in the order of a block sum)
+        if (MODE == kModeConsistent && it > 0 && tid == 64) add_residual<NT>(a, red[s ^ 1], cloth_prev[s ^ 1], k);
         const PatchHdr& h = hring[it % 3];
         if (tid == 0 && q < sa.npatch) {
             const PatchHdr& hq = hring[(it + 1) % 3];
@@ -376,13 +399,15 @@ __global__ void __launch_bounds__(NT, 768 / NT) k_stream(IterArgs a, StreamArgs 
             }
         }
 
-        // patch q's lists have landed (or the wait gave up) and every
-        // thread's contributions to p's slots are stored: one barrier
+        // Patch q's lists have landed (or the wait gave up); its halo is
+        // fetched before the barrier that ends p's cells, by the first
+        // threads, which are the ones without a cell in the last round.
         const int b1 = s ^ 1;
         bool got = true;
         if (q < sa.npatch) {
             got = mbar_wait(&bar[b1], (parity >> b1) & 1u, sa.spin_budget);
             parity ^= 1u << b1;
+            if (got) gather_halo(a, sa, Dk, hring[(it + 1) % 3], st1, tid, NT);
         }
         if (!__syncthreads_and(got)) {
             // give up: record the error, let copies in flight land, leave
@@ -396,9 +421,6 @@ __global__ void __launch_bounds__(NT, 768 / NT) k_stream(IterArgs a, StreamArgs 
             __syncthreads();
             return;
         }
-        // patch q's halo, gathered while patch p is finished
-        if (q < sa.npatch) gather_halo(a, sa, Dk, hring[(it + 1) % 3], st1, tid, NT);
-
         // global step of patch p
         if (!dp_.skip) {
             const int nown = h.nown, vbegin = h.vbegin, npad = h.vm_npad;
@@ -429,10 +451,16 @@ __global__ void __launch_bounds__(NT, 768 / NT) k_stream(IterArgs a, StreamArgs 
                     Dn[g] = update_literal(d, y, f);
                 }
             }
-            if (MODE == kModeConsistent) block_residual<NT>(r2, red, a.acc + (size_t)h.cloth * a.acc_stride + k);
+            if (MODE == kModeConsistent) {
+                r2 = warp_sum(r2);
+                if ((tid & 31) == 0) red[s][tid >> 5] = r2;
+            }
         }
+        if (MODE == kModeConsistent && tid == 0) cloth_prev[s] = dp_.skip ? -1 : h.cloth;
     }
     cp_async_wait_all();
+    __syncthreads();
+    if (MODE == kModeConsistent && tid == 64) add_residual<NT>(a, red[(it & 1) ^ 1], cloth_prev[(it & 1) ^ 1], k);
 }
 
 namespace {
