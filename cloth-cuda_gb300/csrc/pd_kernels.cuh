@@ -797,26 +797,30 @@ __device__ __forceinline__ void reset_rt(ClothRT* crt, double* acc, int acc_stri
     for (int k = t0; k < acc_stride; k += nt) acc[(size_t)c * acc_stride + k] = 0.0;
 }
 
-// y = x + h v + h^2 a (w = mass); start offset d^0 = x^0 - y into both
-// buffers (w = inverse diagonal, -1 for pinned vertices).
-__device__ __forceinline__ void predict_vertex_xv(int i, float4 x, float4 v, const float4* aux, const float* mass,
-                                                  const int* vcloth, const ClothInfo* cinfo, const float4* warm,
-                                                  float4* Y, float4* A, float4* B)
+// y = x + h v + h^2 a (w = mass) and the start offset d^0 = x^0 - y (w =
+// inverse diagonal, -1 for pinned vertices) of one vertex.
+__device__ __forceinline__ void predict_values(float4 x, float4 v, float4 au, float mass, const ClothInfo& ci,
+                                               const float4* warm, int i, float4& y, float4& s)
 {
-    const ClothInfo& ci = cinfo[vcloth[i]];
     const float h = ci.h, h2 = fmul(h, h);
-    const float4 au = __ldcg(&aux[i]);
-    float4 y;
     y.x = ffma(h2, ci.ext[0], ffma(h, v.x, x.x));
     y.y = ffma(h2, ci.ext[1], ffma(h, v.y, x.y));
     y.z = ffma(h2, ci.ext[2], ffma(h, v.z, x.z));
-    y.w = mass[i];
-    Y[i] = y;
-    float4 s;
+    y.w = mass;
     if (au.w < 0.f)                    s = make_float4(fsub(au.x, y.x), fsub(au.y, y.y), fsub(au.z, y.z), au.w);
     else if (ci.init == 1)             s = make_float4(fsub(x.x, y.x), fsub(x.y, y.y), fsub(x.z, y.z), au.w);
     else if (ci.init >= 2 && warm) {   const float4 w = __ldcg(&warm[i]); s = make_float4(w.x, w.y, w.z, au.w); }
     else                               s = make_float4(0.f, 0.f, 0.f, au.w);
+}
+
+// The same, stored: y, and d^0 into both iterate buffers.
+__device__ __forceinline__ void predict_vertex_xv(int i, float4 x, float4 v, const float4* aux, const float* mass,
+                                                  const int* vcloth, const ClothInfo* cinfo, const float4* warm,
+                                                  float4* Y, float4* A, float4* B)
+{
+    float4 y, s;
+    predict_values(x, v, __ldcg(&aux[i]), mass[i], cinfo[vcloth[i]], warm, i, y, s);
+    Y[i] = y;
     A[i] = s;
     B[i] = s;
 }
@@ -828,74 +832,95 @@ __device__ __forceinline__ void predict_vertex(int i, const float4* X, const flo
     predict_vertex_xv(i, __ldcg(&X[i]), __ldcg(&V[i]), aux, mass, vcloth, cinfo, warm, Y, A, B);
 }
 
-// Cloths still active after the last sweep keep x^max_iter.  A non-finite
-// per-sweep sum marks the cloth as failed (sweeps that ran with neighbour
-// synchronisation skip the per-sweep check).  One warp per cloth: its lanes
-// look through the sums together.  (One thread reading them one after another
-// took 0.3 us per sweep of the cap: 61 us of a 200-sweep frame.)
-__device__ __forceinline__ void frame_stats_cloth(const IterArgs& a, int c)
+// Outcome of a cloth's frame.
+struct FrameEnd {
+    int used, status;
+};
+
+// The end of cloth c's frame, by one warp whose lanes look through the
+// per-sweep sums `acc` together (one thread reading them one after another
+// took 0.3 us per sweep of the cap, 61 us of a 200-sweep frame).  `end`: the
+// outcome of a cloth that stopped before its cap (null: still active).  An
+// active cloth keeps x^max_iter; a non-finite sum marks it as failed (sweeps
+// that ran with neighbour synchronisation skip the per-sweep check).  With
+// `write` the cloth's record is completed; without, it is not looked at, so
+// that another block may write it at the same time.  Valid on every lane.
+__device__ __forceinline__ FrameEnd end_frame(const IterArgs& a, int c, const double* acc, const FrameEnd* stopped,
+                                              bool write)
 {
     ClothRT* rt = a.crt + c;
     const ClothInfo& ci = a.cinfo[c];
-    const double* acc = a.acc + (size_t)c * a.acc_stride;
     const int lane = threadIdx.x & 31;
     const bool consistent = ci.mode == kModeConsistent;
-    const int active = __ldcg(&rt->active);
-    bool finite = true;
-    if (consistent && active)
+    FrameEnd end{ci.max_iter, 0};
+    if (stopped) {
+        end = *stopped;
+    } else if (consistent) {
+        bool finite = true;
         for (int k = lane; k <= ci.max_iter && k < a.acc_stride; k += 32) {
             const double v = __ldcg(&acc[k]);
             finite = finite && isfinite(v);
         }
-    finite = __all_sync(0xffffffffu, finite) != 0;
-    if (lane != 0) return;
-    if (consistent) {
-        const double r0 = __ldcg(&acc[0]);
-        rt->res0_2 = r0;
-        if (!(ci.init >= 2 && a.warm_active)) rt->res_y2 = r0;
+        if (!__all_sync(0xffffffffu, finite)) end.status = -6;
     }
-    if (active) {
-        rt->used = ci.max_iter;
+    if (write && lane == 0) {
         if (consistent) {
-            const double rf = __ldcg(&acc[ci.max_iter]);
-            rt->resf_2 = a.have_final ? rf : -1.0;
-            if (!finite) rt->status = -6;
-        } else {
-            rt->resf_2 = -1.0;
+            const double r0 = __ldcg(&acc[0]);
+            rt->res0_2 = r0;
+            if (!(ci.init >= 2 && a.warm_active)) rt->res_y2 = r0;
         }
-        rt->active = 0;
+        if (!stopped) {
+            rt->used = end.used;
+            rt->resf_2 = consistent && a.have_final ? __ldcg(&acc[ci.max_iter]) : -1.0;
+            if (end.status != 0) rt->status = end.status;
+            rt->active = 0;
+        }
     }
+    return end;
+}
+
+// The same where the record says whether the cloth stopped.
+__device__ __forceinline__ void frame_stats_cloth(const IterArgs& a, int c)
+{
+    const ClothRT* rt = a.crt + c;
+    const FrameEnd end{__ldcg(&rt->used), __ldcg(&rt->status)};
+    end_frame(a, c, a.acc + (size_t)c * a.acc_stride, __ldcg(&rt->active) ? nullptr : &end, true);
 }
 
 // x = y + d^used; v = (x - x_n)(1 - damping)/h, formed without cancellation
 // as (1 - damping)(v_n + h a + d/h) since x - x_n = h v_n + h^2 a + d.
 // Pins go to their target with v = 0.  A cloth whose solve produced
 // NaN/Inf keeps x_n and gets v = 0.
-__device__ __forceinline__ void finalize_vertex(int i, float4* X, float4* V, const float4* Y, const float4* A,
-                                                const float4* B, const float4* aux, const int* vcloth,
-                                                const ClothInfo* cinfo, const ClothRT* crt)
+__device__ __forceinline__ void finalize_vertex(int i, FrameEnd end, const ClothInfo& ci, float4* X, float4* V,
+                                                const float4* Y, const float4* A, const float4* B, const float4* aux)
 {
-    const int c = vcloth[i];
-    const ClothInfo& ci = cinfo[c];
-    const int status = __ldcg(&crt[c].status);
-    const int used = __ldcg(&crt[c].used);
     const float4 au = __ldcg(&aux[i]);
     if (au.w < 0.f) {
         X[i] = make_float4(au.x, au.y, au.z, 0.f);
         V[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         return;
     }
-    if (status != 0) {
+    if (end.status != 0) {
         V[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         return;
     }
-    const float4 d = (used & 1) ? __ldcg(&B[i]) : __ldcg(&A[i]);
+    const float4 d = (end.used & 1) ? __ldcg(&B[i]) : __ldcg(&A[i]);
     const float4 y = __ldcg(&Y[i]);
     const float4 v = __ldcg(&V[i]);
     const float h = ci.h, sc = 1.f - ci.damping, ih = fdiv(1.f, h);
     V[i] = make_float4(fmul(sc, ffma(d.x, ih, ffma(h, ci.ext[0], v.x))), fmul(sc, ffma(d.y, ih, ffma(h, ci.ext[1], v.y))),
                        fmul(sc, ffma(d.z, ih, ffma(h, ci.ext[2], v.z))), 0.f);
     X[i] = make_float4(fadd(y.x, d.x), fadd(y.y, d.y), fadd(y.z, d.z), 0.f);
+}
+
+// The same, its cloth's outcome read from the record.
+__device__ __forceinline__ void finalize_vertex(int i, float4* X, float4* V, const float4* Y, const float4* A,
+                                                const float4* B, const float4* aux, const int* vcloth,
+                                                const ClothInfo* cinfo, const ClothRT* crt)
+{
+    const int c = vcloth[i];
+    const FrameEnd end{__ldcg(&crt[c].used), __ldcg(&crt[c].status)};
+    finalize_vertex(i, end, cinfo[c], X, V, Y, A, B, aux);
 }
 
 }  // namespace pdg

@@ -33,27 +33,28 @@
 
 namespace pdg {
 
-// Barrier `phase` (1, 2, ...) of the frame: one arrival per block on a count
-// that only grows (cleared before the frame), polled until every block of the
-// phase is in.  False once a wait, here or in another block, gave up.
-__device__ __forceinline__ bool grid_barrier_r(unsigned* bar, int* err, long long budget, unsigned& phase)
+// Barrier over the grid on a 64-bit count of arrivals that is never reset:
+// every barrier adds gridDim.x, so a block's own arrival number tells which
+// count ends its barrier.  False once a wait, here or in another block, gave
+// up (the host then clears the count when it reports the error).
+__device__ __forceinline__ bool grid_barrier_r(unsigned* bar, int* err, long long budget)
 {
     __shared__ int ok;
     __syncthreads();
-    ++phase;
     if (threadIdx.x == 0) {
-        const unsigned want = phase * gridDim.x;
+        unsigned long long* cnt = reinterpret_cast<unsigned long long*>(bar);
         __threadfence();
-        atomicAdd(bar, 1u);
-        unsigned v;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(__cvta_generic_to_global(bar)) : "memory");
+        const unsigned long long old = atomicAdd(cnt, 1ull);
+        const unsigned long long want = (old / gridDim.x + 1ull) * gridDim.x;
+        unsigned long long v = old + 1ull;
         if (v < want) {
             const long long t0 = clock64();
             do {
-                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(__cvta_generic_to_global(bar)) : "memory");
+                asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(__cvta_generic_to_global(cnt)) : "memory");
                 if (v < want && (clock64() - t0 > budget || *(volatile int*)err != 0)) { atomicCAS(err, 0, 2); break; }
             } while (v < want);
         }
+        __threadfence();
         ok = (v >= want && *(volatile int*)err == 0);
     }
     __syncthreads();
@@ -246,7 +247,7 @@ __device__ __forceinline__ void compute_residual(float r2, float* red, double* a
 // RANGE (with TOL): sweeps p.k0 .. p.k1 - 1 of a frame whose prediction, start
 // and finalisation are other launches: the streaming plan's sweeps where its
 // patches all fit on the chip at once.  At 54,000 vertices in 128-vertex
-// patches a sweep takes 5.3 us, as launches of the streaming kernel 7.3 us.
+// patches a sweep takes 4.8 us, as launches of the streaming kernel 7.3 us.
 template <int MODE, int NT, bool IO, bool TOL, bool RANGE>
 __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistArgs p)
 {
@@ -258,7 +259,8 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
     __shared__ int dec[2];             // TOL: decision, 0 go on, 1 stop, 2 leave (a wait ran out)
     __shared__ int gone;               // TOL: the compute threads left early
     __shared__ int over;               // RANGE: the cloth is done before the range
-    unsigned phase = 0;                // grid barriers so far
+    __shared__ FrameEnd end_s;         // outcome of this cloth's frame; TOL: set early when it stops
+    __shared__ int stopped;            // TOL: it did
     __shared__ float som[kResOmega];   // Chebyshev weights of this cloth
     const IterArgs& a = p.it;
     const int tid = threadIdx.x;
@@ -322,12 +324,49 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
     const int g = ph.vbegin + tid;
     float4 dprev = make_float4(0.f, 0.f, 0.f, 0.f);
     const int k0 = RANGE ? p.k0 : 0;   // first sweep
+    // The per-sweep sums (and arrivals) of a whole frame come in two sets: a
+    // frame uses the one that p.frame's parity names and clears the other, so
+    // that no block needs to wait for the clearing.  (A range uses the sums
+    // that the frame's first launch cleared.)
+    const unsigned par = RANGE ? 0u : __ldcg(p.frame) & 1u;
+    const size_t set = (size_t)a.ncloth * a.acc_stride;
+    double* acc = a.acc + (RANGE ? 0 : par * set) + (size_t)c * a.acc_stride;
+    int* cnt = TOL ? p.cnt + par * set + (size_t)c * a.acc_stride : nullptr;
     if (first) {
-        if (!RANGE) reset_rt(a.crt, a.acc, a.acc_stride, c, tid, NTT);
-        if (TOL)
-            for (int k = tid; k < a.acc_stride; k += NTT) p.cnt[(size_t)c * a.acc_stride + k] = 0;
+        if (!RANGE && tid == 0) {
+            ClothRT r;
+            r.active = 1; r.used = 0; r.status = 0; r.warm = 0;
+            r.res_y2 = 0.0; r.res0_2 = 0.0; r.resf_2 = -1.0;
+            a.crt[c] = r;
+        }
+        for (int k = tid; k < a.acc_stride; k += NTT) {
+            if (!RANGE) a.acc[(par ^ 1u) * set + (size_t)c * a.acc_stride + k] = 0.0;
+            if (TOL) p.cnt[(RANGE ? 0u : par ^ 1u) * set + (size_t)c * a.acc_stride + k] = 0;
+        }
     }
-    if (TOL && tid == 0) gone = 0;
+    if (TOL && tid == 0) { gone = 0; stopped = 0; }
+    // The frame's exchange tags: tag0 + k for d^k, tag0 from the device word
+    // that the previous frame advanced (so a replayed launch gets new tags).
+    // Before the 32-bit tags would wrap, every block clears its boundary
+    // vertices' words in both buffers and the frame starts again from 0, after
+    // a grid barrier that orders the clearing before any neighbour's poll.
+    const int nsweep = RANGE ? p.k1 : p.max_iter + (p.have_final ? 1 : 0);   // end of the sweeps
+    unsigned tag0 = __ldcg(p.xch_tag);
+    const bool wrap = (unsigned long long)tag0 + (unsigned long long)nsweep > 0xffffffffULL;
+    if (wrap) {
+        tag0 = 0;
+        for (int q = tid; q < 8 * ph.nbnd; q += NTT) {
+            const int l = q >> 3, b = (q >> 2) & 1, w = q & 3;
+            p.xch[((size_t)b * (size_t)p.n + (size_t)(ph.vbegin + l)) * 4 + w] = 0ull;
+        }
+    }
+    // Prediction.  A block predicts its halo vertices too: the state is not
+    // written before every block has met the barrier after the sweeps, so no
+    // block waits for another's prediction.  (With a barrier after the owners'
+    // prediction, and one more between the record and the finalisation, a
+    // 33x33 frame of 10 sweeps took 43.0 us, now 36.9.)  With caller arrays
+    // the vertices are walked in caller order, a grid stride over the compute
+    // threads, and the halo is read after a barrier.
     if (RANGE) {
         // the decision about the sweep before the range, the same in every
         // block of the cloth; all have taken it when the barrier below opens
@@ -337,36 +376,31 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
         if (comp && o0 < p.n) predict_caller_vertex(p, gi0, xi0, vi0);
         for (int o = o0 + (int)gridDim.x * NT; comp && o < p.n; o += (int)gridDim.x * NT)
             predict_caller_vertex(p, __ldg(&p.io_inv[o]), caller_vec(p.in_x, o), caller_vec(p.in_v, o));
-    } else if (own) {
-        predict_vertex(g, p.X, p.V, p.aux, p.mass, p.vcloth, a.cinfo, p.warm, p.Y, a.buf[0], a.buf[1]);
-        dprev = __ldcg(&a.buf[0][g]);
-    }
-    // The frame's exchange tags: tag0 + k for d^k, tag0 from the device word
-    // that the previous frame advanced (so a replayed launch gets new tags).
-    // Before the 32-bit tags would wrap, every block clears its boundary
-    // vertices' words in both buffers and the frame starts again from 0; the
-    // grid barrier below orders the clearing before any neighbour's poll.
-    const int nsweep = RANGE ? p.k1 : p.max_iter + (p.have_final ? 1 : 0);   // end of the sweeps
-    unsigned tag0 = 0;
-    if (p.xch_tag) {
-        const unsigned t = __ldcg(p.xch_tag);
-        if ((unsigned long long)t + (unsigned long long)nsweep <= 0xffffffffULL) {
-            tag0 = t;
-        } else {
-            for (int q = tid; q < 8 * ph.nbnd; q += NTT) {
-                const int l = q >> 3, b = (q >> 2) & 1, w = q & 3;
-                p.xch[((size_t)b * (size_t)p.n + (size_t)(ph.vbegin + l)) * 4 + w] = 0ull;
+    } else {
+        for (int l = tid; l < nlocal; l += NTT) {
+            const int gg = l < nown ? ph.vbegin + l : __ldg(&a.halo[ph.halo_off + l - nown]);
+            float4 y, s;
+            predict_values(__ldcg(&p.X[gg]), __ldcg(&p.V[gg]), __ldcg(&p.aux[gg]), __ldg(&p.mass[gg]), ci, p.warm, gg, y, s);
+            sy[l] = y;
+            sd[l] = s;
+            if (l < nown) {
+                p.Y[gg] = y;
+                a.buf[0][gg] = s;
+                a.buf[1][gg] = s;
+                if (l == tid) dprev = s;
             }
         }
     }
-    if (!grid_barrier_r(p.bar, p.err, p.spin_budget, phase)) return;
-    // every block has read the word: the next frame's base
-    if (p.xch_tag && blockIdx.x == 0 && tid == 0) *p.xch_tag = tag0 + (unsigned)nsweep;
-    if (caller_in && own) dprev = __ldcg(&a.buf[0][g]);
-    for (int l = tid; l < nlocal; l += NTT) {
-        const int gg = l < nown ? ph.vbegin + l : __ldg(&a.halo[ph.halo_off + l - nown]);
-        sy[l] = __ldcg(&a.Y[gg]);
-        sd[l] = __ldcg(&(RANGE && (k0 & 1) ? a.buf[1] : a.buf[0])[gg]);
+    if ((RANGE || caller_in || wrap) && !grid_barrier_r(p.bar, p.err, p.spin_budget)) return;
+    if (RANGE || caller_in) {
+        // (the barrier: every block of a range has read the tag word)
+        if (RANGE && blockIdx.x == 0 && tid == 0) *p.xch_tag = tag0 + (unsigned)nsweep;
+        if (caller_in && own) dprev = __ldcg(&a.buf[0][g]);
+        for (int l = tid; l < nlocal; l += NTT) {
+            const int gg = l < nown ? ph.vbegin + l : __ldg(&a.halo[ph.halo_off + l - nown]);
+            sy[l] = __ldcg(&a.Y[gg]);
+            sd[l] = __ldcg(&(RANGE && (k0 & 1) ? a.buf[1] : a.buf[0])[gg]);
+        }
     }
     // this compute thread's first halo vertex, re-read every sweep
     const int hl0 = nown + tid;
@@ -374,9 +408,14 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
     __syncthreads();
 
     const float gamma = ci.gamma;
-    double* acc = a.acc + (size_t)c * a.acc_stride;
+    // TOL: kept in a register, because the acquiring loads of the spare warp
+    // empty L1 and the reloads would miss it (129x129 to a tolerance 597 ->
+    // 520 us per 200 sweeps).  Otherwise the reloads hit, and the instances
+    // with the register were slower (65x65 111 -> 123 us per 50 sweeps).
+    const int max_iter_r = TOL ? ci.max_iter : 0;
+    auto max_iter = [&]() { return TOL ? max_iter_r : ci.max_iter; };
     // TOL: the end of this cloth's sweeps
-    const int kend = RANGE && over ? k0 : min(nsweep, ci.max_iter + 1);
+    const int kend = RANGE && over ? k0 : min(nsweep, max_iter() + 1);
     if (comp) {
         // ---- compute threads ----
         float4 dpp = make_float4(0.f, 0.f, 0.f, 0.f);   // TOL: own d^(k-2)
@@ -401,7 +440,7 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
                     break;
                 }
             }
-            if (k > k0 && k <= ci.max_iter) {
+            if (k > k0 && k <= max_iter()) {
                 // the neighbours' d^k (written in their sweep k - 1, which
                 // every sweep up to the cloth's cap has): poll the tagged
                 // words of this thread's halo vertices
@@ -433,10 +472,10 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
                 named_sync(1, NT);
             }
             // the cap alone decides: the cloth's record stays active through the sweeps
-            const bool skip_k = k >= ci.max_iter && (k > ci.max_iter || !a.have_final);
+            const bool skip_k = k >= max_iter() && (k > max_iter() || !a.have_final);
             const float omega_k =
                 k < a.omega_stride ? (k < kResOmega ? som[k] : a.omega[c * a.omega_stride + k]) : 1.f;
-            const bool res_only = k >= ci.max_iter;
+            const bool res_only = k >= max_iter();
             float4 o = make_float4(0.f, 0.f, 0.f, 0.f), d = o;
             float r2 = 0.f;
             // Phase A: the records through boundary vertices (a prefix of
@@ -469,7 +508,7 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
                                             cz, (ncell - ph.ncell_a) + (nhin - ph.nhin_a) <= 32);
                 named_sync(1, NT);
             }
-            if (k + 1 < nsweep && k + 1 <= ci.max_iter && hl0 < nlocal)
+            if (k + 1 < nsweep && k + 1 <= max_iter() && hl0 < nlocal)
                 ld_words(p.xch + ((size_t)((k + 1) & 1) * (size_t)p.n + hg0) * 4, pw0, pw1, pw2);
             if (!skip_k && own && tid >= ph.nbnd) {
                 vertex_update<MODE>(npad, sptr, tid, sy, sd, cxy, cz, dprev, gamma, omega_k, o, d, r2);
@@ -486,7 +525,7 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
                 r2 = warp_sum(r2);
                 if ((tid & 31) == 0) red[k & 1][tid >> 5] = r2;
                 named_arrive(2 + (k & 1), NTT);
-            } else if (MODE == kModeConsistent && !skip_k && (k == 0 || k >= ci.max_iter - 1)) {
+            } else if (MODE == kModeConsistent && !skip_k && (k == 0 || k >= max_iter() - 1)) {
                 // fixed sweep counts read only the residual of the start and
                 // of the last sweeps
                 compute_residual<NT>(r2, red[0], acc + k);
@@ -496,11 +535,10 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
             // the last decision, about sweep kend - 2; the last sweep may have
             // only evaluated the residual
             named_sync(4 + (kend & 1), NTT);
-            if (dec[kend & 1] == 1 && own && kend - 1 < ci.max_iter) ((kend & 1) ? a.buf[1] : a.buf[0])[g] = dpp;
+            if (dec[kend & 1] == 1 && own && kend - 1 < max_iter()) ((kend & 1) ? a.buf[1] : a.buf[0])[g] = dpp;
         }
     } else if (TOL) {
         // ---- the spare warp: residual sums and decisions ----
-        int* cnt = p.cnt + (size_t)c * a.acc_stride;
         const int npc = ci.patch_end - ci.patch_begin;
         const int lane = tid & 31;
         // waits for the complete sum of sweep j; false when a wait ran out
@@ -535,6 +573,8 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
                         const bool bad = !isfinite(rk2);
                         if (bad || (tol > 0.f && rk2 <= (double)tol * (double)tol * ry2)) {
                             go = 1;
+                            end_s = FrameEnd{j, bad ? -6 : 0};
+                            stopped = 1;
                             if (first) {
                                 ClothRT* rt = a.crt + c;
                                 if (RANGE) {
@@ -571,24 +611,34 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
         }
         // a cloth whose cap lies inside the range: its record, as the sweep
         // after its last one would have left it
-        const int kq = ci.max_iter + (a.have_final ? 1 : 0);
+        const int kq = max_iter() + (a.have_final ? 1 : 0);
         if (RANGE && first && lane == 0 && !ended && kend > k0 && kq < nsweep && complete(kend - 1))
             cloth_done(a, c, kq, true, true);
     }
     if (RANGE) return;
-    // every per-sweep sum is complete after this barrier
-    if (!grid_barrier_r(p.bar, p.err, p.spin_budget, phase)) return;
-    if (first && tid < 32) frame_stats_cloth(a, c);
-    if (!grid_barrier_r(p.bar, p.err, p.spin_budget, phase)) return;
+    // every per-sweep sum is complete after this barrier, and every block has
+    // read the frame's words
+    if (!grid_barrier_r(p.bar, p.err, p.spin_budget)) return;
+    if (blockIdx.x == 0 && tid == 0) {
+        *p.xch_tag = tag0 + (unsigned)nsweep;
+        *p.frame = par ^ 1u;
+    }
+    if (tid < 32) {
+        const FrameEnd end = end_frame(a, c, acc, TOL && stopped ? &end_s : nullptr, first);
+        if (tid == 0) end_s = end;
+    }
     if (caller_out) {
+        // (vertices of any cloth: their records)
+        if (!grid_barrier_r(p.bar, p.err, p.spin_budget)) return;
         for (int o = o0; comp && o < p.n; o += (int)gridDim.x * NT) {
             const int gv = __ldg(&p.io_inv[o]);
             finalize_vertex(gv, p.Xw, p.V, p.Y, a.buf[0], a.buf[1], p.aux, p.vcloth, a.cinfo, a.crt);
             store_frame_state(p, o, gv);
         }
-    } else if (own) {
-        finalize_vertex(g, p.Xw, p.V, p.Y, a.buf[0], a.buf[1], p.aux, p.vcloth, a.cinfo, a.crt);
+        return;
     }
+    __syncthreads();
+    if (own) finalize_vertex(g, end_s, ci, p.Xw, p.V, p.Y, a.buf[0], a.buf[1], p.aux);
 }
 
 // NT compute threads plus one warp: 480 + 32 threads, one block (one patch)
@@ -681,8 +731,6 @@ cudaError_t launch_resident_range(const PersistArgs& p, int variant, int grid, s
     const ResVariant* v = res_variants(&n);
     if (variant < 0 || variant >= n || grid <= 0) return cudaErrorInvalidValue;
     if (p.k1 <= p.k0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(p.bar, 0, 2 * sizeof(unsigned), s);
-    if (e != cudaSuccess) return e;
     PersistArgs copy = p;
     void* args[] = {&copy};
     return cudaLaunchCooperativeKernel(v[variant].f[5], dim3(grid), dim3(v[variant].nt + 32), args, smem, s);

@@ -66,7 +66,7 @@ struct PersistArgs {
     int max_iter;        // largest cap over cloths
     int have_final;      // evaluate r(x) of the returned iterate
     int mode;
-    unsigned* bar;       // [0] arrive counter, [1] generation
+    unsigned* bar;       // persistent kernel: arrivals, generation; resident kernel: one 64-bit count
     int* err;            // set when a grid barrier times out
     long long spin_budget;  // clock64 cycles a barrier may wait
     // neighbour synchronisation of the resident kernel (fixed sweep counts):
@@ -80,6 +80,7 @@ struct PersistArgs {
     // resident kernel, with a tolerance: per cloth and sweep (acc_stride
     // entries each) the patches that have added their part of the residual
     int* cnt;
+    unsigned* frame;     // resident kernel: parity of the frame's set of sums (it.acc and cnt hold two)
     int k0, k1;          // launch_resident_range: sweeps k0 .. k1 - 1
     // caller state moved inside the frame launch (resident kernel only): x, v
     // read by the prediction and written by the finalisation, AoS xyz in

@@ -81,19 +81,20 @@ int upload_all(pdg_solver* s)
     CK(s->cinfo.upload(L.cinfo, st));
     CK(s->crt.alloc(L.ncloth));
     s->acc_stride = L.cap + 4;   // sweeps 0..cap, then r(y) and r(learned start)
-    CK(s->acc.alloc((size_t)L.ncloth * s->acc_stride));
-    CK(cudaMemsetAsync(s->acc.p, 0, sizeof(double) * (size_t)L.ncloth * s->acc_stride, st));
+    CK(s->acc.alloc(2 * (size_t)L.ncloth * s->acc_stride));   // the resident kernel alternates between two sets
+    CK(cudaMemsetAsync(s->acc.p, 0, sizeof(double) * s->acc.n, st));
     if (s->kernel == PDG_KERNEL_RESIDENT || s->range_variant >= 0) {
         CK(s->xch.alloc(8 * (size_t)L.ntot));
         CK(cudaMemsetAsync(s->xch.p, 0, sizeof(unsigned long long) * 8 * (size_t)L.ntot, st));
-        CK(s->res_cnt.alloc((size_t)L.ncloth * s->acc_stride));
+        CK(s->res_cnt.alloc(2 * (size_t)L.ncloth * s->acc_stride));
+        CK(cudaMemsetAsync(s->res_cnt.p, 0, sizeof(int) * s->res_cnt.n, st));
         CK(s->xch_tag.alloc(1));
         CK(cudaMemsetAsync(s->xch_tag.p, 0, sizeof(unsigned), st));
     }
     CK(s->X.alloc(L.ntot)); CK(s->V.alloc(L.ntot)); CK(s->Y.alloc(L.ntot));
     CK(s->A.alloc(L.ntot)); CK(s->B.alloc(L.ntot));
     CK(s->stage_x.alloc(3 * (size_t)L.ntot)); CK(s->stage_v.alloc(3 * (size_t)L.ntot));
-    CK(s->bar.alloc(4));   // [0] arrivals, [1] generation, [2] error word
+    CK(s->bar.alloc(4));   // [0] [1] barrier, [2] error word, [3] the resident kernel's frame parity
     CK(cudaMemsetAsync(s->bar.p, 0, 4 * sizeof(unsigned), st));
     CK(cudaMemsetAsync(s->crt.p, 0, sizeof(ClothRT) * L.ncloth, st));
     CK(cudaMemsetAsync(s->Y.p, 0, sizeof(float4) * L.ntot, st));
@@ -137,6 +138,7 @@ PersistArgs persist_args(pdg_solver* s)
     p.xch_tag = s->xch_tag.p;
     p.nbr_sync = s->nbr_sync;
     p.cnt = s->res_cnt.p;
+    p.frame = s->bar.p + 3;
     p.k0 = p.k1 = 0;
     p.in_x = p.in_v = nullptr;
     p.out_x = p.out_v = nullptr;
@@ -437,7 +439,7 @@ int pdg::create_solver(int n, const pdg_config* cfgs, const pdg_mesh* const* mes
     }
     // Streaming plan: where every patch is resident at once, the resident
     // kernel runs the sweeps of a frame in one launch.  A sweep of 54,000
-    // vertices in 434 patches of 128 then takes 5.3 us instead of 7.3 us.
+    // vertices in 434 patches of 128 then takes 4.8 us instead of 7.3 us.
     if (s->kernel == PDG_KERNEL_STREAM && s->mode == PDG_MODE_CONSISTENT)
         s->range_variant = resident_range_pick(s->L.max_nown, s->L.npatch, s->L.smem_resident);
     int rc = upload_all(s.get());
@@ -646,7 +648,10 @@ static int take_wait_error(pdg_solver* s)
     CK(cudaMemcpyAsync(&e, s->bar.p + 2, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     if (!e) return PDG_OK;
-    CK(cudaMemsetAsync(s->bar.p + 2, 0, sizeof(int), s->stream));
+    // the blocks that gave up left the barrier count and the sums half way
+    CK(cudaMemsetAsync(s->bar.p, 0, 4 * sizeof(unsigned), s->stream));
+    CK(cudaMemsetAsync(s->acc.p, 0, sizeof(double) * s->acc.n, s->stream));
+    if (s->res_cnt.p) CK(cudaMemsetAsync(s->res_cnt.p, 0, sizeof(int) * s->res_cnt.n, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     return set_error(PDG_ERR_TIMEOUT, "bounded wait ran out (%s)",
                      e == 1 ? "grid barrier" : e == 2 ? "resident grid barrier" : "neighbour exchange");
@@ -666,10 +671,11 @@ static int enqueue_frames(pdg_solver* s, int nframes, const FrameIO* io)
 {
     for (int f = 0; f < nframes; ++f) {
         if (s->kernel == PDG_KERNEL_PERSISTENT || s->kernel == PDG_KERNEL_RESIDENT) {
-            // barrier counter and generation start clean every frame; the
-            // error word stays set until it is reported, and a kernel that
-            // finds it set leaves at its first barrier
-            CK(cudaMemsetAsync(s->bar.p, 0, 2 * sizeof(unsigned), s->stream));
+            // the persistent kernel's barrier words start clean every frame;
+            // the error word stays set until it is reported, and a kernel
+            // that finds it set leaves at its first barrier
+            if (s->kernel == PDG_KERNEL_PERSISTENT)
+                CK(cudaMemsetAsync(s->bar.p, 0, 2 * sizeof(unsigned), s->stream));
             PersistArgs p = persist_args(s);
             if (io && f == 0) { p.in_x = io->in_x; p.in_v = io->in_v; }
             if (io && f == nframes - 1) { p.out_x = io->out_x; p.out_v = io->out_v; }
@@ -1007,7 +1013,8 @@ int pdg_solver_time_frames(pdg_solver* s, int nframes, float* frame_ms, float* s
     for (int f = 0; f < nframes && rc == PDG_OK; ++f) {
         cudaEventRecord(e[0], st);
         if (s->kernel == PDG_KERNEL_PERSISTENT || s->kernel == PDG_KERNEL_RESIDENT) {
-            cudaError_t err = cudaMemsetAsync(s->bar.p, 0, 2 * sizeof(unsigned), st);
+            cudaError_t err = s->kernel == PDG_KERNEL_PERSISTENT
+                                  ? cudaMemsetAsync(s->bar.p, 0, 2 * sizeof(unsigned), st) : cudaSuccess;
             cudaEventRecord(e[0], st);   // the frame's events bracket the launch only
             const PersistArgs p = persist_args(s);
             if (err == cudaSuccess)
