@@ -28,13 +28,23 @@ namespace gnn {
 
 using bf16 = __nv_bfloat16;
 
-enum { EPI_RELU = 1, EPI_STORE1 = 2, EPI_RESID2 = 4, EPI_STOREF = 8, EPI_ACCF = 16, EPI_RESIDA = 32 };
+enum { EPI_RELU = 1, EPI_STORE1 = 2, EPI_RESID2 = 4, EPI_STOREF = 8, EPI_ACCF = 16, EPI_RESIDA = 32,
+       EPI_MASKA = 64, EPI_SPLIT = 128 };
 
 __device__ __forceinline__ uint32_t ld_pair(const bf16* p) { return *reinterpret_cast<const uint32_t*>(p); }
 __device__ __forceinline__ uint32_t ld_pair(const float* p)
 {
     const float2 f = *reinterpret_cast<const float2*>(p);
     __nv_bfloat162 b = __floats2bfloat162_rn(f.x, f.y);
+    return *reinterpret_cast<uint32_t*>(&b);
+}
+
+// a pair of fp32 values as bf16, zero where ref is not positive (ReLU backward)
+__device__ __forceinline__ uint32_t ld_pair_masked(const float* p, const bf16* ref)
+{
+    const float2 f = *reinterpret_cast<const float2*>(p);
+    const float2 r = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(ref));
+    __nv_bfloat162 b = __floats2bfloat162_rn(r.x > 0.f ? f.x : 0.f, r.y > 0.f ? f.y : 0.f);
     return *reinterpret_cast<uint32_t*>(&b);
 }
 
@@ -55,13 +65,17 @@ __device__ __forceinline__ void mma_bf16(float* c, uint32_t a0, uint32_t a1, uin
 // (gemm_grid sizes the grid to the resident blocks).
 // Epilogue: optional ReLU; Y1 <- bf16(v); Y2 <- bf16(R + v) (R read, or taken
 // from the A fragments when it is X's first NOUT columns); Yf <- v or += v.
+// The backward pass also has EPI_MASKA: X (fp32) counts as zero where R
+// [M][K] is not positive, and EPI_SPLIT (K = NOUT / 2): Yf <- X + v for the
+// first K columns of v, Yg <- v for the others.
 template <typename TA, int K, int NOUT, int EPI>
 __global__ void __launch_bounds__(128) k_gemm(const TA* __restrict__ X, int ldx, int M, const bf16* __restrict__ W,
                                               const float* __restrict__ bias, const bf16* __restrict__ R, int ldr,
                                               bf16* __restrict__ Y1, int ld1, bf16* __restrict__ Y2, int ld2,
-                                              float* __restrict__ Yf, int ldf)
+                                              float* __restrict__ Yf, int ldf, float* __restrict__ Yg, int ldg)
 {
     static_assert(K % 16 == 0 && NOUT % 8 == 0, "mma tile shape");
+    static_assert(!(EPI & EPI_SPLIT) || NOUT == 2 * K, "the split is at K");
     static_assert(!(EPI & EPI_RESIDA) || NOUT <= K, "the residual is part of the A operand");
     __shared__ __align__(16) bf16 sW[NOUT * (K + 8)];
     __shared__ float sb[NOUT];
@@ -79,6 +93,19 @@ __global__ void __launch_bounds__(128) k_gemm(const TA* __restrict__ X, int ldx,
         const bool ok0 = r0 + g < M, ok1 = r0 + g + 8 < M;
         const TA* x0 = X + (size_t)(r0 + g) * ldx;
         const TA* x1 = X + (size_t)(r0 + g + 8) * ldx;
+        if constexpr ((EPI & EPI_MASKA) != 0) {
+            const bf16* m0 = R + (size_t)(r0 + g) * ldr;
+            const bf16* m1 = R + (size_t)(r0 + g + 8) * ldr;
+            #pragma unroll
+            for (int ks = 0; ks < K / 16; ++ks) {
+                const int c0 = ks * 16 + 2 * t;
+                f[ks][0] = ok0 ? ld_pair_masked(x0 + c0, m0 + c0) : 0u;
+                f[ks][1] = ok1 ? ld_pair_masked(x1 + c0, m1 + c0) : 0u;
+                f[ks][2] = ok0 ? ld_pair_masked(x0 + c0 + 8, m0 + c0 + 8) : 0u;
+                f[ks][3] = ok1 ? ld_pair_masked(x1 + c0 + 8, m1 + c0 + 8) : 0u;
+            }
+            return;
+        }
         #pragma unroll
         for (int ks = 0; ks < K / 16; ++ks) {
             const int c0 = ks * 16 + 2 * t;
@@ -140,6 +167,14 @@ __global__ void __launch_bounds__(128) k_gemm(const TA* __restrict__ X, int ldx,
                     const float2 o = *p;
                     *p = make_float2(o.x + v0, o.y + v1);
                 }
+                if constexpr ((EPI & EPI_SPLIT) != 0) {
+                    if (n * 8 < K) {
+                        const float2 x = *reinterpret_cast<const float2*>(X + (size_t)row * ldx + col);
+                        *reinterpret_cast<float2*>(Yf + (size_t)row * ldf + col) = make_float2(x.x + v0, x.y + v1);
+                    } else {
+                        *reinterpret_cast<float2*>(Yg + (size_t)row * ldg + col - K) = make_float2(v0, v1);
+                    }
+                }
             }
         #pragma unroll
         for (int ks = 0; ks < K / 16; ++ks)
@@ -180,10 +215,10 @@ int gemm_grid(int M)
 // Launch of k_gemm on `st` with the grid above.
 template <typename TA, int K, int NOUT, int EPI>
 void gemm(cudaStream_t st, const TA* X, int ldx, int M, const bf16* W, const float* bias, const bf16* R, int ldr,
-          bf16* Y1, int ld1, bf16* Y2, int ld2, float* Yf, int ldf)
+          bf16* Y1, int ld1, bf16* Y2, int ld2, float* Yf, int ldf, float* Yg = nullptr, int ldg = 0)
 {
     k_gemm<TA, K, NOUT, EPI><<<gemm_grid<TA, K, NOUT, EPI>(M), 128, 0, st>>>(X, ldx, M, W, bias, R, ldr, Y1, ld1, Y2,
-                                                                            ld2, Yf, ldf);
+                                                                            ld2, Yf, ldf, Yg, ldg);
 }
 
 // ---- fused inference kernels ----------------------------------------------
@@ -473,9 +508,10 @@ __device__ __forceinline__ void ldsm_x4_t(const bf16* p, uint32_t& r0, uint32_t&
 // NP x KP: the output padded to mma tiles (nout <= NP <= ldy, K <= KP <= ldx;
 // the padding columns of dY and X are read and their products dropped).
 // 16-byte alignment of the rows of dY and X is a multiple of ldy and ldx.
-template <int NP, int KP>
+// MASK: dY counts as zero where ref [M][NP] is not positive (ReLU backward).
+template <int NP, int KP, bool MASK>
 __global__ void __launch_bounds__(256) k_wgrad(const float* __restrict__ dY, int ldy, int nout,
-                                               const bf16* __restrict__ X, int ldx, int K, int M,
+                                               const bf16* __restrict__ ref, int ldr, const bf16* __restrict__ X, int ldx, int K, int M,
                                                float* __restrict__ part)
 {
     constexpr int RT = kWgradRows, NT = 256;
@@ -499,7 +535,16 @@ __global__ void __launch_bounds__(256) k_wgrad(const float* __restrict__ dY, int
         __syncthreads();
         for (int r = br; r < RT; r += NT / (NP / 4)) {
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (r0 + r < M) v = *reinterpret_cast<const float4*>(dY + (size_t)(r0 + r) * ldy + bc);
+            if (r0 + r < M) {
+                v = *reinterpret_cast<const float4*>(dY + (size_t)(r0 + r) * ldy + bc);
+                if (MASK) {
+                    const uint2 u = *reinterpret_cast<const uint2*>(ref + (size_t)(r0 + r) * ldr + bc);
+                    const float2 m01 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
+                    const float2 m23 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+                    v = make_float4(m01.x > 0.f ? v.x : 0.f, m01.y > 0.f ? v.y : 0.f, m23.x > 0.f ? v.z : 0.f,
+                                    m23.y > 0.f ? v.w : 0.f);
+                }
+            }
             bacc.x += v.x; bacc.y += v.y; bacc.z += v.z; bacc.w += v.w;
             __align__(8) bf16 h[4], m[4], l[4];
             split3(v.x, h[0], m[0], l[0]); split3(v.y, h[1], m[1], l[1]);
@@ -558,16 +603,30 @@ __global__ void __launch_bounds__(256) k_wgrad(const float* __restrict__ dY, int
     }
 }
 
-// dW[i] = sum_b part[b][i] (i < nw), db[i] = sum_b part[b][nw + i] (i < nb,
-// db may be null).  A block sums 32 entries: 8 threads each add every eighth
-// block in order, then the 8 sums are added in order.  (One thread per entry
-// adding all blocks took 25 us for 8,256 entries of 304 blocks.)
-__global__ void __launch_bounds__(256) k_sum_parts(const float* __restrict__ part, int nblocks, int nw, int nbias,
-                                                   float* __restrict__ dW, float* __restrict__ db)
+// Sums of per-block partials, for every gradient of the backward pass at once:
+// segment j holds part_j[nblocks_j][nw_j + nbias_j], of which dW_j[i] =
+// sum_b part_j[b][i] (i < nw_j) and db_j[i] = sum_b part_j[b][nw_j + i]
+// (db may be null).
+constexpr int kSumSegs = 2 + 3 * L;
+struct SumTable {
+    const float* part[kSumSegs];
+    float *dW[kSumSegs], *db[kSumSegs];
+    int nblocks[kSumSegs], nw[kSumSegs], nbias[kSumSegs];
+    int first[kSumSegs + 1];   // first block of each segment's entries
+};
+
+// A block sums 32 entries: 8 threads each add every eighth block in order,
+// then the 8 sums are added in order.  (One thread per entry adding all blocks
+// took 25 us for 8,256 entries of 304 blocks.)
+__global__ void __launch_bounds__(256) k_sum_parts(SumTable t)
 {
     __shared__ float sp[8][32];
+    int j = 0;
+    while (j + 1 < kSumSegs && (int)blockIdx.x >= t.first[j + 1]) ++j;
+    const float* __restrict__ part = t.part[j];
+    const int nblocks = t.nblocks[j], nw = t.nw[j], width = nw + t.nbias[j];
     const int col = threadIdx.x & 31, grp = threadIdx.x >> 5;
-    const int i = blockIdx.x * 32 + col, width = nw + nbias;
+    const int i = ((int)blockIdx.x - t.first[j]) * 32 + col;
     float s = 0.f;
     if (i < width) {
         #pragma unroll 8
@@ -575,10 +634,10 @@ __global__ void __launch_bounds__(256) k_sum_parts(const float* __restrict__ par
     }
     sp[grp][col] = s;
     __syncthreads();
-    if (grp != 0 || i >= width || (i >= nw && !db)) return;
+    if (grp != 0 || i >= width || (i >= nw && !t.db[j])) return;
     #pragma unroll
     for (int g = 1; g < 8; ++g) s += sp[g][col];
-    if (i < nw) dW[i] = s; else db[i - nw] = s;
+    if (i < nw) t.dW[j][i] = s; else t.db[j][i - nw] = s;
 }
 
 // Messages of layer l:
@@ -677,14 +736,14 @@ __global__ void __launch_bounds__(256) k_msg_fwd(int N, const int* __restrict__ 
 inline int msg_grid(int N) { return resident_grid<k_msg_fwd>(256, 0, ((((long long)N + 1) >> 1) + 7) / 8); }
 
 // Backward of the messages: dP_i = sum_j g_ij, dQ_j = sum_i g_ij with
-// g_ij = [z_ij > 0] da_i / deg_i (da = dcat[:, H:2H]); dC, dc reduced per
+// g_ij = [z_ij > 0] da_i / deg_i (da [N][H]); dC, dc reduced per
 // block into `part`.  Each warp handles node n as receiver (dP) and as sender (dQ, via
 // the reverse edge's features).
 __global__ void __launch_bounds__(256) k_msg_bwd(int N, const int* __restrict__ ptr, const int* __restrict__ adj,
                                                  const int* __restrict__ rev, const float4* __restrict__ ef,
                                                  const float* __restrict__ deg_inv, const bf16* __restrict__ PQ,
                                                  const float* __restrict__ C, const float* __restrict__ cb,
-                                                 const float* __restrict__ dcat, float* __restrict__ dpq,
+                                                 const float* __restrict__ da_, float* __restrict__ dpq,
                                                  float* __restrict__ part)
 {
     __shared__ float red[8][H * (EF + 1)];
@@ -696,7 +755,7 @@ __global__ void __launch_bounds__(256) k_msg_bwd(int N, const int* __restrict__ 
     for (int node = blockIdx.x * 8 + warp; node < N; node += gridDim.x * 8) {
         const float2 Pn = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(PQ + (size_t)node * 2 * H + ch));
         const float2 Qn = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(PQ + (size_t)node * 2 * H + H + ch));
-        const float2 dan = *reinterpret_cast<const float2*>(dcat + (size_t)node * 2 * H + H + ch);
+        const float2 dan = *reinterpret_cast<const float2*>(da_ + (size_t)node * H + ch);
         const float din = deg_inv[node];
         float dP0 = 0.f, dP1 = 0.f, dQ0 = 0.f, dQ1 = 0.f;
         for (int e = ptr[node]; e < ptr[node + 1]; ++e) {
@@ -717,7 +776,7 @@ __global__ void __launch_bounds__(256) k_msg_bwd(int N, const int* __restrict__ 
             {
                 const float4 f = ef[rev[e]];
                 const float2 P = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(PQ + (size_t)j * 2 * H + ch));
-                const float2 da = *reinterpret_cast<const float2*>(dcat + (size_t)j * 2 * H + H + ch);
+                const float2 da = *reinterpret_cast<const float2*>(da_ + (size_t)j * H + ch);
                 const float dj = deg_inv[j];
                 const float z0 = P.x + Qn.x + C0.x * f.x + C0.y * f.y + C0.z * f.z + C0.w * f.w + c0;
                 const float z1 = P.y + Qn.y + C1.x * f.x + C1.y * f.y + C1.z * f.z + C1.w * f.w + c1;
@@ -785,25 +844,6 @@ __global__ void k_loss(int N, const float* __restrict__ out, const float* __rest
     }
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if ((threadIdx.x & 31) == 0 && s != 0.f) atomicAdd(loss, (double)s * inv_cnt);
-}
-
-// dst = src * mask(ref > 0) (ReLU backward; ref is the bf16 ReLU output)
-__global__ void k_relu_bwd(int N, int cols, const float* __restrict__ src, int lds, const bf16* __restrict__ ref,
-                           int ldr, float* __restrict__ dst, int ldd)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N * cols) return;
-    const int r = i / cols, c = i % cols;
-    dst[(size_t)r * ldd + c] = __bfloat162float(ref[(size_t)r * ldr + c]) > 0.f ? src[(size_t)r * lds + c] : 0.f;
-}
-
-// dst[:, 0:cols] += src[:, 0:cols]
-__global__ void k_add(int N, int cols, const float* __restrict__ src, int lds, float* __restrict__ dst, int ldd)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N * cols) return;
-    const int r = i / cols, c = i % cols;
-    dst[(size_t)r * ldd + c] += src[(size_t)r * lds + c];
 }
 
 __global__ void k_adam(int n, float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
