@@ -35,6 +35,7 @@ struct pdg_warmstart {
     DevBuf<float> rest, deg_inv;
     DevBuf<float4> ef, stat, Xn, Vn, Dn;
     DevBuf<float> ew;     // per directed edge: weight of the energy-norm term of the loss
+    DevBuf<uint2> mask[L];   // per edge: signs of the message's channels
     DevBuf<bf16> xin, cat[L], pq[L], uo[L], hfin;
     DevBuf<float> out, target, freew, dout, dh, dtmp, da, dpq;
     DevBuf<double> loss;
@@ -56,7 +57,7 @@ namespace {
 inline int nb(long long n, int b) { return (int)((n + b - 1) / b); }
 
 constexpr int kWgradBlocks = 304;        // at most, blocks of a weight-gradient reduction
-constexpr int kMsgBwdBlocks = 4 * 152;   // at most, blocks of the message backward
+constexpr int kMsgBwdBlocks = 3 * 152;   // at most, blocks of the message backward (those resident at once)
 
 int refresh_bf16(pdg_warmstart* w, cudaStream_t st)
 {
@@ -115,6 +116,7 @@ int alloc_graph(pdg_warmstart* w, int N, int E)
     GK(w->xin.reserve((size_t)N * NFP));
     for (int l = 0; l < L; ++l) {
         GK(w->cat[l].reserve((size_t)N * 2 * H)); GK(w->pq[l].reserve((size_t)N * 2 * H)); GK(w->uo[l].reserve((size_t)N * H));
+        GK(w->mask[l].reserve(E));
     }
     GK(w->hfin.reserve((size_t)N * H));
     GK(w->out.reserve((size_t)N * 16)); GK(w->target.reserve((size_t)N * 3)); GK(w->freew.reserve(N));
@@ -137,8 +139,8 @@ int forward(pdg_warmstart* w, cudaStream_t st)
     for (int l = 0; l < L; ++l) {
         gemm<bf16, H, 2 * H, EPI_STORE1>(st, w->cat[l].p, 2 * H, N, w->W.AB[l], nullptr, nullptr, 0, w->pq[l].p, 2 * H,
                                          nullptr, 0, nullptr, 0);
-        k_msg_fwd<<<msg_grid(N), 256, 0, st>>>(N, w->ptr.p, w->adj.p, w->ef.p, w->deg_inv.p, w->pq[l].p,
-                                                             p + y.C[l], p + y.c[l], w->cat[l].p);
+        messages<true>(st, N, w->ptr.p, w->adj.p, w->ef.p, w->deg_inv.p, w->pq[l].p, p + y.C[l], p + y.c[l], w->cat[l].p,
+                       w->mask[l].p);
         bf16* next = l + 1 < L ? w->cat[l + 1].p : w->hfin.p;
         const int ldn = l + 1 < L ? 2 * H : H;
         // h <- h + relu(U [h; a] + u): the residual h is the A operand's
@@ -206,11 +208,10 @@ int backward(pdg_warmstart* w, float inv_cnt, const float* ew, cudaStream_t st)
     for (int l = L - 1; l >= 0; --l) {
         wgrad<H, 2 * H, true>(gs, dh, H, H, w->uo[l].p, H, w->cat[l].p, 2 * H, 2 * H, N, g + y.U[l], g + y.u[l], st);
         gemm<float, H, 2 * H, EPI_MASKA | EPI_SPLIT>(st, dh, H, N, w->W.Ut[l], nullptr, w->uo[l].p, H, nullptr, 0,
-                                                     nullptr, 0, dn, H, w->da.p, H);
-        const int gm = std::max(1, std::min(kMsgBwdBlocks, nb(N, 8)));
+                                                     nullptr, 0, dn, H, w->da.p, H, w->deg_inv.p);
+        const int gm = std::max(1, std::min(kMsgBwdBlocks, nb(N, 16)));
         float* part = gs.add(gm, H * EF, H, g + y.C[l], g + y.c[l]);
-        k_msg_bwd<<<gm, 256, 0, st>>>(N, w->ptr.p, w->adj.p, w->rev.p, w->ef.p, w->deg_inv.p, w->pq[l].p, p + y.C[l],
-                                      p + y.c[l], w->da.p, w->dpq.p, part);
+        k_msg_bwd<<<gm, 256, 0, st>>>(N, w->ptr.p, w->adj.p, w->rev.p, w->ef.p, w->mask[l].p, w->da.p, w->dpq.p, part);
         wgrad<2 * H, H, false>(gs, w->dpq.p, 2 * H, 2 * H, nullptr, 0, w->cat[l].p, 2 * H, H, N, g + y.A[l], nullptr, st);
         gemm<float, 2 * H, H, EPI_ACCF>(st, w->dpq.p, 2 * H, N, w->W.ABt[l], nullptr, nullptr, 0, nullptr, 0, nullptr, 0,
                                         dn, H);
@@ -281,8 +282,8 @@ int warm_infer_enqueue(pdg_warmstart* w, pdg_solver* s)
     fused<FUSE_ENC_PQ>(st, w->xin.p, NFP, N, w->W.We, p + y.be, w->W.AB[0], nullptr, w->cat[0].p, 2 * H, w->pq[0].p,
                        nullptr, nullptr, nullptr);
     for (int l = 0; l < L; ++l) {
-        k_msg_fwd<<<msg_grid(N), 256, 0, st>>>(N, w->ptr.p, w->adj.p, w->ef.p, w->deg_inv.p, w->pq[l].p, p + y.C[l],
-                                              p + y.c[l], w->cat[l].p);
+        messages<false>(st, N, w->ptr.p, w->adj.p, w->ef.p, w->deg_inv.p, w->pq[l].p, p + y.C[l], p + y.c[l], w->cat[l].p,
+                        nullptr);
         if (l + 1 < L)
             fused<FUSE_UPD_PQ>(st, w->cat[l].p, 2 * H, N, w->W.U[l], p + y.u[l], w->W.AB[l + 1], nullptr,
                                w->cat[l + 1].p, 2 * H, w->pq[l + 1].p, nullptr, nullptr, nullptr);
