@@ -61,16 +61,7 @@ constexpr int kMsgBwdBlocks = 3 * 152;   // at most, blocks of the message backw
 
 int refresh_bf16(pdg_warmstart* w, cudaStream_t st)
 {
-    const Layout& y = w->lay;
-    const float* p = w->p.p;
-    k_to_bf16<<<nb(H * NF, 256), 256, 0, st>>>(p + y.We, H, NF, w->W.We, NFP, nullptr, 0);
-    for (int l = 0; l < L; ++l) {
-        k_to_bf16<<<nb(H * H, 256), 256, 0, st>>>(p + y.A[l], H, H, w->W.AB[l], H, w->W.ABt[l], 2 * H);
-        k_to_bf16<<<nb(H * H, 256), 256, 0, st>>>(p + y.B[l], H, H, w->W.AB[l] + H * H, H, w->W.ABt[l] + H, 2 * H);
-        k_to_bf16<<<nb(H * 2 * H, 256), 256, 0, st>>>(p + y.U[l], H, 2 * H, w->W.U[l], 2 * H, w->W.Ut[l], H);
-    }
-    k_to_bf16<<<nb(NO * H, 256), 256, 0, st>>>(p + y.Wd, NO, H, w->W.Wd, H, w->W.Wdt, 16);
-    GK(cudaMemcpyAsync(w->bdp.p, p + y.bd, sizeof(float) * NO, cudaMemcpyDeviceToDevice, st));
+    k_copies<<<nb(w->lay.total, 256), 256, 0, st>>>(w->lay.total, w->p.p, w->lay, w->W, w->bdp.p);
     GK(cudaGetLastError());
     return PDG_OK;
 }
@@ -230,9 +221,9 @@ int adam_step(pdg_warmstart* w, float lr, cudaStream_t st)
     const float bc1 = 1.f - (float)std::pow((double)b1, (double)w->t);
     const float bc2 = 1.f - (float)std::pow((double)b2, (double)w->t);
     k_adam<<<nb(w->lay.total, 256), 256, 0, st>>>(w->lay.total, w->p.p, w->g.p, w->m.p, w->v.p, lr, b1, b2, eps, bc1,
-                                                  bc2);
+                                                  bc2, w->lay, w->W, w->bdp.p);
     GK(cudaGetLastError());
-    return refresh_bf16(w, st);
+    return PDG_OK;
 }
 
 // Room for the graph, and its arrays on `st`: the reverse-edge index and the
@@ -547,8 +538,8 @@ int pdg_warmstart_train_frame(pdg_warmstart* w, pdg_solver* s, float lr, float* 
         if (rc) return rc;
     }
     // features and target 3, forward 2 + 3L, loss and backward 5 + 5L,
-    // Adam and the bf16 refresh 3 + 3L
-    s->launches += 3 + (2 + 3 * L) + (5 + 5 * L) + (lr > 0.f ? 3 + 3 * L : 0);
+    // Adam 1
+    s->launches += 3 + (2 + 3 * L) + (5 + 5 * L) + (lr > 0.f ? 1 : 0);
     double l = 0.0;
     GK(cudaMemcpyAsync(&l, w->loss.p, sizeof(double), cudaMemcpyDeviceToHost, st));
     GK(cudaStreamSynchronize(st));
@@ -595,7 +586,7 @@ int pdg_warmstart_train_pair(pdg_warmstart* w, pdg_solver* traj, pdg_solver* dee
         rc = adam_step(w, lr, st);
         if (rc) return rc;
     }
-    traj->launches += 3 + (2 + 3 * L) + (5 + 5 * L) + (lr > 0.f ? 3 + 3 * L : 0);
+    traj->launches += 3 + (2 + 3 * L) + (5 + 5 * L) + (lr > 0.f ? 1 : 0);
     double l = 0.0;
     GK(cudaMemcpyAsync(&l, w->loss.p, sizeof(double), cudaMemcpyDeviceToHost, st));
     GK(cudaStreamSynchronize(st));

@@ -904,8 +904,37 @@ __global__ void k_loss(int N, const float* __restrict__ out, const float* __rest
     if ((threadIdx.x & 31) == 0 && s != 0.f) atomicAdd(loss, (double)s * inv_cnt);
 }
 
+// Parameter i with value v into the bf16 copies: each weight matrix and its
+// transpose, the decoder's bias (padded, fp32); other biases have no copy.
+__device__ __forceinline__ void put_copy(const Layout& y, const Bf16Weights& W, float* bdp, int i, float v)
+{
+    const bf16 b = __float2bfloat16_rn(v);
+    if (i < y.be) { W.We[(i / NF) * NFP + i % NF] = b; return; }
+    if (i >= y.bd) { bdp[i - y.bd] = v; return; }
+    if (i >= y.Wd) { const int q = i - y.Wd, r = q / H, c = q % H; W.Wd[r * H + c] = b; W.Wdt[c * 16 + r] = b; return; }
+    #pragma unroll
+    for (int l = 0; l < L; ++l) {
+        if (i >= y.A[l] && i < y.C[l]) {          // A, then B: rows 0..H-1 and H..2H-1 of one matrix
+            const int q = i - y.A[l], r = q / H, c = q % H;
+            W.AB[l][r * H + c] = b; W.ABt[l][c * 2 * H + r] = b;
+        } else if (i >= y.U[l] && i < y.u[l]) {
+            const int q = i - y.U[l], r = q / (2 * H), c = q % (2 * H);
+            W.U[l][r * 2 * H + c] = b; W.Ut[l][c * H + r] = b;
+        }
+    }
+}
+
+// The copies of all parameters, which k_adam also refreshes (ten launches
+// after it otherwise: 2.5 us each).
+__global__ void k_copies(int n, const float* __restrict__ p, Layout y, Bf16Weights W, float* bdp)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) put_copy(y, W, bdp, i, p[i]);
+}
+
 __global__ void k_adam(int n, float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
-                       float* __restrict__ v, float lr, float b1, float b2, float eps, float bc1, float bc2)
+                       float* __restrict__ v, float lr, float b1, float b2, float eps, float bc1, float bc2, Layout y,
+                       Bf16Weights W, float* bdp)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -914,20 +943,9 @@ __global__ void k_adam(int n, float* __restrict__ p, const float* __restrict__ g
     const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
     m[i] = mi;
     v[i] = vi;
-    p[i] -= lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
-}
-
-// bf16 copy of a [rows][cols] fp32 tensor into dst[rows_pad][ld] (and its
-// transpose into dstT[cols][ldT]); padding rows/cols are left as zero.
-__global__ void k_to_bf16(const float* __restrict__ src, int rows, int cols, bf16* __restrict__ dst, int ld,
-                          bf16* __restrict__ dstT, int ldT)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= rows * cols) return;
-    const int r = i / cols, c = i % cols;
-    const bf16 b = __float2bfloat16_rn(src[i]);
-    if (dst) dst[(size_t)r * ld + c] = b;
-    if (dstT) dstT[(size_t)c * ldT + r] = b;
+    const float q = p[i] - lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
+    p[i] = q;
+    put_copy(y, W, bdp, i, q);
 }
 
 // ---- caller graphs ---------------------------------------------------------
