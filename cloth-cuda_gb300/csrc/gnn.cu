@@ -125,6 +125,8 @@ int forward(pdg_warmstart* w, cudaStream_t st)
     const int N = w->N;
     const Layout& y = w->lay;
     const float* p = w->p.p;
+    // (the backward pass's; here it parts no two kernels)
+    GK(cudaMemsetAsync(w->loss.p, 0, sizeof(double), st));
     gemm<bf16, NFP, H, EPI_RELU | EPI_STORE1>(st, w->xin.p, NFP, N, w->W.We, p + y.be, nullptr, 0, w->cat[0].p, 2 * H,
                                               nullptr, 0, nullptr, 0);
     for (int l = 0; l < L; ++l) {
@@ -163,7 +165,7 @@ struct GradSums {
         ++n;
         return q;
     }
-    void run(cudaStream_t st) { k_sum_parts<<<t.first[n], 256, 0, st>>>(t); }
+    void run(cudaStream_t st) { launch_after(k_sum_parts, t.first[n], 256, 0, st, t); }
 };
 
 // Partial sums of dW (nout x K) and db (nout, may be null) of dY^T X over M
@@ -174,11 +176,11 @@ void wgrad(GradSums& gs, const float* dY, int ldy, int nout, const bf16* ref, in
 {
     const int gw = wgrad_grid(M);
     float* part = gs.add(gw, nout * K, nout, dW, db);
-    k_wgrad<NP, KP, MASK><<<gw, 256, 0, st>>>(dY, ldy, nout, ref, ldr, X, ldx, K, M, part);
+    launch_after(k_wgrad<NP, KP, MASK>, gw, 256, 0, st, dY, ldy, nout, ref, ldr, X, ldx, K, M, part);
 }
 
 // gradients of the loss w.r.t. all parameters into w->g; loss accumulated into
-// w->loss; ew: per-edge weights of the smoothness term (null: 1).  The ReLU
+// w->loss (cleared by forward); ew: per-edge weights of the smoothness term (null: 1).  The ReLU
 // masks are applied where their operand is read and the residual path is added
 // where its partner is written.  With both in kernels of their own and one
 // launch of sums per gradient a training step on 16 cloths took 2,220 us (now
@@ -190,8 +192,7 @@ int backward(pdg_warmstart* w, float inv_cnt, const float* ew, cudaStream_t st)
     const float* p = w->p.p;
     float* g = w->g.p;
     GradSums gs(w->part.p);
-    GK(cudaMemsetAsync(w->loss.p, 0, sizeof(double), st));
-    k_loss<<<nb(N, 256), 256, 0, st>>>(N, w->out.p, w->target.p, w->freew.p, w->ptr.p, w->adj.p, ew, w->smooth,
+    launch_after(k_loss, nb(N, 256), 256, 0, st, N, w->out.p, w->target.p, w->freew.p, w->ptr.p, w->adj.p, ew, w->smooth,
                                        inv_cnt, w->dout.p, w->loss.p);
     wgrad<16, H, false>(gs, w->dout.p, 16, NO, nullptr, 0, w->hfin.p, H, H, N, g + y.Wd, g + y.bd, st);
     float *dh = w->dh.p, *dn = w->dtmp.p;   // d loss / d h of layer l, of layer l - 1
@@ -202,7 +203,7 @@ int backward(pdg_warmstart* w, float inv_cnt, const float* ew, cudaStream_t st)
                                                      nullptr, 0, dn, H, w->da.p, H, w->deg_inv.p);
         const int gm = std::max(1, std::min(kMsgBwdBlocks, nb(N, 16)));
         float* part = gs.add(gm, H * EF, H, g + y.C[l], g + y.c[l]);
-        k_msg_bwd<<<gm, 256, 0, st>>>(N, w->ptr.p, w->adj.p, w->rev.p, w->ef.p, w->mask[l].p, w->da.p, w->dpq.p, part);
+        launch_after(k_msg_bwd, gm, 256, 0, st, N, w->ptr.p, w->adj.p, w->rev.p, w->ef.p, w->mask[l].p, w->da.p, w->dpq.p, part);
         wgrad<2 * H, H, false>(gs, w->dpq.p, 2 * H, 2 * H, nullptr, 0, w->cat[l].p, 2 * H, H, N, g + y.A[l], nullptr, st);
         gemm<float, 2 * H, H, EPI_ACCF>(st, w->dpq.p, 2 * H, N, w->W.ABt[l], nullptr, nullptr, 0, nullptr, 0, nullptr, 0,
                                         dn, H);
@@ -220,7 +221,7 @@ int adam_step(pdg_warmstart* w, float lr, cudaStream_t st)
     w->t += 1;
     const float bc1 = 1.f - (float)std::pow((double)b1, (double)w->t);
     const float bc2 = 1.f - (float)std::pow((double)b2, (double)w->t);
-    k_adam<<<nb(w->lay.total, 256), 256, 0, st>>>(w->lay.total, w->p.p, w->g.p, w->m.p, w->v.p, lr, b1, b2, eps, bc1,
+    launch_after(k_adam, nb(w->lay.total, 256), 256, 0, st, w->lay.total, w->p.p, w->g.p, w->m.p, w->v.p, lr, b1, b2, eps, bc1,
                                                   bc2, w->lay, w->W, w->bdp.p);
     GK(cudaGetLastError());
     return PDG_OK;
@@ -264,7 +265,7 @@ int warm_infer_enqueue(pdg_warmstart* w, pdg_solver* s)
     const int N = w->N;
     k_node_feat<<<nb(N, 256), 256, 0, st>>>(N, s->X.p, s->V.p, s->Y.p, s->aux.p, w->stat.p, s->vcloth.p, s->cinfo.p,
                                             s->dprev.p, w->xin.p);
-    k_edge_feat<<<nb(N, 256), 256, 0, st>>>(N, w->ptr.p, w->adj.p, w->rest.p, s->Y.p, w->ef.p);
+    launch_after(k_edge_feat, nb(N, 256), 256, 0, st, N, w->ptr.p, w->adj.p, w->rest.p, s->Y.p, w->ef.p);
     // encoder + layer 0's P, Q; per layer the messages, then the update fused
     // with the next layer's P, Q or, after the last layer, with the decoder
     // and the start offsets
@@ -525,8 +526,8 @@ int pdg_warmstart_train_frame(pdg_warmstart* w, pdg_solver* s, float lr, float* 
     // inputs from (x_n, v_n, y, d_prev), target (x* - y - d_prev)/s from the solve
     k_node_feat<<<nb(N, 256), 256, 0, st>>>(N, w->Xn.p, w->Vn.p, s->Y.p, s->aux.p, w->stat.p, s->vcloth.p, s->cinfo.p,
                                             w->Dn.p, w->xin.p);
-    k_edge_feat<<<nb(N, 256), 256, 0, st>>>(N, w->ptr.p, w->adj.p, w->rest.p, s->Y.p, w->ef.p);
-    k_target<<<nb(N, 256), 256, 0, st>>>(N, s->X.p, s->Y.p, s->aux.p, w->Dn.p, w->target.p, w->freew.p);
+    launch_after(k_edge_feat, nb(N, 256), 256, 0, st, N, w->ptr.p, w->adj.p, w->rest.p, s->Y.p, w->ef.p);
+    launch_after(k_target, nb(N, 256), 256, 0, st, N, s->X.p, s->Y.p, s->aux.p, w->Dn.p, w->target.p, w->freew.p);
     int nfree = 0;
     for (const auto& a : s->L.aux) nfree += a.w >= 0.f ? 1 : 0;
     rc = forward(w, st);
@@ -574,8 +575,8 @@ int pdg_warmstart_train_pair(pdg_warmstart* w, pdg_solver* traj, pdg_solver* dee
     // y of both solvers is the same prediction from the same state
     k_node_feat<<<nb(N, 256), 256, 0, st>>>(N, w->Xn.p, w->Vn.p, traj->Y.p, traj->aux.p, w->stat.p, traj->vcloth.p,
                                             traj->cinfo.p, w->Dn.p, w->xin.p);
-    k_edge_feat<<<nb(N, 256), 256, 0, st>>>(N, w->ptr.p, w->adj.p, w->rest.p, traj->Y.p, w->ef.p);
-    k_target<<<nb(N, 256), 256, 0, st>>>(N, deep->X.p, traj->Y.p, traj->aux.p, w->Dn.p, w->target.p, w->freew.p);
+    launch_after(k_edge_feat, nb(N, 256), 256, 0, st, N, w->ptr.p, w->adj.p, w->rest.p, traj->Y.p, w->ef.p);
+    launch_after(k_target, nb(N, 256), 256, 0, st, N, deep->X.p, traj->Y.p, traj->aux.p, w->Dn.p, w->target.p, w->freew.p);
     int nfree = 0;
     for (const auto& a : traj->L.aux) nfree += a.w >= 0.f ? 1 : 0;
     rc = forward(w, st);

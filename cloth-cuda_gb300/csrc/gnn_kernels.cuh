@@ -28,6 +28,40 @@ namespace gnn {
 
 using bf16 = __nv_bfloat16;
 
+// The kernels below follow one another on a stream and are launched as
+// programmatic dependents: a kernel may be scheduled, and stage its weights,
+// while the one before it still runs.  Each calls `after_previous` before it
+// reads or writes anything but weights and the graph's own arrays (neither is
+// written by these kernels; k_adam's successors are launched after a host
+// synchronisation).  It waits until the previous kernel has completed, which
+// itself waited so, hence all earlier ones.  Data of earlier kernels is read
+// through pointers without __restrict__, so that it does not go through the
+// read-only path, which such an overlap would not allow.
+// Launched one after the other these chains of 7 to 24 short kernels were bound
+// by the gaps: gradients of a 9x9 graph 245 us, of a 97x97 graph 385, the
+// inference of 5 cloths 74 and of 64 cloths 537; now 186, 344, 56 and 510.
+__device__ __forceinline__ void after_previous()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+void launch_after(void (*kern)(P...), int grid, int block, size_t smem, cudaStream_t st, A... args)
+{
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 enum { EPI_RELU = 1, EPI_STORE1 = 2, EPI_RESID2 = 4, EPI_STOREF = 8, EPI_ACCF = 16, EPI_RESIDA = 32,
        EPI_MASKA = 64, EPI_SPLIT = 128 };
 
@@ -69,8 +103,8 @@ __device__ __forceinline__ void mma_bf16(float* c, uint32_t a0, uint32_t a1, uin
 // [M][K] is not positive, and EPI_SPLIT (K = NOUT / 2): Yf <- X + v for the
 // first K columns of v, Yg <- v rs[row] for the others.
 template <typename TA, int K, int NOUT, int EPI>
-__global__ void __launch_bounds__(128) k_gemm(const TA* __restrict__ X, int ldx, int M, const bf16* __restrict__ W,
-                                              const float* __restrict__ bias, const bf16* __restrict__ R, int ldr,
+__global__ void __launch_bounds__(128) k_gemm(const TA* X, int ldx, int M, const bf16* __restrict__ W,
+                                              const float* __restrict__ bias, const bf16* R, int ldr,
                                               bf16* __restrict__ Y1, int ld1, bf16* __restrict__ Y2, int ld2,
                                               float* __restrict__ Yf, int ldf, float* __restrict__ Yg, int ldg,
                                               const float* __restrict__ rs)
@@ -86,6 +120,7 @@ __global__ void __launch_bounds__(128) k_gemm(const TA* __restrict__ X, int ldx,
     }
     for (int i = threadIdx.x; i < NOUT; i += 128) sb[i] = bias ? bias[i] : 0.f;
     __syncthreads();
+    after_previous();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int ntile = (M + 15) >> 4, stride = gridDim.x * 4;
     // A fragments of row tile `tl` (zero rows past M)
@@ -219,8 +254,8 @@ template <typename TA, int K, int NOUT, int EPI>
 void gemm(cudaStream_t st, const TA* X, int ldx, int M, const bf16* W, const float* bias, const bf16* R, int ldr,
           bf16* Y1, int ld1, bf16* Y2, int ld2, float* Yf, int ldf, float* Yg = nullptr, int ldg = 0, const float* rs = nullptr)
 {
-    k_gemm<TA, K, NOUT, EPI><<<gemm_grid<TA, K, NOUT, EPI>(M), 128, 0, st>>>(X, ldx, M, W, bias, R, ldr, Y1, ld1, Y2,
-                                                                            ld2, Yf, ldf, Yg, ldg, rs);
+    launch_after(k_gemm<TA, K, NOUT, EPI>, gemm_grid<TA, K, NOUT, EPI>(M), 128, 0, st, X, ldx, M, W, bias, R, ldr, Y1, ld1,
+                 Y2, ld2, Yf, ldf, Yg, ldg, rs);
 }
 
 // ---- fused inference kernels ----------------------------------------------
@@ -311,11 +346,11 @@ struct FusedShape {
 };
 
 template <int MODE>
-__global__ void __launch_bounds__(128, 4) k_fused(const bf16* __restrict__ X, int ldx, int M,
+__global__ void __launch_bounds__(128, 4) k_fused(const bf16* X, int ldx, int M,
                                                   const bf16* __restrict__ W1, const float* __restrict__ b1,
                                                   const bf16* __restrict__ W2, const float* __restrict__ b2,
                                                   bf16* __restrict__ hout, int ldh, bf16* __restrict__ pq,
-                                                  const float4* __restrict__ A, const float4* __restrict__ Dp,
+                                                  const float4* A, const float4* Dp,
                                                   float4* __restrict__ warm)
 {
     using S = FusedShape<MODE>;
@@ -335,6 +370,7 @@ __global__ void __launch_bounds__(128, 4) k_fused(const bf16* __restrict__ X, in
     for (int i = threadIdx.x; i < H; i += 128) sb1[i] = b1[i];
     for (int i = threadIdx.x; i < N2; i += 128) sb2[i] = b2 ? b2[i] : 0.f;
     __syncthreads();
+    after_previous();
     const unsigned full = 0xffffffffu;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     bf16* sO = sW2 + N2 * (H + 8) + warp * 16 * (S::OCOLS + 8);   // this warp's output tile
@@ -460,7 +496,7 @@ void fused(cudaStream_t st, const bf16* X, int ldx, int M, const bf16* W1, const
 {
     const size_t smem = FusedShape<MODE>::smem;
     const int grid = resident_grid<k_fused<MODE>>(128, smem, ((((long long)M + 15) >> 4) + 3) / 4);
-    k_fused<MODE><<<grid, 128, smem, st>>>(X, ldx, M, W1, b1, W2, b2, hout, ldh, pq, A, Dp, warm);
+    launch_after(k_fused<MODE>, grid, 128, smem, st, X, ldx, M, W1, b1, W2, b2, hout, ldh, pq, A, Dp, warm);
 }
 
 __device__ __forceinline__ float tofloat(float v) { return v; }
@@ -512,8 +548,8 @@ __device__ __forceinline__ void ldsm_x4_t(const bf16* p, uint32_t& r0, uint32_t&
 // 16-byte alignment of the rows of dY and X is a multiple of ldy and ldx.
 // MASK: dY counts as zero where ref [M][NP] is not positive (ReLU backward).
 template <int NP, int KP, bool MASK>
-__global__ void __launch_bounds__(256) k_wgrad(const float* __restrict__ dY, int ldy, int nout,
-                                               const bf16* __restrict__ ref, int ldr, const bf16* __restrict__ X, int ldx, int K, int M,
+__global__ void __launch_bounds__(256) k_wgrad(const float* dY, int ldy, int nout,
+                                               const bf16* ref, int ldr, const bf16* X, int ldx, int K, int M,
                                                float* __restrict__ part)
 {
     constexpr int RT = kWgradRows, NT = 256;
@@ -533,6 +569,7 @@ __global__ void __launch_bounds__(256) k_wgrad(const float* __restrict__ dY, int
     // bias: each thread adds four columns of every (NT / (NP/4))-th row
     const int bc = (tid % (NP / 4)) * 4, br = tid / (NP / 4);
     float4 bacc = make_float4(0.f, 0.f, 0.f, 0.f);
+    after_previous();
     for (int r0 = blockIdx.x * RT; r0 < M; r0 += gridDim.x * RT) {
         __syncthreads();
         for (int r = br; r < RT; r += NT / (NP / 4)) {
@@ -625,11 +662,12 @@ __global__ void __launch_bounds__(256) k_sum_parts(SumTable t)
     __shared__ float sp[8][32];
     int j = 0;
     while (j + 1 < kSumSegs && (int)blockIdx.x >= t.first[j + 1]) ++j;
-    const float* __restrict__ part = t.part[j];
+    const float* part = t.part[j];
     const int nblocks = t.nblocks[j], nw = t.nw[j], width = nw + t.nbias[j];
     const int col = threadIdx.x & 31, grp = threadIdx.x >> 5;
     const int i = ((int)blockIdx.x - t.first[j]) * 32 + col;
     float s = 0.f;
+    after_previous();
     if (i < width) {
         #pragma unroll 8
         for (int b = grp; b < nblocks; b += 8) s += part[(size_t)b * width + i];
@@ -656,8 +694,8 @@ __global__ void __launch_bounds__(256) k_sum_parts(SumTable t)
 // backward pass, 16 bits per k of the channels 4s + k, bit s.
 template <bool MASK>
 __global__ void __launch_bounds__(256) k_msg_fwd(int N, const int* __restrict__ ptr, const int* __restrict__ adj,
-                                                 const float4* __restrict__ ef, const float* __restrict__ deg_inv,
-                                                 const bf16* __restrict__ PQ, const float* __restrict__ C,
+                                                 const float4* ef, const float* __restrict__ deg_inv,
+                                                 const bf16* PQ, const float* __restrict__ C,
                                                  const float* __restrict__ cb, bf16* __restrict__ cat,
                                                  uint2* __restrict__ mask)
 {
@@ -667,6 +705,7 @@ __global__ void __launch_bounds__(256) k_msg_fwd(int N, const int* __restrict__ 
     float cv[4];
     #pragma unroll
     for (int k = 0; k < 4; ++k) { Cw[k] = *reinterpret_cast<const float4*>(C + (ch + k) * EF); cv[k] = cb[ch + k]; }
+    after_previous();
     const int npair = (N + 1) >> 1, stride = gridDim.x * (blockDim.x >> 5);
     // the pair index is the same for the whole warp, so every lane takes
     // part in every shuffle below
@@ -753,7 +792,7 @@ void messages(cudaStream_t st, int N, const int* ptr, const int* adj, const floa
               const bf16* PQ, const float* C, const float* cb, bf16* cat, uint2* mask)
 {
     const int grid = resident_grid<k_msg_fwd<MASK>>(256, 0, ((((long long)N + 1) >> 1) + 7) / 8);
-    k_msg_fwd<MASK><<<grid, 256, 0, st>>>(N, ptr, adj, ef, deg_inv, PQ, C, cb, cat, mask);
+    launch_after(k_msg_fwd<MASK>, grid, 256, 0, st, N, ptr, adj, ef, deg_inv, PQ, C, cb, cat, mask);
 }
 
 // Backward of the messages: dP_i = sum_j g_ij, dQ_j = sum_i g_ij with
@@ -765,8 +804,8 @@ void messages(cudaStream_t st, int N, const int* ptr, const int* adj, const floa
 // edge instead of 296): 46 us for 54,440 nodes, now 30; gradients of a 160x160
 // graph 717 us, now 680.
 __global__ void __launch_bounds__(256) k_msg_bwd(int N, const int* __restrict__ ptr, const int* __restrict__ adj,
-                                                 const int* __restrict__ rev, const float4* __restrict__ ef,
-                                                 const uint2* __restrict__ mask, const float* __restrict__ da_s,
+                                                 const int* __restrict__ rev, const float4* ef, const uint2* mask,
+                                                 const float* da_s,
                                                  float* __restrict__ dpq, float* __restrict__ part)
 {
     __shared__ float red[16][H * (EF + 1)];
@@ -779,6 +818,7 @@ __global__ void __launch_bounds__(256) k_msg_bwd(int N, const int* __restrict__ 
         #pragma unroll
         for (int q = 0; q < EF; ++q) gC[k][q] = 0.f;
     }
+    after_previous();
     const int npair = (N + 1) >> 1, stride = gridDim.x * 8;
     // sign of channel 4s + k from an edge's mask
     auto on = [&](const uint2& m, int k) { return ((k < 2 ? m.x : m.y) >> ((k & 1) * 16 + s)) & 1u; };
@@ -867,13 +907,13 @@ __global__ void __launch_bounds__(256) k_msg_bwd(int N, const int* __restrict__ 
 // error, K approximated by a graph Laplacian with K's own diagonal.
 // dout_i = inv_cnt [2 d_i + 2 lam sum_j k_ij w_j (d_i - d_j)] w_i, one thread
 // per vertex, no atomics.
-__global__ void k_loss(int N, const float* __restrict__ out, const float* __restrict__ target,
-                       const float* __restrict__ freew, const int* __restrict__ ptr, const int* __restrict__ adj,
+__global__ void k_loss(int N, const float* out, const float* target, const float* freew, const int* __restrict__ ptr, const int* __restrict__ adj,
                        const float* __restrict__ ew, float lam, float inv_cnt, float* __restrict__ dout,
                        double* __restrict__ loss)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     float s = 0.f;
+    after_previous();
     if (i < N) {
         const float w = freew[i];
         float d[NO], gsum[NO];
@@ -932,11 +972,12 @@ __global__ void k_copies(int n, const float* __restrict__ p, Layout y, Bf16Weigh
     if (i < n) put_copy(y, W, bdp, i, p[i]);
 }
 
-__global__ void k_adam(int n, float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
+__global__ void k_adam(int n, float* __restrict__ p, const float* g, float* __restrict__ m,
                        float* __restrict__ v, float lr, float b1, float b2, float eps, float bc1, float bc2, Layout y,
                        Bf16Weights W, float* bdp)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    after_previous();
     if (i >= n) return;
     const float gi = g[i];
     const float mi = b1 * m[i] + (1.f - b1) * gi;
@@ -1025,9 +1066,10 @@ __global__ void k_node_feat(int N, const float4* __restrict__ X, const float4* _
 
 // edge features of (i <- j): log(rest / 1 cm), (y_j - y_i) / rest
 __global__ void k_edge_feat(int N, const int* __restrict__ ptr, const int* __restrict__ adj,
-                            const float* __restrict__ rest, const float4* __restrict__ Y, float4* __restrict__ ef)
+                            const float* __restrict__ rest, const float4* Y, float4* __restrict__ ef)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    after_previous();
     if (i >= N) return;
     const float4 yi = Y[i];
     for (int e = ptr[i]; e < ptr[i + 1]; ++e) {
@@ -1040,11 +1082,12 @@ __global__ void k_edge_feat(int N, const int* __restrict__ ptr, const int* __res
 // Target of the network: (x* - y - d_prev)/s, i.e. the change of the
 // converged offset since the previous frame where d_prev is valid (the
 // prediction adds d_prev back, a skip connection in fp32), and the free weight.
-__global__ void k_target(int N, const float4* __restrict__ Xs, const float4* __restrict__ Y,
-                         const float4* __restrict__ aux, const float4* __restrict__ Dp, float* __restrict__ target,
+__global__ void k_target(int N, const float4* Xs, const float4* Y,
+                         const float4* __restrict__ aux, const float4* Dp, float* __restrict__ target,
                          float* __restrict__ freew)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    after_previous();
     if (i >= N) return;
     const float4 x = Xs[i], y = Y[i];
     const float4 dp = Dp ? Dp[i] : make_float4(0.f, 0.f, 0.f, 0.f);
