@@ -22,16 +22,17 @@
 // must start at zero, and calls that overlap on the GPU (different streams,
 // or different host threads) race on it.
 //
-// The frame is one cooperative launch.  Its sweeps alternate two phases with a
-// grid barrier after each: the elements (one thread per triangle or hinge)
-// add their corner forces to the accumulator, the vertices take their update
-// and clear it.  What bounds it is latency, not bytes: a 129x129 cloth moves
-// about 5 MB per sweep through L2.  The former form issued five launches per
-// sweep (control, clear, triangles, hinges, update; three scalar atomics per
-// corner).  A frame of 32 sweeps at 129x129 took 875 us in that form, 355 us
-// as one launch with one 16-byte reduction per corner, and takes 220 us with
-// what a frame does not change kept in registers and one arrival per block
-// and barrier.  The float reductions add in any order, so results match
+// The frame is one cooperative launch: the elements (one thread per triangle
+// or hinge) add their corner forces to an accumulator, grid barrier, the
+// vertices are updated from it.  Where every element and vertex has its own
+// thread each element updates its corners itself (k_na_one), which leaves one
+// barrier per sweep; larger cloths take two (k_na_frame).  What bounds it is
+// latency, not bytes: a 129x129 cloth moves about 5 MB per sweep through L2.
+// A frame of 32 sweeps at 129x129 took 875 us as five launches per sweep
+// (control, clear, triangles, hinges, update; three scalar atomics per
+// corner), 220 us as one launch with two barriers per sweep, one 16-byte
+// reduction per corner and what a frame does not change kept in registers, and
+// takes 156 us now.  The float reductions add in any order, so results match
 // pdg_solver_step to rounding, not bitwise.
 #include <cuda_runtime.h>
 
@@ -102,28 +103,30 @@ struct NaArgs {
 
 // Barrier `phase` (1, 2, ...) of the frame over the grid: one arrival per
 // block on a count that only grows, polled until all blocks of the phase are
-// in.  False on every thread of a block once a wait, here or in another
-// block, gave up.
+// in.  False once a wait, here or in another block, gave up.  na_wait is the
+// part of one thread, between two block barriers.
+__device__ __forceinline__ bool na_wait(NaCtl* c, unsigned phase)
+{
+    const unsigned want = phase * gridDim.x;
+    __threadfence();
+    atomicAdd(&c->bar, 1u);
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(__cvta_generic_to_global(&c->bar)) : "memory");
+    if (v < want) {
+        const long long t0 = clock64();
+        do {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(__cvta_generic_to_global(&c->bar)) : "memory");
+            if (clock64() - t0 > kNaWaitCycles) { atomicCAS(&c->err, 0, 1); break; }
+        } while (v < want);
+    }
+    return v >= want;
+}
 __device__ __forceinline__ bool na_barrier(NaCtl* c, unsigned& phase)
 {
     __shared__ int ok;
     __syncthreads();
     ++phase;
-    if (threadIdx.x == 0) {
-        const unsigned want = phase * gridDim.x;
-        __threadfence();
-        atomicAdd(&c->bar, 1u);
-        unsigned v;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(__cvta_generic_to_global(&c->bar)) : "memory");
-        if (v < want) {
-            const long long t0 = clock64();
-            do {
-                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(__cvta_generic_to_global(&c->bar)) : "memory");
-                if (clock64() - t0 > kNaWaitCycles) { atomicCAS(&c->err, 0, 1); break; }
-            } while (v < want);
-        }
-        ok = v >= want;
-    }
+    if (threadIdx.x == 0) ok = na_wait(c, phase);
     __syncthreads();
     return ok != 0;
 }
@@ -172,11 +175,9 @@ __device__ __forceinline__ NaElem na_element(const NaArgs& a, long long q)
     return m;
 }
 
-// Adds the element's corner forces at offsets D to F.
-__device__ __forceinline__ void na_apply(const NaElem& m, const float4* D, float4* F)
+// Adds the element's corner forces at its corners' offsets to F.
+__device__ __forceinline__ void na_apply(const NaElem& m, float4 d0, float4 d1, float4 d2, float4 d3, float4* F)
 {
-    const float4 d0 = __ldcg(&D[m.i0]), d1 = __ldcg(&D[m.i1]), d2 = __ldcg(&D[m.i2]);
-    const float4 d3 = m.i3 >= 0 ? __ldcg(&D[m.i3]) : d0;
     const float3 e1 = fadd3(m.e1, na_sub(d1, d0)), e2 = fadd3(m.e2, na_sub(d2, d0));
     if (m.i3 < 0) {
         float3 c0, c1, c2;
@@ -195,13 +196,9 @@ __device__ __forceinline__ void na_apply(const NaElem& m, const float4* D, float
     }
 }
 
-// Two 512-thread blocks per SM at 64 registers: a 129x129 cloth's 80,000
-// elements are then one per thread on all 152 SMs.
-// ONE: no thread has more than one element; its element's constants and rest
-// of the prediction then stay in registers for the frame, so that a sweep's
-// only loads are the offsets of its corners (one trip to L2).  Likewise each
+// The frame at any size, two barriers per sweep: threads may have several
+// elements and vertices.  Two 512-thread blocks per SM at 64 registers.  Each
 // thread keeps its first vertex's mass, prediction and last two offsets.
-template <bool ONE>
 __global__ void __launch_bounds__(kNaThreads, 2) k_na_frame(NaArgs a)
 {
     __shared__ float red[kNaThreads / 32];
@@ -241,8 +238,6 @@ __global__ void __launch_bounds__(kNaThreads, 2) k_na_frame(NaArgs a)
         if (!na_barrier(ctl, phase)) return;
     }
 
-    NaElem el;
-    if (ONE && gtid < a.T + a.E) el = na_element(a, gtid);
     float4 vd = make_float4(0.f, 0.f, 0.f, 0.f), vp = vd, vy = vd;   // vertex gtid: d^k, d^(k-1), y
     if (gtid < a.N) { vd = __ldcg(&s.A[gtid]); vp = vd; vy = __ldcg(&s.Y[gtid]); }
 
@@ -274,10 +269,10 @@ __global__ void __launch_bounds__(kNaThreads, 2) k_na_frame(NaArgs a)
         const float4* D = (k & 1) ? s.B : s.A;
         float4* Dn = (k & 1) ? s.A : s.B;
         // elements
-        if (ONE) {
-            if (gtid < a.T + a.E) na_apply(el, D, s.F);
-        } else {
-            for (long long q = gtid; q < (long long)a.T + a.E; q += gstride) na_apply(na_element(a, q), D, s.F);
+        for (long long q = gtid; q < (long long)a.T + a.E; q += gstride) {
+            const NaElem m = na_element(a, q);
+            const float4 d0 = __ldcg(&D[m.i0]);
+            na_apply(m, d0, __ldcg(&D[m.i1]), __ldcg(&D[m.i2]), m.i3 >= 0 ? __ldcg(&D[m.i3]) : d0, s.F);
         }
         if (!na_barrier(ctl, phase)) return;
         // vertices; the accumulator is left clear for the next sweep
@@ -341,12 +336,188 @@ __global__ void __launch_bounds__(kNaThreads, 2) k_na_frame(NaArgs a)
     }
 }
 
+// The frame where no thread has more than one element or vertex: a sweep then
+// takes one grid barrier.  Each thread keeps its element's constants and its
+// corners' last two offsets in registers and forms the corners' updates itself
+// from the summed forces, as every other element at that corner does with the
+// same operations; the force sums rotate through three arrays (the one read,
+// the one added to, the one being cleared).  Phase p evaluates the forces at
+// d^p after taking the update of sweep p - 1; thread i < N also takes vertex i,
+// for the residual, the cleared sum and the frame's end.
+// With the corners' offsets read back from memory a sweep took two barriers
+// and two more trips to L2: 32 sweeps of a 129x129 cloth 220 us, now 156;
+// 100x100 195 us, now 134; 9x9 144 us, now 87.
+template <int NT>
+__global__ void __launch_bounds__(NT, 1) k_na_one(NaArgs a)
+{
+    __shared__ float red[NT / 32];
+    __shared__ int ok_s, done_s, status_s;
+    const Scratch s = a.s;
+    NaCtl* ctl = s.ctl;
+    const int gtid = blockIdx.x * NT + threadIdx.x;
+    const float h = a.h, h2 = fmul(h, h);
+    const int nsweep = a.cap + a.have_final;
+    const bool own = gtid < a.N, elem = gtid < a.T + a.E, has_own = (int)(blockIdx.x * NT) < a.N;
+    unsigned phase = 0;
+
+    // prediction, start offsets (A), cleared sums
+    if (gtid < a.cap + 2) s.acc[gtid] = 0.0;
+    for (int i = gtid + (int)gridDim.x * NT; i < a.cap + 2; i += (int)gridDim.x * NT) s.acc[i] = 0.0;
+    float4 vy = make_float4(0.f, 0.f, 0.f, 0.f), vd = vy;   // vertex gtid: y, d^k
+    if (own) {
+        vy.x = ffma(h2, a.ax, ffma(h, a.vel[3 * gtid], a.pos[3 * gtid]));
+        vy.y = ffma(h2, a.ay, ffma(h, a.vel[3 * gtid + 1], a.pos[3 * gtid + 1]));
+        vy.z = ffma(h2, a.az, ffma(h, a.vel[3 * gtid + 2], a.pos[3 * gtid + 2]));
+        vy.w = a.mass[gtid];
+        s.Y[gtid] = vy;
+        const float dg = a.diag[gtid];
+        s.A[gtid] = make_float4(0.f, 0.f, 0.f, dg > 1e-10f ? 1.0f / dg : 0.f);   // inertial start
+        s.F[gtid] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    if (!na_barrier(ctl, phase)) return;
+    if (a.P > 0) {
+        for (int q = gtid; q < a.P; q += (int)gridDim.x * NT) {
+            const int i = a.pin_idx[q];
+            const float4 y = __ldcg(&s.Y[i]);
+            s.A[i] = make_float4(fsub(a.pin_target[3 * q], y.x), fsub(a.pin_target[3 * q + 1], y.y),
+                                 fsub(a.pin_target[3 * q + 2], y.z), -1.f);
+        }
+        if (!na_barrier(ctl, phase)) return;
+    }
+
+    NaElem el;
+    float4 cd[4];            // corners: d^k, 1 / diagonal (pinned: -1)
+    float3 cp[4];            // d^(k-1)
+    float cm[4];             // mass
+    if (elem) {
+        el = na_element(a, gtid);
+        const int id[4] = {el.i0, el.i1, el.i2, el.i3 >= 0 ? el.i3 : el.i0};
+        #pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            cd[c] = __ldcg(&s.A[id[c]]);
+            cp[c] = f3(cd[c]);
+            cm[c] = __ldcg(&s.Y[id[c]]).w;
+        }
+    }
+    if (own) vd = __ldcg(&s.A[gtid]);
+    float3 vp = f3(vd);
+
+    // Y is not read again: the third array of the rotation
+    float4 *fr = s.Y, *fw = s.F, *fc = s.B;   // read, add to, clear
+    bool active = true;
+    float om = 1.f;
+    int nstop = 0;
+    for (int p = 0; p <= nsweep; ++p) {
+        const int k = p - 1;   // the sweep whose update is taken
+        float r2 = 0.f;
+        if (p > 0) {
+            const bool res_only = k >= a.cap;
+            if (!res_only) {   // Chebyshev weight of sweep k (the solver's recurrence)
+                if (!a.use_cheb || k < a.cheb_delay) om = 1.f;
+                else if (k == a.cheb_delay) om = fdiv(2.f, fsub(2.f, a.rho2));
+                else om = fdiv(4.f, fsub(4.f, fmul(a.rho2, om)));
+            }
+            const float w = res_only ? 1.f : om;
+            auto update = [&](float4& d, float3& dp, float m, float4 f, float& rv) {
+                const float4 dq = res_only ? d : make_float4(dp.x, dp.y, dp.z, 0.f);
+                const float4 o = update_consistent(d, make_float4(0.f, 0.f, 0.f, m), f3(f), dq, a.gamma, w, rv);
+                if (!res_only) { dp = f3(d); d = o; }
+            };
+            if (elem && p < nsweep) {
+                const float4 f0 = __ldcg(&fr[el.i0]), f1 = __ldcg(&fr[el.i1]), f2 = __ldcg(&fr[el.i2]);
+                const float4 f3_ = el.i3 >= 0 ? __ldcg(&fr[el.i3]) : f0;
+                float rv;
+                update(cd[0], cp[0], cm[0], f0, rv);
+                update(cd[1], cp[1], cm[1], f1, rv);
+                update(cd[2], cp[2], cm[2], f2, rv);
+                update(cd[3], cp[3], cm[3], f3_, rv);
+            }
+            if (own) update(vd, vp, vy.w, __ldcg(&fr[gtid]), r2);
+        }
+        if (p < nsweep) {
+            if (elem) na_apply(el, cd[0], cd[1], cd[2], cd[3], fw);
+            if (own) fc[gtid] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        // barrier; its thread also adds the block's residual before it and,
+        // with a tolerance, takes the decision about sweep k after it (the same
+        // in every block)
+        if (has_own && p > 0) {
+            r2 = warp_sum(r2);
+            if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = r2;
+        }
+        __syncthreads();
+        ++phase;
+        float v = 0.f;
+        if (has_own && p > 0 && threadIdx.x < 32) v = warp_sum(threadIdx.x < NT / 32 ? red[threadIdx.x] : 0.f);
+        if (threadIdx.x == 0) {
+            if (has_own && p > 0) atomicAdd(s.acc + k, (double)v);
+            ok_s = na_wait(ctl, phase);
+            int done = 0;
+            if (a.tol > 0.f && p > 0 && p < nsweep) {
+                const double acc0 = __ldcg(&s.acc[0]), rk2 = __ldcg(&s.acc[k]);
+                done = !isfinite(rk2) || rk2 <= (double)a.tol * (double)a.tol * acc0;
+            }
+            done_s = done;
+        }
+        __syncthreads();
+        if (!ok_s) return;
+        if (done_s) { active = false; nstop = k; break; }
+        float4* t = fr; fr = fw; fw = fc; fc = t;
+    }
+
+    // the frame's outcome from the sums, found by every block for itself
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        // without a tolerance no decision was taken: the first sum that is not
+        // finite ended the frame
+        int bad = 0x7fffffff;
+        bool finite = true;
+        for (int k = lane; k <= a.cap; k += 32) {
+            const bool f = isfinite(__ldcg(&s.acc[k]));
+            finite = finite && f;
+            if (active && !f && k + 1 < nsweep) bad = min(bad, k);
+        }
+        bad = __reduce_min_sync(0xffffffffu, bad);
+        finite = __all_sync(0xffffffffu, finite) != 0;
+        if (lane == 0) {
+            const int j = !active ? nstop : (bad != 0x7fffffff ? bad : -1);   // ended after sweep j
+            const int used = j >= 0 ? j : a.cap;
+            const double rf = j >= 0 || a.have_final ? __ldcg(&s.acc[used]) : -1.0;
+            status_s = j >= 0 ? (isfinite(rf) ? 0 : -6) : (finite ? 0 : -6);
+            if (blockIdx.x == 0) {
+                const double acc0 = __ldcg(&s.acc[0]);
+                ctl->res0_2 = acc0; ctl->res_y2 = acc0; ctl->resf_2 = rf;
+                ctl->used = used; ctl->status = status_s; ctl->active = 0;
+            }
+        }
+    }
+    __syncthreads();
+    const float sc = 1.f - a.damping, ih = fdiv(1.f, h);
+    if (own && vd.w >= 0.f) {   // (pinned: written below)
+        const float3 d = active ? f3(vd) : vp;
+        if (status_s != 0) {    // failed frame: keep x_n, stop the cloth
+            a.vel[3 * gtid] = 0.f; a.vel[3 * gtid + 1] = 0.f; a.vel[3 * gtid + 2] = 0.f;
+        } else {
+            a.vel[3 * gtid] = fmul(sc, ffma(d.x, ih, ffma(h, a.ax, a.vel[3 * gtid])));
+            a.vel[3 * gtid + 1] = fmul(sc, ffma(d.y, ih, ffma(h, a.ay, a.vel[3 * gtid + 1])));
+            a.vel[3 * gtid + 2] = fmul(sc, ffma(d.z, ih, ffma(h, a.az, a.vel[3 * gtid + 2])));
+            a.pos[3 * gtid] = fadd(vy.x, d.x); a.pos[3 * gtid + 1] = fadd(vy.y, d.y); a.pos[3 * gtid + 2] = fadd(vy.z, d.z);
+        }
+    }
+    for (int q = gtid; q < a.P; q += (int)gridDim.x * NT) {
+        const int i = a.pin_idx[q];
+        a.pos[3 * i] = a.pin_target[3 * q]; a.pos[3 * i + 1] = a.pin_target[3 * q + 1]; a.pos[3 * i + 2] = a.pin_target[3 * q + 2];
+        a.vel[3 * i] = 0.f; a.vel[3 * i + 1] = 0.f; a.vel[3 * i + 2] = 0.f;
+    }
+}
+
 // Device address of the scratch array, looked up once per device.
 std::mutex g_mu;
 unsigned char* g_addr[64] = {};
-int g_blocks[64] = {};   // blocks of k_na_frame resident at once
+int g_blocks[64] = {};   // blocks of k_na_frame resident at once (of k_na_one: one per SM)
+int g_sms[64] = {};
 
-int scratch_of(int dev, unsigned char** out, int* blocks)
+int scratch_of(int dev, unsigned char** out, int* blocks, int* sms)
 {
     if (dev < 0 || dev >= 64) return set_error(PDG_ERR_ARG, "pdg_step_noalloc: device %d out of range", dev);
     std::lock_guard<std::mutex> lock(g_mu);
@@ -355,17 +526,17 @@ int scratch_of(int dev, unsigned char** out, int* blocks)
         const cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
         if (e != cudaSuccess || !p)
             return set_error(PDG_ERR_CUDA, "pdg_step_noalloc: cudaGetSymbolAddress failed: %s", cudaGetErrorString(e));
-        int nsm = 0, per = 0, per2 = 0;
+        int nsm = 0, per = 0;
         if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_na_frame<true>, kNaThreads, 0) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per2, k_na_frame<false>, kNaThreads, 0) != cudaSuccess ||
-            std::min(per, per2) <= 0)
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_na_frame, kNaThreads, 0) != cudaSuccess || per <= 0)
             return set_error(PDG_ERR_CUDA, "pdg_step_noalloc: occupancy query failed");
-        g_blocks[dev] = nsm * std::min(per, per2);
+        g_blocks[dev] = nsm * per;
+        g_sms[dev] = nsm;
         g_addr[dev] = static_cast<unsigned char*>(p);
     }
     *out = g_addr[dev];
     *blocks = g_blocks[dev];
+    *sms = g_sms[dev];
     return PDG_OK;
 }
 
@@ -413,8 +584,8 @@ extern "C" int pdg_step_noalloc(const pdg_config* cfg, int N, float* d_pos, floa
                              sdev, dev);
     }
     unsigned char* base = nullptr;
-    int max_blocks = 0;
-    const int rc = scratch_of(dev, &base, &max_blocks);
+    int max_blocks = 0, nsm = 0;
+    const int rc = scratch_of(dev, &base, &max_blocks, &nsm);
     if (rc) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
 
@@ -430,14 +601,24 @@ extern "C" int pdg_step_noalloc(const pdg_config* cfg, int N, float* d_pos, floa
     a.cap = cfg->max_iterations;
     a.have_final = (cfg->compute_final_residual || cfg->tolerance > 0.f) ? 1 : 0;
     a.use_cheb = cfg->use_chebyshev; a.cheb_delay = cfg->cheb_delay;
-    // one element per thread as far as the resident blocks go
     const long long work = std::max((long long)T + E, (long long)N);
-    const int grid = (int)std::max(1LL, std::min((long long)max_blocks, (work + kNaThreads - 1) / kNaThreads));
     NA_CK(cudaMemsetAsync(a.s.ctl, 0, sizeof(NaCtl), st));
     void* args[] = {&a};
-    const void* kernel = (long long)T + E <= (long long)grid * kNaThreads ? (const void*)k_na_frame<true>
-                                                                          : (const void*)k_na_frame<false>;
-    NA_CK(cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(kNaThreads), args, 0, st));
+    // One block per SM, of the fewest threads that give each element and vertex
+    // its own: a barrier waits for few arrivals and a block's barrier for few
+    // warps.  32 sweeps of a 33x33 cloth take 97 us in blocks of 128 threads,
+    // 139 of 640; 100x100 134 us in blocks of 512 (one per SM), 135 of 256 and
+    // 140 of 128 (two and four per SM); 129x129 156 us in blocks of 640, 160
+    // of 320 and 192 of 128.
+    struct { int nt; const void* kernel; } const one[] = {
+        {128, (const void*)k_na_one<128>}, {256, (const void*)k_na_one<256>}, {512, (const void*)k_na_one<512>},
+        {640, (const void*)k_na_one<640>}, {768, (const void*)k_na_one<768>}, {1024, (const void*)k_na_one<1024>}};
+    int nt = kNaThreads, blocks = max_blocks;
+    const void* kernel = (const void*)k_na_frame;
+    for (const auto& o : one)
+        if (work <= (long long)nsm * o.nt) { nt = o.nt; blocks = nsm; kernel = o.kernel; break; }
+    const int grid = (int)std::min((long long)blocks, (work + nt - 1) / nt);
+    NA_CK(cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(nt), args, 0, st));
 
     if (stats) {
         NaCtl c;
