@@ -569,13 +569,17 @@ __global__ void __launch_bounds__(256) k_wgrad(const float* dY, int ldy, int nou
     // bias: each thread adds four columns of every (NT / (NP/4))-th row
     const int bc = (tid % (NP / 4)) * 4, br = tid / (NP / 4);
     float4 bacc = make_float4(0.f, 0.f, 0.f, 0.f);
-    after_previous();
-    for (int r0 = blockIdx.x * RT; r0 < M; r0 += gridDim.x * RT) {
-        __syncthreads();
-        for (int r = br; r < RT; r += NT / (NP / 4)) {
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (r0 + r < M) {
-                v = *reinterpret_cast<const float4*>(dY + (size_t)(r0 + r) * ldy + bc);
+    // this thread's pieces of a tile, read one tile ahead
+    constexpr int BR = NT / (NP / 4), PY = (RT + BR - 1) / BR, PX = (RT * (KP / 8) + NT - 1) / NT;
+    float4 vy[PY];
+    uint4 vx[PX];
+    auto fetch = [&](int r0) {
+        #pragma unroll
+        for (int i = 0; i < PY; ++i) {
+            const int r = br + i * BR;
+            vy[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (r < RT && r0 + r < M) {
+                float4 v = *reinterpret_cast<const float4*>(dY + (size_t)(r0 + r) * ldy + bc);
                 if (MASK) {
                     const uint2 u = *reinterpret_cast<const uint2*>(ref + (size_t)(r0 + r) * ldr + bc);
                     const float2 m01 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
@@ -583,7 +587,25 @@ __global__ void __launch_bounds__(256) k_wgrad(const float* dY, int ldy, int nou
                     v = make_float4(m01.x > 0.f ? v.x : 0.f, m01.y > 0.f ? v.y : 0.f, m23.x > 0.f ? v.z : 0.f,
                                     m23.y > 0.f ? v.w : 0.f);
                 }
+                vy[i] = v;
             }
+        }
+        #pragma unroll
+        for (int i = 0; i < PX; ++i) {
+            const int e = tid + i * NT, r = e / (KP / 8), c = (e % (KP / 8)) * 8;
+            vx[i] = make_uint4(0u, 0u, 0u, 0u);
+            if (r < RT && r0 + r < M) vx[i] = *reinterpret_cast<const uint4*>(X + (size_t)(r0 + r) * ldx + c);
+        }
+    };
+    after_previous();
+    fetch(blockIdx.x * RT);
+    for (int r0 = blockIdx.x * RT; r0 < M; r0 += gridDim.x * RT) {
+        __syncthreads();
+        #pragma unroll
+        for (int i = 0; i < PY; ++i) {
+            const int r = br + i * BR;
+            if (r >= RT) break;
+            const float4 v = vy[i];
             bacc.x += v.x; bacc.y += v.y; bacc.z += v.z; bacc.w += v.w;
             __align__(8) bf16 h[4], m[4], l[4];
             split3(v.x, h[0], m[0], l[0]); split3(v.y, h[1], m[1], l[1]);
@@ -592,13 +614,13 @@ __global__ void __launch_bounds__(256) k_wgrad(const float* dY, int ldy, int nou
             *reinterpret_cast<uint2*>(&sy[1][r * SY + bc]) = *reinterpret_cast<const uint2*>(m);
             *reinterpret_cast<uint2*>(&sy[2][r * SY + bc]) = *reinterpret_cast<const uint2*>(l);
         }
-        for (int i = tid; i < RT * (KP / 8); i += NT) {
-            const int r = i / (KP / 8), c = (i % (KP / 8)) * 8;
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (r0 + r < M) v = *reinterpret_cast<const uint4*>(X + (size_t)(r0 + r) * ldx + c);
-            *reinterpret_cast<uint4*>(&sx[r * SX + c]) = v;
+        #pragma unroll
+        for (int i = 0; i < PX; ++i) {
+            const int e = tid + i * NT, r = e / (KP / 8), c = (e % (KP / 8)) * 8;
+            if (r < RT) *reinterpret_cast<uint4*>(&sx[r * SX + c]) = vx[i];
         }
         __syncthreads();
+        fetch(r0 + gridDim.x * RT);
         const int g = lane >> 3, q = lane & 7;
         #pragma unroll
         for (int ks = 0; ks < RT / 16; ++ks) {
