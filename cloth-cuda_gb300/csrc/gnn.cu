@@ -34,6 +34,7 @@ struct pdg_warmstart {
     DevBuf<int> ptr, adj, rev;
     DevBuf<float> rest, deg_inv;
     DevBuf<float4> ef, stat, Xn, Vn, Dn;
+    DevBuf<float4> Xd;    // the deep solve's x* in the trajectory's vertex order
     DevBuf<float> ew;     // per directed edge: weight of the energy-norm term of the loss
     DevBuf<uint2> mask[L];   // per edge: signs of the message's channels
     DevBuf<bf16> xin, cat[L], pq[L], uo[L], hfin;
@@ -553,10 +554,20 @@ int pdg_warmstart_train_pair(pdg_warmstart* w, pdg_solver* traj, pdg_solver* dee
     if (!w || !traj || !deep || w->solver != traj)
         return set_error(PDG_ERR_STATE, "pdg_warmstart_train_pair: the network must be attached to `traj`");
     if (deep == traj || deep->L.ntot != traj->L.ntot || deep->L.ncloth != traj->L.ncloth ||
-        deep->L.perm_global != traj->L.perm_global || deep->kernel == PDG_KERNEL_PERSISTENT ||
-        deep->kernel == PDG_KERNEL_RESIDENT)
+        deep->kernel == PDG_KERNEL_PERSISTENT || deep->kernel == PDG_KERNEL_RESIDENT)
         return set_error(PDG_ERR_ARG, "pdg_warmstart_train_pair: `deep` must solve the same cloths with the same "
                                       "vertex layout (same patch plan, per-sweep kernels)");
+    // (patch sizes that the plans chose themselves may differ: the state then
+    // goes from one vertex order to the other through the caller's)
+    const bool same = deep->L.perm_global == traj->L.perm_global;
+    int rc = PDG_OK;
+    if (!same) {
+        const std::vector<int>*a = nullptr, *b = nullptr;
+        if ((rc = usual_order(traj, &a)) || (rc = usual_order(deep, &b))) return rc;
+        if (*a != *b)
+            return set_error(PDG_ERR_ARG, "pdg_warmstart_train_pair: `deep` must solve the same cloths with the same "
+                                          "vertex layout (same patch plan, per-sweep kernels)");
+    }
     cudaStream_t st = traj->stream;
     const int N = w->N;
     GK(cudaStreamSynchronize(deep->stream));
@@ -564,10 +575,16 @@ int pdg_warmstart_train_pair(pdg_warmstart* w, pdg_solver* traj, pdg_solver* dee
     GK(cudaMemcpyAsync(w->Xn.p, traj->X.p, sizeof(float4) * N, cudaMemcpyDeviceToDevice, st));
     GK(cudaMemcpyAsync(w->Vn.p, traj->V.p, sizeof(float4) * N, cudaMemcpyDeviceToDevice, st));
     GK(cudaMemcpyAsync(w->Dn.p, traj->dprev.p, sizeof(float4) * N, cudaMemcpyDeviceToDevice, st));
-    GK(cudaMemcpyAsync(deep->X.p, traj->X.p, sizeof(float4) * N, cudaMemcpyDeviceToDevice, st));
-    GK(cudaMemcpyAsync(deep->V.p, traj->V.p, sizeof(float4) * N, cudaMemcpyDeviceToDevice, st));
+    if (same) {
+        GK(cudaMemcpyAsync(deep->X.p, traj->X.p, sizeof(float4) * N, cudaMemcpyDeviceToDevice, st));
+        GK(cudaMemcpyAsync(deep->V.p, traj->V.p, sizeof(float4) * N, cudaMemcpyDeviceToDevice, st));
+    } else {
+        GK(w->Xd.reserve(N));
+        GK(launch_take_state(traj->X.p, traj->V.p, traj->stage_x.p, traj->stage_v.p, traj->inv_global.p, N, st));
+        GK(launch_put_state(traj->stage_x.p, traj->stage_v.p, deep->X.p, deep->V.p, deep->inv_global.p, N, st, nullptr));
+    }
     GK(cudaStreamSynchronize(st));
-    int rc = pdg_solver_step(deep, 1, nullptr);   // the target: x* of this frame
+    rc = pdg_solver_step(deep, 1, nullptr);   // the target: x* of this frame
     if (rc) return rc;
     GK(cudaStreamSynchronize(deep->stream));
     rc = pdg_solver_step(traj, 1, nullptr);       // the trajectory and its kept offsets advance
@@ -576,7 +593,13 @@ int pdg_warmstart_train_pair(pdg_warmstart* w, pdg_solver* traj, pdg_solver* dee
     k_node_feat<<<nb(N, 256), 256, 0, st>>>(N, w->Xn.p, w->Vn.p, traj->Y.p, traj->aux.p, w->stat.p, traj->vcloth.p,
                                             traj->cinfo.p, w->Dn.p, w->xin.p);
     launch_after(k_edge_feat, nb(N, 256), 256, 0, st, N, w->ptr.p, w->adj.p, w->rest.p, traj->Y.p, w->ef.p);
-    launch_after(k_target, nb(N, 256), 256, 0, st, N, deep->X.p, traj->Y.p, traj->aux.p, w->Dn.p, w->target.p, w->freew.p);
+    const float4* xs = deep->X.p;
+    if (!same) {
+        GK(launch_take_state(deep->X.p, nullptr, traj->stage_x.p, nullptr, deep->inv_global.p, N, st));
+        GK(launch_put_state(traj->stage_x.p, nullptr, w->Xd.p, nullptr, traj->inv_global.p, N, st, nullptr));
+        xs = w->Xd.p;
+    }
+    launch_after(k_target, nb(N, 256), 256, 0, st, N, xs, traj->Y.p, traj->aux.p, w->Dn.p, w->target.p, w->freew.p);
     int nfree = 0;
     for (const auto& a : traj->L.aux) nfree += a.w >= 0.f ? 1 : 0;
     rc = forward(w, st);
@@ -587,7 +610,7 @@ int pdg_warmstart_train_pair(pdg_warmstart* w, pdg_solver* traj, pdg_solver* dee
         rc = adam_step(w, lr, st);
         if (rc) return rc;
     }
-    traj->launches += 3 + (2 + 3 * L) + (5 + 5 * L) + (lr > 0.f ? 1 : 0);
+    traj->launches += (same ? 3 : 7) + (2 + 3 * L) + (5 + 5 * L) + (lr > 0.f ? 1 : 0);
     double l = 0.0;
     GK(cudaMemcpyAsync(&l, w->loss.p, sizeof(double), cudaMemcpyDeviceToHost, st));
     GK(cudaStreamSynchronize(st));

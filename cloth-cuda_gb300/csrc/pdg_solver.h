@@ -137,6 +137,8 @@ struct pdg_solver {
     std::vector<pdg::ClothRT> h_rt;
     bool warm_valid = false;
     pdg_warmstart* ws = nullptr;   // attached learned warm start (not owned)
+    int open_verts = 0;            // patch size before the plan chose another one (0: it chose none)
+    std::vector<int> usual;        // vertex order at that size (usual_order)
     bool any_warm = false;         // some cloth asks for a learned start
     bool any_keep = false;         // some cloth always keeps it (PDG_INIT_WARMSTART_KEEP)
     std::vector<pdg_tune_entry> tune;   // autotuner candidate table
@@ -158,4 +160,6 @@ int warm_kernel_count();
 // start residuals)
 int warm_judge_sweeps(const pdg_warmstart* w);
 void warm_detach(pdg_warmstart* w, const pdg_solver* s);
+// solver.cpp: vertex order of the solver's cloths in patches of the usual size
+int usual_order(pdg_solver* s, const std::vector<int>** order);
 }  // namespace pdg

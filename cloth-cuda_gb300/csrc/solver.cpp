@@ -303,6 +303,23 @@ int stream_patch_verts(const std::vector<ClothSetup>& cl, int nsm)
     return cost(192, 4.85) < cost(256, 6.1) ? 192 : 256;
 }
 
+// The layout of a per-sweep plan with at most pv vertices per patch: fewer
+// (halved, in pv) where a patch would not fit shared memory.
+int per_sweep_layout(const pdg_solver* s, int smem_optin, int& pv, HostLayout& L, StreamArgs& sa, size_t& smem)
+{
+    for (;; pv /= 2) {
+        std::string err;
+        if (!build_layout(s->cloths, pv, L, err)) return set_error(PDG_ERR_ARG, "%s", err.c_str());
+        if (s->kernel == PDG_KERNEL_STREAM) {
+            stream_layout(s->nt, L.max_nown, L.max_nhalo, L.max_nlocal, L.max_vm_nslot, sa, smem);
+            if (smem + 2048 <= (size_t)smem_optin) return PDG_OK;
+        } else if (L.smem_bytes + 1024 <= (size_t)std::min(smem_optin, 200 * 1024)) {
+            return PDG_OK;
+        }
+        if (pv <= 16) return set_error(PDG_ERR_ARG, "mesh too dense for the shared-memory patch layout");
+    }
+}
+
 int build_graph(pdg_solver* s)
 {
     if (s->graph) { cudaGraphExecDestroy(s->graph); s->graph = nullptr; }
@@ -319,6 +336,32 @@ int build_graph(pdg_solver* s)
 }
 
 }  // namespace
+
+namespace pdg {
+
+// The vertex order that the solver's cloths have in patches of the usual size,
+// whatever size its own plan has: what two solvers over the same cloths have
+// in common where the plan chose the size.
+int usual_order(pdg_solver* s, const std::vector<int>** order)
+{
+    *order = &s->L.perm_global;
+    if (!s->open_verts) return PDG_OK;
+    if (s->usual.empty()) {
+        int dev = 0, smem_optin = 0, pv = s->open_verts;
+        CK(cudaGetDevice(&dev));
+        CK(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+        HostLayout L;
+        StreamArgs sa;
+        size_t smem = 0;
+        const int rc = per_sweep_layout(s, smem_optin, pv, L, sa, smem);
+        if (rc) return rc;
+        s->usual = L.perm_global;
+    }
+    *order = &s->usual;
+    return PDG_OK;
+}
+
+}  // namespace pdg
 
 // The cloths of a solver, checked: each mesh with its own constraints, valid
 // configurations, one mode.
@@ -417,19 +460,14 @@ int pdg::create_solver(int n, const pdg_config* cfgs, const pdg_mesh* const* mes
         }
     }
     // (a learned start sums its messages in layout order: its plan stays)
-    if (s->kernel == PDG_KERNEL_STREAM && !c0.patch_verts && !c0.block_threads && !s->any_warm)
+    if (s->kernel == PDG_KERNEL_STREAM && !c0.patch_verts && !c0.block_threads && !s->any_warm) {
+        const int open = s->patch_verts;
         s->patch_verts = stream_patch_verts(s->cloths, nsm);
-    for (; s->kernel != PDG_KERNEL_RESIDENT;) {
-        if (!build_layout(s->cloths, s->patch_verts, s->L, err)) return set_error(PDG_ERR_ARG, "%s", err.c_str());
-        if (s->kernel == PDG_KERNEL_STREAM) {
-            const HostLayout& L = s->L;
-            stream_layout(s->nt, L.max_nown, L.max_nhalo, L.max_nlocal, L.max_vm_nslot, s->sargs, s->stream_smem);
-            if (s->stream_smem + 2048 <= (size_t)smem_optin) break;
-        } else if (s->L.smem_bytes + 1024 <= (size_t)std::min(smem_optin, 200 * 1024)) {
-            break;
-        }
-        if (s->patch_verts <= 16) return set_error(PDG_ERR_ARG, "mesh too dense for the shared-memory patch layout");
-        s->patch_verts /= 2;
+        if (s->patch_verts != open) s->open_verts = open;
+    }
+    if (s->kernel != PDG_KERNEL_RESIDENT) {
+        const int rc = per_sweep_layout(s.get(), smem_optin, s->patch_verts, s->L, s->sargs, s->stream_smem);
+        if (rc) return rc;
     }
     if (stream) {
         s->stream = (cudaStream_t)stream;
