@@ -32,7 +32,7 @@
 // (control, clear, triangles, hinges, update; three scalar atomics per
 // corner), 220 us as one launch with two barriers per sweep, one 16-byte
 // reduction per corner and what a frame does not change kept in registers, and
-// takes 156 us now.  The float reductions add in any order, so results match
+// takes 145 us now.  The float reductions add in any order, so results match
 // pdg_solver_step to rounding, not bitwise.
 #include <cuda_runtime.h>
 
@@ -104,13 +104,14 @@ struct NaArgs {
 // Barrier `phase` (1, 2, ...) of the frame over the grid: one arrival per
 // block on a count that only grows, polled until all blocks of the phase are
 // in.  False once a wait, here or in another block, gave up.  na_wait is the
-// part of one thread, between two block barriers.
+// part of one thread, between two block barriers; its arrival releases what
+// the block did before (with a full fence and a relaxed arrival 32 sweeps of a
+// 129x129 cloth took 156 us instead of 150).
 __device__ __forceinline__ bool na_wait(NaCtl* c, unsigned phase)
 {
     const unsigned want = phase * gridDim.x;
-    __threadfence();
-    atomicAdd(&c->bar, 1u);
     unsigned v;
+    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(__cvta_generic_to_global(&c->bar)), "r"(1u) : "memory");
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(__cvta_generic_to_global(&c->bar)) : "memory");
     if (v < want) {
         const long long t0 = clock64();
@@ -345,8 +346,8 @@ __global__ void __launch_bounds__(kNaThreads, 2) k_na_frame(NaArgs a)
 // d^p after taking the update of sweep p - 1; thread i < N also takes vertex i,
 // for the residual, the cleared sum and the frame's end.
 // With the corners' offsets read back from memory a sweep took two barriers
-// and two more trips to L2: 32 sweeps of a 129x129 cloth 220 us, now 156;
-// 100x100 195 us, now 134; 9x9 144 us, now 87.
+// and two more trips to L2: 32 sweeps of a 129x129 cloth 220 us, now 145;
+// 100x100 195 us, now 127; 9x9 144 us, now 86.
 template <int NT>
 __global__ void __launch_bounds__(NT, 1) k_na_one(NaArgs a)
 {
@@ -438,19 +439,23 @@ __global__ void __launch_bounds__(NT, 1) k_na_one(NaArgs a)
             if (elem) na_apply(el, cd[0], cd[1], cd[2], cd[3], fw);
             if (own) fc[gtid] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        // barrier; its thread also adds the block's residual before it and,
-        // with a tolerance, takes the decision about sweep k after it (the same
-        // in every block)
+        // barrier; with a tolerance the decision about sweep k follows it (the
+        // same in every block), so the block's residual is added before the
+        // arrival, otherwise only after the last phase: the next barrier
+        // makes it visible (129x129: 145 us instead of 150)
         if (has_own && p > 0) {
             r2 = warp_sum(r2);
             if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = r2;
         }
         __syncthreads();
         ++phase;
-        float v = 0.f;
-        if (has_own && p > 0 && threadIdx.x < 32) v = warp_sum(threadIdx.x < NT / 32 ? red[threadIdx.x] : 0.f);
+        const bool late = !(a.tol > 0.f) && p < nsweep;
+        if (has_own && p > 0 && (threadIdx.x >> 5) == (late ? 1 : 0)) {
+            const int lane = threadIdx.x & 31;
+            const float v = warp_sum(lane < NT / 32 ? red[lane] : 0.f);
+            if (lane == 0) atomicAdd(s.acc + k, (double)v);
+        }
         if (threadIdx.x == 0) {
-            if (has_own && p > 0) atomicAdd(s.acc + k, (double)v);
             ok_s = na_wait(ctl, phase);
             int done = 0;
             if (a.tol > 0.f && p > 0 && p < nsweep) {
@@ -606,7 +611,7 @@ extern "C" int pdg_step_noalloc(const pdg_config* cfg, int N, float* d_pos, floa
     void* args[] = {&a};
     // One block per SM, of the fewest threads that give each element and vertex
     // its own: a barrier waits for few arrivals and a block's barrier for few
-    // warps.  32 sweeps of a 33x33 cloth take 97 us in blocks of 128 threads,
+    // warps.  Measured beside one another, 32 sweeps of a 33x33 cloth take 97 us in blocks of 128 threads,
     // 139 of 640; 100x100 134 us in blocks of 512 (one per SM), 135 of 256 and
     // 140 of 128 (two and four per SM); 129x129 156 us in blocks of 640, 160
     // of 320 and 192 of 128.
