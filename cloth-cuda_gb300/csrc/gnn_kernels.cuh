@@ -3,7 +3,7 @@
 // A 2-layer mesh message-passing network (hidden 64) predicts, per vertex,
 // the offset d = x* - y of the converged position from the inertial
 // prediction.  Node GEMMs run on the tensor cores (bf16 mma.sync m16n8k16,
-// fp32 accumulation, bf16 activations); edge messages are warp-per-node
+// fp32 accumulation, bf16 activations); edge messages are half-a-warp-per-node
 // gathers over the mesh adjacency (deterministic, no atomics); weight
 // gradients are fp32 per-block partial sums added in a fixed block order
 // (bitwise reproducible); Adam keeps fp32 master weights and refreshes their

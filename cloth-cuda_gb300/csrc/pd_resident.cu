@@ -247,7 +247,7 @@ __device__ __forceinline__ void compute_residual(float r2, float* red, double* a
 // RANGE (with TOL): sweeps p.k0 .. p.k1 - 1 of a frame whose prediction, start
 // and finalisation are other launches: the streaming plan's sweeps where its
 // patches all fit on the chip at once.  At 54,000 vertices in 128-vertex
-// patches a sweep takes 4.8 us, as launches of the streaming kernel 7.3 us.
+// patches a sweep takes 3.7 us, as launches of the streaming kernel 7.3 us.
 template <int MODE, int NT, bool IO, bool TOL, bool RANGE>
 __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistArgs p)
 {

@@ -1,5 +1,6 @@
 // Streaming sweep: one launch per Jacobi sweep (replayed from the frame's CUDA
-// graph) on a persistent grid of resident blocks.  Block b walks the patches
+// graph) on a persistent grid of resident blocks, for cloths whose patches do
+// not all fit the chip (those run pd_resident.cu's ranges).  Block b walks the patches
 // b, b + G, b + 2G, ... (G = grid size) and software-pipelines their staging
 // so that the memory round trips of patch p + G overlap the arithmetic of
 // patch p:

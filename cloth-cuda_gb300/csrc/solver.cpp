@@ -290,10 +290,10 @@ long long patch_count(const std::vector<ClothSetup>& cl, int pv)
 // the threads) took about 6.1 us, a 192-vertex one (255 cells, one round) 4.85
 // us; a part-filled last wave counts half of what it leaves empty, because the
 // next sweep's blocks start in it.  The rule picks the measured best on
-// 300x300 (256: 8.1 against 9.2 us per sweep), 333x500 (192: 11.8 against
-// 13.6), 400x400 (192: 12.4 against 13.9), 700x700 (256: 29.1 against 31.0),
-// 1025x1025 (256: 57.1 against 59.7) and batches of 32 and 96 cloths (256:
-// 14.2 against 16.5, 32.0 against 35.0); 513x513 keeps 256 (18.1 against 17.4).
+// 300x300 (256: 8.1 against 9.1 us per sweep), 333x500 (192: 11.7 against
+// 13.6), 400x400 (192: 12.2 against 13.6), 700x700 (256: 27.8 against 30.6),
+// 1025x1025 (256: 55.0 against 58.8) and a batch of 96 cloths (256: 30.7
+// against 34.4); 513x513 keeps 256 (17.6 against 17.2).
 int stream_patch_verts(const std::vector<ClothSetup>& cl, int nsm)
 {
     auto cost = [&](int pv, double us) {
@@ -399,9 +399,9 @@ int pdg::create_solver(int n, const pdg_config* cfgs, const pdg_mesh* const* mes
     s->mode = c0.mode;
     s->have_final = (c0.mode == PDG_MODE_CONSISTENT) && (c0.compute_final_residual || c0.tolerance > 0.f);
     // defaults: 256-vertex patches on 256 threads, the measured best plan of
-    // the streaming kernel (512-cloth batch 167.9 against 174.0 us per sweep
-    // at 128 / 128, 1025x1025 57.3 against 62.6 us) and of the per-patch
-    // graph kernel
+    // the per-patch graph kernel and, but for stream_patch_verts below, of the
+    // streaming kernel (96 cloths 30.7 against 31.9 us per sweep at 128 / 128,
+    // 1025x1025 55.0 against 58.5 us)
     s->nt = c0.block_threads ? c0.block_threads : 256;
     if (s->nt != 128 && s->nt != 256 && s->nt != 512)
         return set_error(PDG_ERR_ARG, "block_threads must be 128, 256 or 512");
@@ -477,7 +477,7 @@ int pdg::create_solver(int n, const pdg_config* cfgs, const pdg_mesh* const* mes
     }
     // Streaming plan: where every patch is resident at once, the resident
     // kernel runs the sweeps of a frame in one launch.  A sweep of 54,000
-    // vertices in 434 patches of 128 then takes 4.8 us instead of 7.3 us.
+    // vertices in 434 patches of 128 then takes 3.7 us instead of 7.3 us.
     if (s->kernel == PDG_KERNEL_STREAM && s->mode == PDG_MODE_CONSISTENT)
         s->range_variant = resident_range_pick(s->L.max_nown, s->L.npatch, s->L.smem_resident);
     int rc = upload_all(s.get());

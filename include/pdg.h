@@ -54,7 +54,8 @@ extern "C" {
                                     kernel (no timing)                       */
 #define PDG_KERNEL_GRAPH      1  /* one fused launch per iteration, frame in a CUDA graph */
 #define PDG_KERNEL_PERSISTENT 2  /* one cooperative launch per frame, bounded grid barrier */
-#define PDG_KERNEL_RESIDENT   3  /* persistent, one patch per block, records kept on chip */
+#define PDG_KERNEL_RESIDENT   3  /* one cooperative launch per frame, one patch
+                                    per block, records kept on chip          */
 #define PDG_KERNEL_AUTOTUNE   4  /* time every launch plan that fits (launch
                                     structure, patch size, threads per block)
                                     on this problem and keep the fastest;
@@ -64,7 +65,13 @@ extern "C" {
                                     persistent grid; each block stages its
                                     next patch's vertex data with bulk (TMA)
                                     and asynchronous copies while it solves
-                                    the current one                          */
+                                    the current one.  Where every patch is
+                                    resident at once, the sweeps of a frame
+                                    run in one cooperative launch instead.
+                                    patch_verts and block_threads 0: 192 or
+                                    256 vertices, whichever fills the last
+                                    wave of blocks better (256 with a learned
+                                    start), on 256 threads                   */
 
 /* Solver configuration.  Mirrors PDSolverConfig (include/pd_solver.h:4-15);
  * fields after `damping` extend it. */
@@ -370,7 +377,8 @@ int  pdg_warmstart_train_frame(pdg_warmstart* w, pdg_solver* s, float lr, float*
 /* Training on a trajectory of `traj` (the network attached to it) with the
  * targets of a deeper solve: `deep` solves the same cloths with the same
  * vertex layout (created from the same meshes, constraints and launch plan,
- * with a larger cap or a lower tolerance).  One step copies traj's state
+ * with a larger cap or a lower tolerance; patch sizes left open may come out
+ * differently).  One step copies traj's state
  * into `deep`, runs one frame of `deep` (the target x*), one frame of `traj`
  * (the trajectory and its kept offsets advance as in use), then one Adam
  * step (lr > 0) on (x_n, v_n, y, d_prev of traj) -> (x* - y - d_prev). */
