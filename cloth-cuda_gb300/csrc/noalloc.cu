@@ -32,7 +32,7 @@
 // (control, clear, triangles, hinges, update; three scalar atomics per
 // corner), 220 us as one launch with two barriers per sweep, one 16-byte
 // reduction per corner and what a frame does not change kept in registers, and
-// takes 145 us now.  The float reductions add in any order, so results match
+// takes 141 us now.  The float reductions add in any order, so results match
 // pdg_solver_step to rounding, not bitwise.
 #include <cuda_runtime.h>
 
@@ -152,6 +152,8 @@ __device__ __forceinline__ float3 na_sub(float4 p, float4 q)
     return make_float3(fsub(p.x, q.x), fsub(p.y, q.y), fsub(p.z, q.z));
 }
 
+// STEP 1: the predictions in an array, 2: paired with the offsets.
+template <int STEP>
 __device__ __forceinline__ NaElem na_element(const NaArgs& a, long long q)
 {
     NaElem m;
@@ -169,8 +171,8 @@ __device__ __forceinline__ NaElem na_element(const NaArgs& a, long long q)
         m.s = h2 * a.kb[e];
         m.nrest = a.nrest[e];
     }
-    const float4 y0 = __ldcg(&a.s.Y[m.i0]), y1 = __ldcg(&a.s.Y[m.i1]), y2 = __ldcg(&a.s.Y[m.i2]);
-    const float4 y3 = m.i3 >= 0 ? __ldcg(&a.s.Y[m.i3]) : y0;
+    const float4 y0 = a.s.Y[STEP * m.i0], y1 = a.s.Y[STEP * m.i1], y2 = a.s.Y[STEP * m.i2];
+    const float4 y3 = m.i3 >= 0 ? a.s.Y[STEP * m.i3] : y0;
     m.e1 = na_sub(y1, y0); m.e2 = na_sub(y2, y0); m.e3 = na_sub(y3, y0);
     m.y0 = f3(y0);
     return m;
@@ -197,144 +199,212 @@ __device__ __forceinline__ void na_apply(const NaElem& m, float4 d0, float4 d1, 
     }
 }
 
-// The frame at any size, two barriers per sweep: threads may have several
-// elements and vertices.  Two 512-thread blocks per SM at 64 registers.  Each
-// thread keeps its first vertex's mass, prediction and last two offsets.
-__global__ void __launch_bounds__(kNaThreads, 2) k_na_frame(NaArgs a)
+// The frame's outcome from the sums, found by a warp of every block for itself:
+// its status, and the frame's record (block 0).  stop: the sweep after which
+// the tolerance ended the frame, or -1.
+__device__ __forceinline__ void na_outcome(const NaArgs& a, int stop, int& status)
 {
-    __shared__ float red[kNaThreads / 32];
-    __shared__ int done_s;
     const Scratch s = a.s;
-    NaCtl* ctl = s.ctl;
-    const int gtid = blockIdx.x * kNaThreads + threadIdx.x, gstride = gridDim.x * kNaThreads;
-    const float h = a.h, h2 = fmul(h, h);
-    const int nsweep = a.cap + a.have_final;
-    unsigned phase = 0;
+    const int lane = threadIdx.x, nsweep = a.cap + a.have_final;
+    // without a tolerance no decision was taken: the first sum that is not
+    // finite ended the frame
+    int bad = 0x7fffffff;
+    bool finite = true;
+    for (int k = lane; k <= a.cap; k += 32) {
+        const bool f = isfinite(__ldcg(&s.acc[k]));
+        finite = finite && f;
+        if (stop < 0 && !f && k + 1 < nsweep) bad = min(bad, k);
+    }
+    bad = __reduce_min_sync(0xffffffffu, bad);
+    finite = __all_sync(0xffffffffu, finite) != 0;
+    if (lane == 0) {
+        const int j = stop >= 0 ? stop : (bad != 0x7fffffff ? bad : -1);   // ended after sweep j
+        const int used = j >= 0 ? j : a.cap;
+        const double rf = j >= 0 || a.have_final ? __ldcg(&s.acc[used]) : -1.0;
+        status = j >= 0 ? (isfinite(rf) ? 0 : -6) : (finite ? 0 : -6);
+        if (blockIdx.x == 0) {
+            const double acc0 = __ldcg(&s.acc[0]);
+            s.ctl->res0_2 = acc0; s.ctl->res_y2 = acc0; s.ctl->resf_2 = rf;
+            s.ctl->used = used; s.ctl->status = status; s.ctl->active = 0;
+        }
+    }
+}
 
-    // prediction, start offsets, cleared sums
-    for (int i = gtid; i < a.cap + 2; i += gstride) s.acc[i] = 0.0;
-    for (int i = gtid; i < a.N; i += gstride) {
-        float4 y;
-        y.x = ffma(h2, a.ax, ffma(h, a.vel[3 * i], a.pos[3 * i]));
-        y.y = ffma(h2, a.ay, ffma(h, a.vel[3 * i + 1], a.pos[3 * i + 1]));
-        y.z = ffma(h2, a.az, ffma(h, a.vel[3 * i + 2], a.pos[3 * i + 2]));
-        y.w = a.mass[i];
-        s.Y[i] = y;
-        const float dg = a.diag[i];
-        const float4 d0 = make_float4(0.f, 0.f, 0.f, dg > 1e-10f ? 1.0f / dg : 0.f);   // inertial start
-        s.A[i] = d0;
-        s.B[i] = d0;
-        s.F[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+// The barrier that ends sweep k: the block's residual (r2 of its threads) is
+// added to the sweep's sum, and with a tolerance the decision about sweep k
+// follows, the same in every block (done).  With a tolerance the residual is
+// added before the arrival, otherwise only after the last sweep: the next
+// barrier makes it visible (129x129: 145 us instead of 150).  False once a
+// wait gave up.
+template <int NT>
+__device__ __forceinline__ bool na_end_sweep(const NaArgs& a, unsigned& phase, int k, bool last, bool has_own, float r2,
+                                             int& done)
+{
+    __shared__ float red[NT / 32];
+    __shared__ int ok_s, done_s;
+    const bool sum = has_own && k >= 0;
+    if (sum) {
+        r2 = warp_sum(r2);
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = r2;
     }
-    if (!na_barrier(ctl, phase)) return;
-    if (a.P > 0) {
-        for (int q = gtid; q < a.P; q += gstride) {
-            const int i = a.pin_idx[q];
-            const float4 y = __ldcg(&s.Y[i]);
-            const float4 d = make_float4(fsub(a.pin_target[3 * q], y.x), fsub(a.pin_target[3 * q + 1], y.y),
-                                         fsub(a.pin_target[3 * q + 2], y.z), -1.f);
-            s.A[i] = d;
-            s.B[i] = d;
+    __syncthreads();
+    ++phase;
+    const bool late = !(a.tol > 0.f) && !last;
+    if (sum && (threadIdx.x >> 5) == (late ? 1 : 0)) {
+        const int lane = threadIdx.x & 31;
+        const float v = warp_sum(lane < NT / 32 ? red[lane] : 0.f);
+        if (lane == 0) atomicAdd(a.s.acc + k, (double)v);
+    }
+    if (threadIdx.x == 0) {
+        ok_s = na_wait(a.s.ctl, phase);
+        int d = 0;
+        if (a.tol > 0.f && k >= 0 && !last) {
+            const double acc0 = __ldcg(&a.s.acc[0]), rk2 = __ldcg(&a.s.acc[k]);
+            d = !isfinite(rk2) || rk2 <= (double)a.tol * (double)a.tol * acc0;
         }
-        if (!na_barrier(ctl, phase)) return;
+        done_s = d;
     }
+    __syncthreads();
+    done = done_s;
+    return ok_s != 0;
+}
 
-    float4 vd = make_float4(0.f, 0.f, 0.f, 0.f), vp = vd, vy = vd;   // vertex gtid: d^k, d^(k-1), y
-    if (gtid < a.N) { vd = __ldcg(&s.A[gtid]); vp = vd; vy = __ldcg(&s.Y[gtid]); }
+// Chebyshev weight of sweep k from that of the sweep before (the solver's
+// recurrence).
+__device__ __forceinline__ float na_omega(const NaArgs& a, int k, float om)
+{
+    if (!a.use_cheb || k < a.cheb_delay) return 1.f;
+    if (k == a.cheb_delay) return fdiv(2.f, fsub(2.f, a.rho2));
+    return fdiv(4.f, fsub(4.f, fmul(a.rho2, om)));
+}
 
-    bool active = true;
-    float om = 1.f;
-    for (int k = 0; k < nsweep; ++k) {
-        const bool res_only = k >= a.cap;
-        if (!res_only) {   // Chebyshev weight of sweep k (the solver's recurrence)
-            if (!a.use_cheb || k < a.cheb_delay) om = 1.f;
-            else if (k == a.cheb_delay) om = fdiv(2.f, fsub(2.f, a.rho2));
-            else om = fdiv(4.f, fsub(4.f, fmul(a.rho2, om)));
-        }
-        // the decision at the start of sweep k, the same in every block:
-        // converged or failed frames end here
-        if (k >= 1) {
-            if (threadIdx.x == 0) {
-                const double acc0 = __ldcg(&s.acc[0]), rk2 = __ldcg(&s.acc[k - 1]);
-                const bool bad = !isfinite(rk2);
-                const bool conv = a.tol > 0.f && rk2 <= (double)a.tol * (double)a.tol * acc0;
-                done_s = bad || conv;
-                if (blockIdx.x == 0) {
-                    if (k == 1) { ctl->res0_2 = acc0; ctl->res_y2 = acc0; }
-                    if (done_s) { ctl->status = bad ? -6 : 0; ctl->used = k - 1; ctl->resf_2 = rk2; ctl->active = 0; }
-                }
-            }
-            __syncthreads();
-            if (done_s) { active = false; break; }
-        }
-        const float4* D = (k & 1) ? s.B : s.A;
-        float4* Dn = (k & 1) ? s.A : s.B;
-        // elements
-        for (long long q = gtid; q < (long long)a.T + a.E; q += gstride) {
-            const NaElem m = na_element(a, q);
-            const float4 d0 = __ldcg(&D[m.i0]);
-            na_apply(m, d0, __ldcg(&D[m.i1]), __ldcg(&D[m.i2]), m.i3 >= 0 ? __ldcg(&D[m.i3]) : d0, s.F);
-        }
-        if (!na_barrier(ctl, phase)) return;
-        // vertices; the accumulator is left clear for the next sweep
-        float r2 = 0.f;
-        for (int i = gtid; i < a.N; i += gstride) {
-            const bool first = i == gtid;
-            const float4 f4 = __ldcg(&s.F[i]);
-            const float4 d = first ? vd : __ldcg(&D[i]), y = first ? vy : __ldcg(&s.Y[i]);
-            const float4 dp = res_only ? d : (first ? vp : __ldcg(&Dn[i]));
-            float rv;
-            const float4 o = update_consistent(d, y, make_float3(f4.x, f4.y, f4.z), dp, a.gamma, res_only ? 1.f : om, rv);
-            r2 += rv;
-            if (!res_only) Dn[i] = o;
-            s.F[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (first && !res_only) { vp = d; vd = o; }
-        }
-        block_residual<kNaThreads>(r2, red, s.acc + k);
-        if (!na_barrier(ctl, phase)) return;
+// A vertex's new state after the sweeps (d: its offset), or what a failed
+// frame leaves.
+__device__ __forceinline__ void na_finalize(const NaArgs& a, int i, float4 y, float3 d, int status)
+{
+    if (status != 0) {         // keep x_n, stop the cloth
+        a.vel[3 * i] = 0.f; a.vel[3 * i + 1] = 0.f; a.vel[3 * i + 2] = 0.f;
+        return;
     }
+    const float h = a.h, sc = 1.f - a.damping, ih = fdiv(1.f, h);
+    a.vel[3 * i] = fmul(sc, ffma(d.x, ih, ffma(h, a.ax, a.vel[3 * i])));
+    a.vel[3 * i + 1] = fmul(sc, ffma(d.y, ih, ffma(h, a.ay, a.vel[3 * i + 1])));
+    a.vel[3 * i + 2] = fmul(sc, ffma(d.z, ih, ffma(h, a.az, a.vel[3 * i + 2])));
+    a.pos[3 * i] = fadd(y.x, d.x); a.pos[3 * i + 1] = fadd(y.y, d.y); a.pos[3 * i + 2] = fadd(y.z, d.z);
+}
 
-    // the frame's record (block 0, a warp looks through the sums), known to
-    // the other blocks after one more barrier
-    if (blockIdx.x == 0 && threadIdx.x < 32) {
-        if (a.cap <= 1 && threadIdx.x == 0) { ctl->res0_2 = __ldcg(&s.acc[0]); ctl->res_y2 = __ldcg(&s.acc[0]); }
-        if (active) {
-            bool finite = true;
-            for (int k = threadIdx.x; k <= a.cap; k += 32) {
-                const double v = __ldcg(&s.acc[k]);
-                finite = finite && isfinite(v);
-            }
-            finite = __all_sync(0xffffffffu, finite) != 0;
-            if (threadIdx.x == 0) {
-                ctl->used = a.cap;
-                ctl->resf_2 = a.have_final ? __ldcg(&s.acc[a.cap]) : -1.0;
-                ctl->status = finite ? 0 : -6;
-                ctl->active = 0;
-            }
-        }
-    }
-    if (!na_barrier(ctl, phase)) return;
-    const int status = __ldcg(&ctl->status), used = __ldcg(&ctl->used);
-    const float4* D = (used & 1) ? s.B : s.A;
-    const float sc = 1.f - a.damping, ih = fdiv(1.f, h);
-    for (int i = gtid; i < a.N; i += gstride) {
-        const float4 d = __ldcg(&D[i]);
-        if (d.w < 0.f) continue;   // pinned: written below
-        if (status != 0) {         // failed frame: keep x_n, stop the cloth
-            a.vel[3 * i] = 0.f; a.vel[3 * i + 1] = 0.f; a.vel[3 * i + 2] = 0.f;
-            continue;
-        }
-        const float4 y = __ldcg(&s.Y[i]);
-        a.vel[3 * i] = fmul(sc, ffma(d.x, ih, ffma(h, a.ax, a.vel[3 * i])));
-        a.vel[3 * i + 1] = fmul(sc, ffma(d.y, ih, ffma(h, a.ay, a.vel[3 * i + 1])));
-        a.vel[3 * i + 2] = fmul(sc, ffma(d.z, ih, ffma(h, a.az, a.vel[3 * i + 2])));
-        a.pos[3 * i] = fadd(y.x, d.x); a.pos[3 * i + 1] = fadd(y.y, d.y); a.pos[3 * i + 2] = fadd(y.z, d.z);
-    }
+// Pinned vertices to their targets, at rest.
+__device__ __forceinline__ void na_pins(const NaArgs& a, int gtid, int gstride)
+{
     for (int q = gtid; q < a.P; q += gstride) {
         const int i = a.pin_idx[q];
         a.pos[3 * i] = a.pin_target[3 * q]; a.pos[3 * i + 1] = a.pin_target[3 * q + 1]; a.pos[3 * i + 2] = a.pin_target[3 * q + 2];
         a.vel[3 * i] = 0.f; a.vel[3 * i + 1] = 0.f; a.vel[3 * i + 2] = 0.f;
     }
+}
+
+// Prediction y of vertex i and its offset at the inertial start (d.w: 1 /
+// diagonal).
+__device__ __forceinline__ float4 na_predict(const NaArgs& a, int i, float4& d0)
+{
+    const float h = a.h, h2 = fmul(h, h);
+    const float dg = a.diag[i];
+    d0 = make_float4(0.f, 0.f, 0.f, dg > 1e-10f ? 1.0f / dg : 0.f);
+    float4 y;
+    y.x = ffma(h2, a.ax, ffma(h, a.vel[3 * i], a.pos[3 * i]));
+    y.y = ffma(h2, a.ay, ffma(h, a.vel[3 * i + 1], a.pos[3 * i + 1]));
+    y.z = ffma(h2, a.az, ffma(h, a.vel[3 * i + 2], a.pos[3 * i + 2]));
+    y.w = a.mass[i];
+    return y;
+}
+
+// Offset of pin q's vertex, whose prediction is y.
+__device__ __forceinline__ float4 na_pin_offset(const NaArgs& a, int q, float4 y)
+{
+    return make_float4(fsub(a.pin_target[3 * q], y.x), fsub(a.pin_target[3 * q + 1], y.y),
+                       fsub(a.pin_target[3 * q + 2], y.z), -1.f);
+}
+
+// The frame at any size, two barriers per sweep: threads may have several
+// elements and vertices.  Two 512-thread blocks per SM at 64 registers.  y and
+// d of a vertex lie in one 32-byte pair (the arrays Y and A as one), which an
+// element reads through L1: in two arrays read from L2 32 sweeps of a 257x257
+// cloth took 505 us, now 424; 360x360 738, now 615.  What bounds it is the
+// reductions and corner reads in L2 (327,000 elements a sweep at 257x257).
+// Each thread keeps its first vertex's mass, prediction and last two offsets.
+__global__ void __launch_bounds__(kNaThreads, 2) k_na_frame(NaArgs a)
+{
+    __shared__ int status_s;
+    const Scratch s = a.s;
+    float4* YD = s.Y;
+    const int gtid = blockIdx.x * kNaThreads + threadIdx.x, gstride = gridDim.x * kNaThreads;
+    const int nsweep = a.cap + a.have_final;
+    const bool has_own = (int)(blockIdx.x * kNaThreads) < a.N;
+    unsigned phase = 0;
+
+    // prediction, start offsets, cleared sums
+    for (int i = gtid; i < a.cap + 2; i += gstride) s.acc[i] = 0.0;
+    for (int i = gtid; i < a.N; i += gstride) {
+        float4 d0;
+        YD[2 * i] = na_predict(a, i, d0);
+        YD[2 * i + 1] = d0;
+        s.B[i] = d0;
+        s.F[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    if (!na_barrier(s.ctl, phase)) return;
+    if (a.P > 0) {
+        for (int q = gtid; q < a.P; q += gstride) {
+            const int i = a.pin_idx[q];
+            const float4 d = na_pin_offset(a, q, YD[2 * i]);
+            YD[2 * i + 1] = d;
+            s.B[i] = d;
+        }
+        if (!na_barrier(s.ctl, phase)) return;
+    }
+
+    float4 vd = make_float4(0.f, 0.f, 0.f, 0.f), vp = vd, vy = vd;   // vertex gtid: d^k, d^(k-1), y
+    if (gtid < a.N) { vy = YD[2 * gtid]; vd = YD[2 * gtid + 1]; vp = vd; }
+
+    int nstop = -1;
+    float om = 1.f;
+    for (int k = 0; k < nsweep; ++k) {
+        const bool res_only = k >= a.cap;
+        if (!res_only) om = na_omega(a, k, om);
+        for (long long q = gtid; q < (long long)a.T + a.E; q += gstride) {
+            const NaElem m = na_element<2>(a, q);
+            const float4 d0 = YD[2 * m.i0 + 1];
+            na_apply(m, d0, YD[2 * m.i1 + 1], YD[2 * m.i2 + 1], m.i3 >= 0 ? YD[2 * m.i3 + 1] : d0, s.F);
+        }
+        if (!na_barrier(s.ctl, phase)) return;
+        // vertices; the accumulator is left clear for the next sweep
+        float r2 = 0.f;
+        for (int i = gtid; i < a.N; i += gstride) {
+            const bool first = i == gtid;
+            const float4 f4 = s.F[i];
+            const float4 d = first ? vd : YD[2 * i + 1], y = first ? vy : YD[2 * i];
+            const float4 dp = res_only ? d : (first ? vp : s.B[i]);
+            float rv;
+            const float4 o = update_consistent(d, y, make_float3(f4.x, f4.y, f4.z), dp, a.gamma, res_only ? 1.f : om, rv);
+            r2 += rv;
+            s.F[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (res_only) continue;
+            YD[2 * i + 1] = o;
+            if (first) { vp = d; vd = o; } else s.B[i] = d;
+        }
+        int done;
+        if (!na_end_sweep<kNaThreads>(a, phase, k, k + 1 == nsweep, has_own, r2, done)) return;
+        if (done) { nstop = k; break; }
+    }
+
+    if (threadIdx.x < 32) na_outcome(a, nstop, status_s);
+    __syncthreads();
+    // (stopped after sweep k: d^k, which the sweep's update moved on from)
+    for (int i = gtid; i < a.N; i += gstride) {
+        const bool first = i == gtid;
+        const float4 d = first ? (nstop >= 0 ? vp : vd) : (nstop >= 0 ? s.B[i] : YD[2 * i + 1]);
+        if (d.w >= 0.f) na_finalize(a, i, first ? vy : YD[2 * i], f3(d), status_s);   // (pinned: below)
+    }
+    na_pins(a, gtid, gstride);
 }
 
 // The frame where no thread has more than one element or vertex: a sweep then
@@ -346,17 +416,16 @@ __global__ void __launch_bounds__(kNaThreads, 2) k_na_frame(NaArgs a)
 // d^p after taking the update of sweep p - 1; thread i < N also takes vertex i,
 // for the residual, the cleared sum and the frame's end.
 // With the corners' offsets read back from memory a sweep took two barriers
-// and two more trips to L2: 32 sweeps of a 129x129 cloth 220 us, now 145;
-// 100x100 195 us, now 127; 9x9 144 us, now 86.
+// and two more trips to L2: 32 sweeps of a 129x129 cloth 220 us, now 141;
+// 100x100 195 us, now 125; 9x9 144 us, now 83.  (The sums are read through L1,
+// which the barrier's acquiring load empties: 141 us, from L2 145.)
 template <int NT>
 __global__ void __launch_bounds__(NT, 1) k_na_one(NaArgs a)
 {
-    __shared__ float red[NT / 32];
-    __shared__ int ok_s, done_s, status_s;
+    __shared__ int status_s;
     const Scratch s = a.s;
     NaCtl* ctl = s.ctl;
     const int gtid = blockIdx.x * NT + threadIdx.x;
-    const float h = a.h, h2 = fmul(h, h);
     const int nsweep = a.cap + a.have_final;
     const bool own = gtid < a.N, elem = gtid < a.T + a.E, has_own = (int)(blockIdx.x * NT) < a.N;
     unsigned phase = 0;
@@ -366,22 +435,16 @@ __global__ void __launch_bounds__(NT, 1) k_na_one(NaArgs a)
     for (int i = gtid + (int)gridDim.x * NT; i < a.cap + 2; i += (int)gridDim.x * NT) s.acc[i] = 0.0;
     float4 vy = make_float4(0.f, 0.f, 0.f, 0.f), vd = vy;   // vertex gtid: y, d^k
     if (own) {
-        vy.x = ffma(h2, a.ax, ffma(h, a.vel[3 * gtid], a.pos[3 * gtid]));
-        vy.y = ffma(h2, a.ay, ffma(h, a.vel[3 * gtid + 1], a.pos[3 * gtid + 1]));
-        vy.z = ffma(h2, a.az, ffma(h, a.vel[3 * gtid + 2], a.pos[3 * gtid + 2]));
-        vy.w = a.mass[gtid];
+        vy = na_predict(a, gtid, vd);
         s.Y[gtid] = vy;
-        const float dg = a.diag[gtid];
-        s.A[gtid] = make_float4(0.f, 0.f, 0.f, dg > 1e-10f ? 1.0f / dg : 0.f);   // inertial start
+        s.A[gtid] = vd;
         s.F[gtid] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     if (!na_barrier(ctl, phase)) return;
     if (a.P > 0) {
         for (int q = gtid; q < a.P; q += (int)gridDim.x * NT) {
             const int i = a.pin_idx[q];
-            const float4 y = __ldcg(&s.Y[i]);
-            s.A[i] = make_float4(fsub(a.pin_target[3 * q], y.x), fsub(a.pin_target[3 * q + 1], y.y),
-                                 fsub(a.pin_target[3 * q + 2], y.z), -1.f);
+            s.A[i] = na_pin_offset(a, q, s.Y[i]);
         }
         if (!na_barrier(ctl, phase)) return;
     }
@@ -391,33 +454,28 @@ __global__ void __launch_bounds__(NT, 1) k_na_one(NaArgs a)
     float3 cp[4];            // d^(k-1)
     float cm[4];             // mass
     if (elem) {
-        el = na_element(a, gtid);
+        el = na_element<1>(a, gtid);
         const int id[4] = {el.i0, el.i1, el.i2, el.i3 >= 0 ? el.i3 : el.i0};
         #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            cd[c] = __ldcg(&s.A[id[c]]);
+            cd[c] = s.A[id[c]];
             cp[c] = f3(cd[c]);
-            cm[c] = __ldcg(&s.Y[id[c]]).w;
+            cm[c] = s.Y[id[c]].w;
         }
     }
-    if (own) vd = __ldcg(&s.A[gtid]);
+    if (own) vd = s.A[gtid];
     float3 vp = f3(vd);
 
     // Y is not read again: the third array of the rotation
     float4 *fr = s.Y, *fw = s.F, *fc = s.B;   // read, add to, clear
-    bool active = true;
     float om = 1.f;
-    int nstop = 0;
+    int nstop = -1;
     for (int p = 0; p <= nsweep; ++p) {
         const int k = p - 1;   // the sweep whose update is taken
         float r2 = 0.f;
         if (p > 0) {
             const bool res_only = k >= a.cap;
-            if (!res_only) {   // Chebyshev weight of sweep k (the solver's recurrence)
-                if (!a.use_cheb || k < a.cheb_delay) om = 1.f;
-                else if (k == a.cheb_delay) om = fdiv(2.f, fsub(2.f, a.rho2));
-                else om = fdiv(4.f, fsub(4.f, fmul(a.rho2, om)));
-            }
+            if (!res_only) om = na_omega(a, k, om);
             const float w = res_only ? 1.f : om;
             auto update = [&](float4& d, float3& dp, float m, float4 f, float& rv) {
                 const float4 dq = res_only ? d : make_float4(dp.x, dp.y, dp.z, 0.f);
@@ -425,95 +483,30 @@ __global__ void __launch_bounds__(NT, 1) k_na_one(NaArgs a)
                 if (!res_only) { dp = f3(d); d = o; }
             };
             if (elem && p < nsweep) {
-                const float4 f0 = __ldcg(&fr[el.i0]), f1 = __ldcg(&fr[el.i1]), f2 = __ldcg(&fr[el.i2]);
-                const float4 f3_ = el.i3 >= 0 ? __ldcg(&fr[el.i3]) : f0;
+                const float4 f0 = fr[el.i0], f1 = fr[el.i1], f2 = fr[el.i2];
+                const float4 f3_ = el.i3 >= 0 ? fr[el.i3] : f0;
                 float rv;
                 update(cd[0], cp[0], cm[0], f0, rv);
                 update(cd[1], cp[1], cm[1], f1, rv);
                 update(cd[2], cp[2], cm[2], f2, rv);
                 update(cd[3], cp[3], cm[3], f3_, rv);
             }
-            if (own) update(vd, vp, vy.w, __ldcg(&fr[gtid]), r2);
+            if (own) update(vd, vp, vy.w, fr[gtid], r2);
         }
         if (p < nsweep) {
             if (elem) na_apply(el, cd[0], cd[1], cd[2], cd[3], fw);
             if (own) fc[gtid] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        // barrier; with a tolerance the decision about sweep k follows it (the
-        // same in every block), so the block's residual is added before the
-        // arrival, otherwise only after the last phase: the next barrier
-        // makes it visible (129x129: 145 us instead of 150)
-        if (has_own && p > 0) {
-            r2 = warp_sum(r2);
-            if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = r2;
-        }
-        __syncthreads();
-        ++phase;
-        const bool late = !(a.tol > 0.f) && p < nsweep;
-        if (has_own && p > 0 && (threadIdx.x >> 5) == (late ? 1 : 0)) {
-            const int lane = threadIdx.x & 31;
-            const float v = warp_sum(lane < NT / 32 ? red[lane] : 0.f);
-            if (lane == 0) atomicAdd(s.acc + k, (double)v);
-        }
-        if (threadIdx.x == 0) {
-            ok_s = na_wait(ctl, phase);
-            int done = 0;
-            if (a.tol > 0.f && p > 0 && p < nsweep) {
-                const double acc0 = __ldcg(&s.acc[0]), rk2 = __ldcg(&s.acc[k]);
-                done = !isfinite(rk2) || rk2 <= (double)a.tol * (double)a.tol * acc0;
-            }
-            done_s = done;
-        }
-        __syncthreads();
-        if (!ok_s) return;
-        if (done_s) { active = false; nstop = k; break; }
+        int done;
+        if (!na_end_sweep<NT>(a, phase, k, p == nsweep, has_own, r2, done)) return;
+        if (done) { nstop = k; break; }
         float4* t = fr; fr = fw; fw = fc; fc = t;
     }
 
-    // the frame's outcome from the sums, found by every block for itself
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-        // without a tolerance no decision was taken: the first sum that is not
-        // finite ended the frame
-        int bad = 0x7fffffff;
-        bool finite = true;
-        for (int k = lane; k <= a.cap; k += 32) {
-            const bool f = isfinite(__ldcg(&s.acc[k]));
-            finite = finite && f;
-            if (active && !f && k + 1 < nsweep) bad = min(bad, k);
-        }
-        bad = __reduce_min_sync(0xffffffffu, bad);
-        finite = __all_sync(0xffffffffu, finite) != 0;
-        if (lane == 0) {
-            const int j = !active ? nstop : (bad != 0x7fffffff ? bad : -1);   // ended after sweep j
-            const int used = j >= 0 ? j : a.cap;
-            const double rf = j >= 0 || a.have_final ? __ldcg(&s.acc[used]) : -1.0;
-            status_s = j >= 0 ? (isfinite(rf) ? 0 : -6) : (finite ? 0 : -6);
-            if (blockIdx.x == 0) {
-                const double acc0 = __ldcg(&s.acc[0]);
-                ctl->res0_2 = acc0; ctl->res_y2 = acc0; ctl->resf_2 = rf;
-                ctl->used = used; ctl->status = status_s; ctl->active = 0;
-            }
-        }
-    }
+    if (threadIdx.x < 32) na_outcome(a, nstop, status_s);
     __syncthreads();
-    const float sc = 1.f - a.damping, ih = fdiv(1.f, h);
-    if (own && vd.w >= 0.f) {   // (pinned: written below)
-        const float3 d = active ? f3(vd) : vp;
-        if (status_s != 0) {    // failed frame: keep x_n, stop the cloth
-            a.vel[3 * gtid] = 0.f; a.vel[3 * gtid + 1] = 0.f; a.vel[3 * gtid + 2] = 0.f;
-        } else {
-            a.vel[3 * gtid] = fmul(sc, ffma(d.x, ih, ffma(h, a.ax, a.vel[3 * gtid])));
-            a.vel[3 * gtid + 1] = fmul(sc, ffma(d.y, ih, ffma(h, a.ay, a.vel[3 * gtid + 1])));
-            a.vel[3 * gtid + 2] = fmul(sc, ffma(d.z, ih, ffma(h, a.az, a.vel[3 * gtid + 2])));
-            a.pos[3 * gtid] = fadd(vy.x, d.x); a.pos[3 * gtid + 1] = fadd(vy.y, d.y); a.pos[3 * gtid + 2] = fadd(vy.z, d.z);
-        }
-    }
-    for (int q = gtid; q < a.P; q += (int)gridDim.x * NT) {
-        const int i = a.pin_idx[q];
-        a.pos[3 * i] = a.pin_target[3 * q]; a.pos[3 * i + 1] = a.pin_target[3 * q + 1]; a.pos[3 * i + 2] = a.pin_target[3 * q + 2];
-        a.vel[3 * i] = 0.f; a.vel[3 * i + 1] = 0.f; a.vel[3 * i + 2] = 0.f;
-    }
+    if (own && vd.w >= 0.f) na_finalize(a, gtid, vy, nstop >= 0 ? vp : f3(vd), status_s);   // (pinned: below)
+    na_pins(a, gtid, (int)gridDim.x * NT);
 }
 
 // Device address of the scratch array, looked up once per device.
