@@ -303,6 +303,29 @@ int stream_patch_verts(const std::vector<ClothSetup>& cl, int nsm)
     return cost(192, 4.85) < cost(256, 6.1) ? 192 : 256;
 }
 
+// Patch size of the resident plan on 256-thread blocks (224 compute threads)
+// when the caller leaves the plan open, 0: the 512-thread blocks.  Patches of
+// at most 64 vertices, one per SM, take less time in the smaller blocks, whose
+// barriers wait for fewer warps (per 50 sweeps: 33x33 106.5 against 109.8 us,
+// 65x65 106.7 against 109.0, 97x97 109.6 against 113.0).  Beyond that two
+// patches per SM, as long as their records take one round of the threads (at
+// most 160 vertices): 129x129 123 against 129.5 us, 181x181 142 against 150,
+// 200x230 156.5 against 172; at 225x225 (176 vertices, two rounds) 185 against
+// 176.  With a tolerance the 512-thread blocks stay (129x129, 201 sweeps: 518
+// against 532 us).
+int resident_small_patch(const std::vector<ClothSetup>& cl, int nsm)
+{
+    for (const auto& c : cl)
+        if (c.cfg.tolerance > 0.f) return 0;
+    auto size_for = [&](long long blocks, int most) {
+        for (int pv = 24; pv <= most; pv += 8)
+            if (patch_count(cl, pv) <= blocks) return pv;
+        return 0;
+    };
+    const int one = size_for(nsm, 64);
+    return one ? one : size_for(2LL * nsm, 160);
+}
+
 // The layout of a per-sweep plan with at most pv vertices per patch: fewer
 // (halved, in pv) where a patch would not fit shared memory.
 int per_sweep_layout(const pdg_solver* s, int smem_optin, int& pv, HostLayout& L, StreamArgs& sa, size_t& smem)
@@ -429,20 +452,30 @@ int pdg::create_solver(int n, const pdg_config* cfgs, const pdg_mesh* const* mes
         // Resident kernel: every patch co-resident, one 512-thread block per
         // SM, or (block_threads = 256) two half-size patches per SM; a block
         // is rnt compute threads and one more warp.
-        const int rnt = (c0.kernel == PDG_KERNEL_RESIDENT && c0.block_threads == 256) ? 224 : 480;
+        int rnt = (c0.kernel == PDG_KERNEL_RESIDENT && c0.block_threads == 256) ? 224 : 480;
         const int per_sm = 512 / (rnt + 32);
         int ntot = 0;
         for (const auto& c : s->cloths) ntot += c.mesh->N;
         int P = c0.patch_verts;
         if (!P) P = std::min(rnt, std::max(32, ((ntot + per_sm * nsm - 1) / (per_sm * nsm) + 31) / 32 * 32));
-        // (more patches than blocks cannot fit: no layout is built for them)
-        bool ok = P <= rnt && patch_count(s->cloths, P) <= (long long)per_sm * nsm && build_layout(s->cloths, P, s->L, err);
         int variant = -1;
-        if (ok) {
-            variant = resident_pick(rnt);
-            ok = variant >= 0 && s->L.max_nown <= rnt &&
-                 s->L.smem_resident <= (size_t)std::min(smem_optin / per_sm - 8192, 216 * 1024);
-            if (ok) ok = s->L.npatch <= resident_max_blocks(s->mode, variant, s->L.smem_resident);
+        // (more patches than blocks cannot fit: no layout is built for them)
+        auto fits = [&](int pv, int nt, HostLayout& L) {
+            const int per = 512 / (nt + 32);
+            if (pv > nt || patch_count(s->cloths, pv) > (long long)per * nsm || !build_layout(s->cloths, pv, L, err))
+                return false;
+            variant = resident_pick(nt);
+            return variant >= 0 && L.max_nown <= nt &&
+                   L.smem_resident <= (size_t)std::min(smem_optin / per - 8192, 216 * 1024) &&
+                   L.npatch <= resident_max_blocks(s->mode, variant, L.smem_resident);
+        };
+        bool ok = fits(P, rnt, s->L);
+        const int small = ok && !c0.patch_verts && !c0.block_threads && s->mode == PDG_MODE_CONSISTENT
+                              ? resident_small_patch(s->cloths, nsm) : 0;
+        if (small) {
+            HostLayout L;
+            if (fits(small, 224, L)) { s->L = std::move(L); P = small; rnt = 224; }
+            else variant = resident_pick(rnt);
         }
         if (ok) {
             s->kernel = PDG_KERNEL_RESIDENT;
