@@ -308,22 +308,26 @@ int stream_patch_verts(const std::vector<ClothSetup>& cl, int nsm)
 // at most 64 vertices, one per SM, take less time in the smaller blocks, whose
 // barriers wait for fewer warps (per 50 sweeps: 33x33 106.5 against 109.8 us,
 // 65x65 106.7 against 109.0, 97x97 109.6 against 113.0).  Beyond that two
-// patches per SM, as long as their records take one round of the threads (at
-// most 160 vertices): 129x129 123 against 129.5 us, 181x181 142 against 150,
-// 200x230 156.5 against 172; at 225x225 (176 vertices, two rounds) 185 against
-// 176.  With a tolerance the 512-thread blocks stay (129x129, 201 sweeps: 518
-// against 532 us).
+// patches per SM, which overlap one another's waits, where their records take
+// no more rounds of the threads than one patch's of twice the size take of
+// 480: one up to 160 vertices (129x129 123 against 129.5 us, 181x181 142
+// against 150, 200x230 157 against 172), two above 192 (245x245 189 against
+// 205, 257x257 in 218 vertices 194 against 201); between them not (225x225 182
+// against 175, 235x235 187 against 184.5), nor above 220 (257x257 in 224
+// vertices 217).  With a tolerance the 512-thread blocks stay (129x129, 201
+// sweeps: 518 against 532 us).
 int resident_small_patch(const std::vector<ClothSetup>& cl, int nsm)
 {
     for (const auto& c : cl)
         if (c.cfg.tolerance > 0.f) return 0;
-    auto size_for = [&](long long blocks, int most) {
-        for (int pv = 24; pv <= most; pv += 8)
+    auto size_for = [&](long long blocks, int most, int step) {
+        for (int pv = 24; pv <= most; pv += step)
             if (patch_count(cl, pv) <= blocks) return pv;
         return 0;
     };
-    const int one = size_for(nsm, 64);
-    return one ? one : size_for(2LL * nsm, 160);
+    if (const int one = size_for(nsm, 64, 8)) return one;
+    const int two = size_for(2LL * nsm, 220, 1);
+    return two <= 160 || two > 192 ? two : 0;
 }
 
 // The layout of a per-sweep plan with at most pv vertices per patch: fewer

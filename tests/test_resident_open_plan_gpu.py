@@ -19,12 +19,13 @@ def solve(pdg, kern, shapes, tol, **plan):
     return states, [f["iterations"] for f in st], s.launch_info()
 
 
-# 81 and 3,025 vertices (24 per patch), 9,409 (64, one per SM), 12,769 (48, two),
-# 46,000 (152, two), 47,961 (160, two), 50,625 (one 352-vertex patch per SM);
+# 81 and 3,025 vertices (24 per patch), 9,409 (64, one per SM), 12,769 (43, two),
+# 46,000 (152, two), 47,961 (158, two), 50,625 (one 352-vertex patch per SM), 66,049
+# (218, two), 66,564 (219, two; 304 patches), 68,121 (one of 480);
 # cell centres; uneven cloths with a small last patch each
 @pytest.mark.parametrize("shapes,threads", [
     ([(9, 9, 1)], 256), ([(55, 55, 0)], 256), ([(97, 97, 1)], 256), ([(113, 113, 2)], 256), ([(200, 230, 1)], 256),
-    ([(219, 219, 1)], 256), ([(225, 225, 1)], 512), ([(77, 101, 3)], 256),
+    ([(219, 219, 1)], 256), ([(225, 225, 1)], 512), ([(257, 257, 1)], 256), ([(258, 258, 0)], 256), ([(261, 261, 1)], 512), ([(77, 101, 3)], 256),
     ([(33, 41, 1), (17, 17, 2), (60, 33, 0), (2, 2, 1)], 256)])
 @pytest.mark.parametrize("tol", [0.0, 1e-3])
 def test_open_resident_plan_matches_graph(pdg, shapes, threads, tol):
