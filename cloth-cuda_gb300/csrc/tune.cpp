@@ -74,6 +74,7 @@ std::vector<Plan> candidates(bool warm)
     std::vector<Plan> c;
     if (!warm) {
         c.push_back({PDG_KERNEL_RESIDENT, 0, 0});
+        c.push_back({PDG_KERNEL_RESIDENT, 0, 512});
         c.push_back({PDG_KERNEL_RESIDENT, 0, 256});
         c.push_back({PDG_KERNEL_PERSISTENT, 256, 256});
         c.push_back({PDG_KERNEL_PERSISTENT, 512, 512});
@@ -85,7 +86,7 @@ std::vector<Plan> candidates(bool warm)
                    Plan{PDG_KERNEL_GRAPH, 256, 256}, Plan{PDG_KERNEL_GRAPH, 256, 512}, Plan{PDG_KERNEL_GRAPH, 512, 512},
                    Plan{PDG_KERNEL_GRAPH, 1024, 512}, Plan{PDG_KERNEL_STREAM, 112, 128},
                    Plan{PDG_KERNEL_STREAM, 128, 128}, Plan{PDG_KERNEL_STREAM, 160, 128},
-                   Plan{PDG_KERNEL_STREAM, 256, 256}})
+                   Plan{PDG_KERNEL_STREAM, 192, 256}, Plan{PDG_KERNEL_STREAM, 256, 256}})
         c.push_back(p);
     return c;
 }
