@@ -304,28 +304,29 @@ int stream_patch_verts(const std::vector<ClothSetup>& cl, int nsm)
 }
 
 // Patch size of the resident plan on 256-thread blocks (224 compute threads)
-// when the caller leaves the plan open, 0: the 512-thread blocks.  Patches of
-// at most 64 vertices, one per SM, take less time in the smaller blocks, whose
-// barriers wait for fewer warps (per 50 sweeps: 33x33 106.5 against 109.8 us,
-// 65x65 106.7 against 109.0, 97x97 109.6 against 113.0).  Beyond that two
-// patches per SM, which overlap one another's waits, where their records take
-// no more rounds of the threads than one patch's of twice the size take of
-// 480: one up to 160 vertices (129x129 123 against 129.5 us, 181x181 142
-// against 150, 200x230 157 against 172), two above 192 (245x245 189 against
-// 205, 257x257 in 218 vertices 194 against 201); between them not (225x225 182
-// against 175, 235x235 187 against 184.5), nor above 220 (257x257 in 224
-// vertices 217).  With a tolerance the 512-thread blocks stay (129x129, 201
-// sweeps: 518 against 532 us).
+// when the caller leaves the plan open, 0: the 512-thread blocks.  The smaller
+// blocks' barriers wait for fewer warps, so they take one patch per SM as long
+// as two do not overlap one another's waits to more effect: up to 96 vertices
+// with fixed sweep counts, up to 160 with a tolerance, whose spare warps share
+// the SM (per 100 sweeps, one of 256 threads / two / one of 512: 105x105 204 /
+// 219 / 230 us, 129x129 231 / 228 / 241; to a tolerance 129x129 243 / 264 /
+// 254, 145x145 248 / 263 / 263).  Then two patches per SM where their records
+// take no more rounds of the threads than those of one patch of twice the size
+// take of 480: one up to 160 vertices (per 50 sweeps 181x181 142 against 150
+// us, 200x230 157 against 172; to a tolerance 200x230 310 against 338 per 100),
+// two above 192 (245x245 189 against 205, 257x257 in 218 vertices 194 against
+// 201; 384 against 392); between them not (225x225 182 against 175, 235x235
+// 187 against 184.5), nor above 220 (257x257 in 224 vertices 217).
 int resident_small_patch(const std::vector<ClothSetup>& cl, int nsm)
 {
-    for (const auto& c : cl)
-        if (c.cfg.tolerance > 0.f) return 0;
+    bool tol = false;
+    for (const auto& c : cl) tol = tol || c.cfg.tolerance > 0.f;
     auto size_for = [&](long long blocks, int most, int step) {
         for (int pv = 24; pv <= most; pv += step)
             if (patch_count(cl, pv) <= blocks) return pv;
         return 0;
     };
-    if (const int one = size_for(nsm, 64, 8)) return one;
+    if (const int one = size_for(nsm, tol ? 160 : 96, 8)) return one;
     const int two = size_for(2LL * nsm, 220, 1);
     return two <= 160 || two > 192 ? two : 0;
 }
