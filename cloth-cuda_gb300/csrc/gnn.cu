@@ -468,9 +468,16 @@ int pdg_warmstart_attach(pdg_warmstart* w, pdg_solver* s)
     }
     std::vector<int> ptr(N + 1, 0), adj;
     std::vector<float> rest;
+    // a node's neighbours in the order of the usual plan, whatever plan the
+    // solver has: the messages are summed in that order
+    const std::vector<int>* order = nullptr;
+    if (const int rc = usual_order(s, &order)) return rc;
+    std::vector<int> pos(N), rank(N);
+    for (int g = 0; g < N; ++g) pos[(*order)[g]] = g;
+    for (int g = 0; g < N; ++g) rank[g] = pos[Lh.perm_global[g]];
     for (int i = 0; i < N; ++i) {
-        std::sort(nbr[i].begin(), nbr[i].end(), [](const std::pair<int, float>& a, const std::pair<int, float>& b) {
-            return a.first < b.first;
+        std::sort(nbr[i].begin(), nbr[i].end(), [&](const std::pair<int, float>& a, const std::pair<int, float>& b) {
+            return rank[a.first] < rank[b.first];
         });
         for (auto& q : nbr[i]) { adj.push_back(q.first); rest.push_back(q.second); }
         ptr[i + 1] = (int)adj.size();

@@ -108,9 +108,9 @@ bool resident_moves_state(int mode);
 cudaError_t launch_resident(const PersistArgs& p, int variant, int grid, size_t smem, cudaStream_t s);
 // Sweeps p.k0 .. p.k1 - 1 of a frame of the consistent mode in one cooperative
 // launch, its prediction, start and finalisation in others.  The variant for
-// patches of at most max_nown vertices that are all resident at once with
+// patches of at most max_nown vertices and max_rec records that are all resident at once with
 // `smem` bytes each (-1: none).
-int resident_range_pick(int max_nown, int npatch, size_t smem);
+int resident_range_pick(int max_nown, int max_rec, int npatch, size_t smem);
 cudaError_t launch_resident_range(const PersistArgs& p, int variant, int grid, size_t smem, cudaStream_t s);
 
 // Streaming per-sweep kernel (pd_stream.cu): persistent grid, the vertex

@@ -303,6 +303,27 @@ int stream_patch_verts(const std::vector<ClothSetup>& cl, int nsm)
     return cost(192, 4.85) < cost(256, 6.1) ? 192 : 256;
 }
 
+// Smallest patch size (first, first + step, ... most) with at most `blocks`
+// patches, 0: none.
+int size_for(const std::vector<ClothSetup>& cl, long long blocks, int first, int most, int step)
+{
+    for (int pv = first; pv <= most; pv += step)
+        if (patch_count(cl, pv) <= blocks) return pv;
+    return 0;
+}
+
+// Patch size of a streaming plan left open whose sweeps then run as one launch
+// of the resident kernel, 0: none does.  One patch per SM up to 160 vertices,
+// then two.  Batches, 50 sweeps to a tolerance: 5,289 vertices 160 -> 130 us
+// against 256-vertex patches in 512-thread blocks, 20,031 169 -> 144, 32,001
+// 168 -> 161; 38,982 (256 vertices: a launch per sweep) 352 -> 167, 59,886 419
+// -> 205.
+int range_patch_verts(const std::vector<ClothSetup>& cl, int nsm)
+{
+    const int one = size_for(cl, nsm, 24, 160, 8);
+    return one ? one : size_for(cl, 2LL * nsm, 24, 220, 1);
+}
+
 // Patch size of the resident plan on 256-thread blocks (224 compute threads)
 // when the caller leaves the plan open, 0: the 512-thread blocks.  The smaller
 // blocks' barriers wait for fewer warps, so they take one patch per SM as long
@@ -321,13 +342,8 @@ int resident_small_patch(const std::vector<ClothSetup>& cl, int nsm)
 {
     bool tol = false;
     for (const auto& c : cl) tol = tol || c.cfg.tolerance > 0.f;
-    auto size_for = [&](long long blocks, int most, int step) {
-        for (int pv = 24; pv <= most; pv += step)
-            if (patch_count(cl, pv) <= blocks) return pv;
-        return 0;
-    };
-    if (const int one = size_for(nsm, tol ? 160 : 96, 8)) return one;
-    const int two = size_for(2LL * nsm, 220, 1);
+    if (const int one = size_for(cl, nsm, 24, tol ? 160 : 96, 8)) return one;
+    const int two = size_for(cl, 2LL * nsm, 24, 220, 1);
     return two <= 160 || two > 192 ? two : 0;
 }
 
@@ -453,6 +469,7 @@ int pdg::create_solver(int n, const pdg_config* cfgs, const pdg_mesh* const* mes
     CK(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     std::string err;
+    bool built = false;   // the layout of a per-sweep plan
     if ((c0.kernel == PDG_KERNEL_AUTO && !s->any_warm) || c0.kernel == PDG_KERNEL_RESIDENT) {
         // Resident kernel: every patch co-resident, one 512-thread block per
         // SM, or (block_threads = 256) two half-size patches per SM; a block
@@ -497,13 +514,19 @@ int pdg::create_solver(int n, const pdg_config* cfgs, const pdg_mesh* const* mes
                              (int)patch_count(s->cloths, P), P);
         }
     }
-    // (a learned start sums its messages in layout order: its plan stays)
-    if (s->kernel == PDG_KERNEL_STREAM && !c0.patch_verts && !c0.block_threads && !s->any_warm) {
+    if (s->kernel == PDG_KERNEL_STREAM && !c0.patch_verts && !c0.block_threads) {
         const int open = s->patch_verts;
-        s->patch_verts = stream_patch_verts(s->cloths, nsm);
+        s->patch_verts = s->mode == PDG_MODE_CONSISTENT ? range_patch_verts(s->cloths, nsm) : 0;
+        if (s->patch_verts) {
+            const int rc = per_sweep_layout(s.get(), smem_optin, s->patch_verts, s->L, s->sargs, s->stream_smem);
+            if (rc) return rc;
+            if (resident_range_pick(s->L.max_nown, s->L.max_ncell + s->L.max_nhinge, s->L.npatch, s->L.smem_resident) < 0) s->patch_verts = 0;
+        }
+        built = s->patch_verts != 0;
+        if (!built) s->patch_verts = stream_patch_verts(s->cloths, nsm);
         if (s->patch_verts != open) s->open_verts = open;
     }
-    if (s->kernel != PDG_KERNEL_RESIDENT) {
+    if (s->kernel != PDG_KERNEL_RESIDENT && !built) {
         const int rc = per_sweep_layout(s.get(), smem_optin, s->patch_verts, s->L, s->sargs, s->stream_smem);
         if (rc) return rc;
     }
@@ -517,7 +540,7 @@ int pdg::create_solver(int n, const pdg_config* cfgs, const pdg_mesh* const* mes
     // kernel runs the sweeps of a frame in one launch.  A sweep of 54,000
     // vertices in 434 patches of 128 then takes 3.7 us instead of 7.3 us.
     if (s->kernel == PDG_KERNEL_STREAM && s->mode == PDG_MODE_CONSISTENT)
-        s->range_variant = resident_range_pick(s->L.max_nown, s->L.npatch, s->L.smem_resident);
+        s->range_variant = resident_range_pick(s->L.max_nown, s->L.max_ncell + s->L.max_nhinge, s->L.npatch, s->L.smem_resident);
     int rc = upload_all(s.get());
     if (rc) return rc;
     s->h_rt.resize(s->L.ncloth);

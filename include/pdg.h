@@ -68,10 +68,10 @@ extern "C" {
                                     the current one.  Where every patch is
                                     resident at once, the sweeps of a frame
                                     run in one cooperative launch instead.
-                                    patch_verts and block_threads 0: 192 or
-                                    256 vertices, whichever fills the last
-                                    wave of blocks better (256 with a learned
-                                    start), on 256 threads                   */
+                                    patch_verts and block_threads 0: patches
+                                    small enough for that where two per SM
+                                    are, else 192 or 256 vertices, whichever
+                                    fills the last wave of blocks better     */
 
 /* Solver configuration.  Mirrors PDSolverConfig (include/pd_solver.h:4-15);
  * fields after `damping` extend it. */

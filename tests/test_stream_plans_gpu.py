@@ -38,6 +38,39 @@ def test_stream_instances_match_graph(pdg, rows, cols, mtype, pv, nt, tol):
         assert abs(a["res_final"] - b["res_final"]) <= 1e-5 * abs(a["res_final"])
 
 
+# all patches resident: 379 of 128 vertices (two rounds of 128 threads), and the
+# open plan with one patch per SM (152 vertices), two (160) and two of 198
+@pytest.mark.parametrize("rows,cols,pv,nt", [(220, 220, 128, 128), (150, 150, 0, 0), (220, 220, 0, 0), (240, 250, 0, 0)])
+@pytest.mark.parametrize("tol", [0.0, 0.7])
+def test_resident_stream_plans_match_graph(pdg, rows, cols, pv, nt, tol):
+    r = solve(pdg, pdg.KERNEL_STREAM, rows, cols, 1, pv, nt, tol)
+    assert r[2] == 2 * 5   # the sweeps in one launch
+    g = solve(pdg, pdg.KERNEL_GRAPH, rows, cols, 1, 128, 128, tol)
+    assert [f["iterations"] for f in g[1]] == [f["iterations"] for f in r[1]]
+    assert np.array_equal(g[0][0], r[0][0]) and np.array_equal(g[0][1], r[0][1])
+
+
+# the network's messages are summed in one order whatever the plan: a random
+# network, its start always kept, on the open plan and on the 256-vertex one
+def test_network_start_does_not_depend_on_the_plan(pdg):
+    import scenes
+    out = []
+    for plan in ({}, dict(patch_verts=256, block_threads=256)):
+        ms, cs, cfg, _ = scenes.batch(5, seed=11, n_range=(17, 49), max_iterations=6, tolerance=0.0,
+                                      kernel=pdg.KERNEL_STREAM, init=pdg.INIT_WARMSTART_KEEP, **plan)
+        s = pdg.Solver(cfg, ms, cs)
+        w = pdg.WarmStart(seed=4)
+        p = w.get_params()
+        w.set_params((p + np.random.default_rng(3).normal(0.0, 0.02, p.shape)).astype(np.float32))
+        w.attach(s)
+        s.step(2)
+        out.append((s.launch_info()["patch_verts"], [s.get_state(i)[0] for i in range(len(ms))]))
+        s.close(); w.close()
+    assert out[0][0] != 256
+    for a, b in zip(out[0][1], out[1][1]):
+        assert np.array_equal(a, b)
+
+
 # 333x500: 192 vertices fill the last wave of blocks better on 152 SMs; 512x513:
 # 1,026 patches of 256 (2.25 waves) or 1,368 of 192 (three)
 @pytest.mark.parametrize("rows,cols", [(333, 500), (512, 513)])
