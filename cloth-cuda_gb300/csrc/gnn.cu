@@ -470,10 +470,9 @@ int pdg_warmstart_attach(pdg_warmstart* w, pdg_solver* s)
     std::vector<float> rest;
     // a node's neighbours in the order of the usual plan, whatever plan the
     // solver has: the messages are summed in that order
-    const std::vector<int>* order = nullptr;
-    if (const int rc = usual_order(s, &order)) return rc;
+    const std::vector<int>& order = usual_order(s);
     std::vector<int> pos(N), rank(N);
-    for (int g = 0; g < N; ++g) pos[(*order)[g]] = g;
+    for (int g = 0; g < N; ++g) pos[order[g]] = g;
     for (int g = 0; g < N; ++g) rank[g] = pos[Lh.perm_global[g]];
     for (int i = 0; i < N; ++i) {
         std::sort(nbr[i].begin(), nbr[i].end(), [&](const std::pair<int, float>& a, const std::pair<int, float>& b) {
@@ -569,9 +568,7 @@ int pdg_warmstart_train_pair(pdg_warmstart* w, pdg_solver* traj, pdg_solver* dee
     const bool same = deep->L.perm_global == traj->L.perm_global;
     int rc = PDG_OK;
     if (!same) {
-        const std::vector<int>*a = nullptr, *b = nullptr;
-        if ((rc = usual_order(traj, &a)) || (rc = usual_order(deep, &b))) return rc;
-        if (*a != *b)
+        if (usual_order(traj) != usual_order(deep))
             return set_error(PDG_ERR_ARG, "pdg_warmstart_train_pair: `deep` must solve the same cloths with the same "
                                           "vertex layout (same patch plan, per-sweep kernels)");
     }

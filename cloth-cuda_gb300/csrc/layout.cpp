@@ -314,7 +314,57 @@ void build_cells(const MeshData& m, const Topology& tp, const ConstraintData& cd
     }
 }
 
+// Order of a cloth's vertices (perm: position -> vertex, iperm its inverse):
+// patches by bisection, and within each patch the boundary vertices (bnd) first.
+// A vertex is "boundary" when a cell or lone hinge through it has a corner in
+// another patch (it is then in that patch's halo), so a kernel can finish and
+// publish these before the interior.
+void cloth_order(const MeshData& m, const std::vector<CellBuild>& cells, const std::vector<int>& lone,
+                 const ConstraintData& cd, int patch_verts, std::vector<int>& perm, std::vector<int>& iperm,
+                 std::vector<char>& bnd)
+{
+    const int N = m.N;
+    bisection_order(m, patch_verts, perm);
+    iperm.resize(N);
+    for (int i = 0; i < N; ++i) iperm[perm[i]] = i;
+    bnd.assign(N, 0);
+    auto mark = [&](const int* v, int n) {
+        int p = -1;
+        bool span = false;
+        for (int a = 0; a < n; ++a) {
+            if (v[a] < 0) continue;
+            const int q = iperm[v[a]] / patch_verts;
+            span = span || (p >= 0 && q != p);
+            p = q;
+        }
+        if (span)
+            for (int a = 0; a < n; ++a)
+                if (v[a] >= 0) bnd[v[a]] = 1;
+    };
+    for (const CellBuild& c : cells) mark(c.v, 6);
+    for (int e : lone) mark(&cd.quads[4 * e], 4);
+    for (int p0 = 0; p0 < N; p0 += patch_verts)
+        std::stable_partition(perm.begin() + p0, perm.begin() + std::min(N, p0 + patch_verts),
+                              [&](int o) { return bnd[o] != 0; });
+    for (int i = 0; i < N; ++i) iperm[perm[i]] = i;
+}
+
 }  // namespace
+
+void vertex_order(const std::vector<ClothSetup>& cl, int patch_verts, std::vector<int>& perm_global)
+{
+    perm_global.clear();
+    int vbase = 0;
+    for (const ClothSetup& c : cl) {
+        std::vector<CellBuild> cells;
+        std::vector<int> lone, perm, iperm;
+        std::vector<char> bnd;
+        build_cells(*c.mesh, *c.topo, c.cons, c.cfg.dt * c.cfg.dt, cells, lone);
+        cloth_order(*c.mesh, cells, lone, c.cons, patch_verts, perm, iperm, bnd);
+        for (int o : perm) perm_global.push_back(vbase + o);
+        vbase += c.mesh->N;
+    }
+}
 
 bool build_layout(const std::vector<ClothSetup>& cl, int patch_verts, HostLayout& L, std::string& err)
 {
@@ -342,40 +392,14 @@ bool build_layout(const std::vector<ClothSetup>& cl, int patch_verts, HostLayout
         const ConstraintData& cd = cl[ci].cons;
         const pdg_config& cfg = cl[ci].cfg;
         const int N = m.N;
-        std::vector<int> perm, iperm(N);
-        bisection_order(m, patch_verts, perm);
-        for (int i = 0; i < N; ++i) iperm[perm[i]] = i;
+        std::vector<int> perm, iperm;
+        std::vector<char> bnd;
         const float h2 = cfg.dt * cfg.dt;
         std::vector<CellBuild> cells;
         std::vector<int> lone;
         build_cells(m, tp, cd, h2, cells, lone);
         const int C = (int)cells.size(), H = (int)lone.size();
-        // A vertex is "boundary" when a cell or lone hinge through it has a
-        // corner in another patch (it is then in that patch's halo).  Within
-        // each patch the boundary vertices go first, so a kernel can finish
-        // and publish them before the interior.
-        std::vector<char> bnd(N, 0);
-        {
-            auto mark = [&](const int* v, int n) {
-                int p = -1;
-                bool span = false;
-                for (int a = 0; a < n; ++a) {
-                    if (v[a] < 0) continue;
-                    const int q = iperm[v[a]] / patch_verts;
-                    span = span || (p >= 0 && q != p);
-                    p = q;
-                }
-                if (span)
-                    for (int a = 0; a < n; ++a)
-                        if (v[a] >= 0) bnd[v[a]] = 1;
-            };
-            for (int c = 0; c < C; ++c) mark(cells[c].v, 6);
-            for (int e : lone) mark(&cd.quads[4 * e], 4);
-            for (int p0 = 0; p0 < N; p0 += patch_verts)
-                std::stable_partition(perm.begin() + p0, perm.begin() + std::min(N, p0 + patch_verts),
-                                      [&](int o) { return bnd[o] != 0; });
-            for (int i = 0; i < N; ++i) iperm[perm[i]] = i;
-        }
+        cloth_order(m, cells, lone, cd, patch_verts, perm, iperm, bnd);
 
         std::vector<float> diag;
         jacobi_diag(m, cd, cfg.dt, diag);

@@ -45,6 +45,8 @@ struct HostLayout {
     std::vector<int> nbr_ptr, nbr;  // patches owning each patch's halo vertices
 };
 
+// layout.cpp: perm_global of build_layout alone
+void vertex_order(const std::vector<ClothSetup>& cl, int patch_verts, std::vector<int>& perm_global);
 bool build_layout(const std::vector<ClothSetup>& cl, int patch_verts, HostLayout& L, std::string& err);
 // The properties the sweep kernels rely on (partition, halo, neighbour lists,
 // boundary-first order, each contribution slot written once, every incident
@@ -161,5 +163,5 @@ int warm_kernel_count();
 int warm_judge_sweeps(const pdg_warmstart* w);
 void warm_detach(pdg_warmstart* w, const pdg_solver* s);
 // solver.cpp: vertex order of the solver's cloths in patches of the usual size
-int usual_order(pdg_solver* s, const std::vector<int>** order);
+const std::vector<int>& usual_order(pdg_solver* s);
 }  // namespace pdg

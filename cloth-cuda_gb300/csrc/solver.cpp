@@ -386,23 +386,11 @@ namespace pdg {
 // The vertex order that the solver's cloths have in patches of the usual size,
 // whatever size its own plan has: what two solvers over the same cloths have
 // in common where the plan chose the size.
-int usual_order(pdg_solver* s, const std::vector<int>** order)
+const std::vector<int>& usual_order(pdg_solver* s)
 {
-    *order = &s->L.perm_global;
-    if (!s->open_verts) return PDG_OK;
-    if (s->usual.empty()) {
-        int dev = 0, smem_optin = 0, pv = s->open_verts;
-        CK(cudaGetDevice(&dev));
-        CK(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-        HostLayout L;
-        StreamArgs sa;
-        size_t smem = 0;
-        const int rc = per_sweep_layout(s, smem_optin, pv, L, sa, smem);
-        if (rc) return rc;
-        s->usual = L.perm_global;
-    }
-    *order = &s->usual;
-    return PDG_OK;
+    if (!s->open_verts) return s->L.perm_global;
+    if (s->usual.empty()) vertex_order(s->cloths, s->open_verts, s->usual);
+    return s->usual;
 }
 
 }  // namespace pdg
@@ -491,14 +479,18 @@ int pdg::create_solver(int n, const pdg_config* cfgs, const pdg_mesh* const* mes
                    L.smem_resident <= (size_t)std::min(smem_optin / per - 8192, 216 * 1024) &&
                    L.npatch <= resident_max_blocks(s->mode, variant, L.smem_resident);
         };
-        bool ok = fits(P, rnt, s->L);
-        const int small = ok && !c0.patch_verts && !c0.block_threads && s->mode == PDG_MODE_CONSISTENT
-                              ? resident_small_patch(s->cloths, nsm) : 0;
-        if (small) {
-            HostLayout L;
-            if (fits(small, 224, L)) { s->L = std::move(L); P = small; rnt = 224; }
-            else variant = resident_pick(rnt);
-        }
+        // The open plan's smaller blocks, where the 512-thread blocks would do
+        // as well: their shared memory is less than in proportion to the small
+        // patches', so their layout is built only where that is too much.
+        const int small = !c0.patch_verts && !c0.block_threads && s->mode == PDG_MODE_CONSISTENT &&
+                                  patch_count(s->cloths, P) <= nsm ? resident_small_patch(s->cloths, nsm) : 0;
+        HostLayout Ls;
+        bool ok = small && fits(small, 224, Ls);
+        const int vs = variant;
+        const bool sure = ok && Ls.smem_resident * (double)P <= 200.0 * 1024 * small;
+        const bool large = !sure && fits(P, rnt, s->L);
+        if (ok && (sure || large)) { s->L = std::move(Ls); P = small; rnt = 224; variant = vs; }
+        else ok = large;
         if (ok) {
             s->kernel = PDG_KERNEL_RESIDENT;
             s->patch_verts = P;
