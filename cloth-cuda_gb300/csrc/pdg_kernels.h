@@ -77,8 +77,9 @@ struct PersistArgs {
     unsigned long long* xch;
     unsigned* xch_tag;
     int nbr_sync;        // 1: no cloth has a tolerance
-    // resident kernel, with a tolerance: per cloth and sweep (acc_stride
-    // entries each) the patches that have added their part of the residual
+    // resident kernel: per cloth and sweep (acc_stride entries each) the
+    // patches that have added their part of the residual (tolerances); two
+    // sets, cleared by every frame
     int* cnt;
     unsigned* frame;     // resident kernel: parity of the frame's set of sums (it.acc and cnt hold two)
     int k0, k1;          // launch_resident_range: sweeps k0 .. k1 - 1
