@@ -743,6 +743,13 @@ static int take_wait_error(pdg_solver* s)
     CK(cudaMemsetAsync(s->bar.p, 0, 4 * sizeof(unsigned), s->stream));
     CK(cudaMemsetAsync(s->acc.p, 0, sizeof(double) * s->acc.n, s->stream));
     if (s->res_cnt.p) CK(cudaMemsetAsync(s->res_cnt.p, 0, sizeof(int) * s->res_cnt.n, s->stream));
+    // and offsets published under tags that the next frame would use again (a
+    // frame moves the tag word on when its sweeps are done): the exchange
+    // starts afresh, as at creation
+    if (s->xch.p) {
+        CK(cudaMemsetAsync(s->xch.p, 0, sizeof(unsigned long long) * s->xch.n, s->stream));
+        CK(cudaMemsetAsync(s->xch_tag.p, 0, sizeof(unsigned), s->stream));
+    }
     CK(cudaStreamSynchronize(s->stream));
     return set_error(PDG_ERR_TIMEOUT, "bounded wait ran out (%s)",
                      e == 1 ? "grid barrier" : e == 2 ? "resident grid barrier" : "neighbour exchange");
