@@ -76,7 +76,7 @@ struct PersistArgs {
     // which every frame advances by its sweep count (null: no exchange)
     unsigned long long* xch;
     unsigned* xch_tag;
-    int nbr_sync;        // 1: no cloth has a tolerance
+    int nbr_sync;        // 1: fixed sweep counts (no cloth has a tolerance that its mode looks at)
     // resident kernel: per cloth and sweep (acc_stride entries each) the
     // patches that have added their part of the residual (tolerances); two
     // sets, cleared by every frame

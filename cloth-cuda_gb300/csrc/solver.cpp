@@ -276,6 +276,16 @@ int launches_per_frame(const pdg_solver* s)
     return 4 + (s->range_variant >= 0 ? 1 : s->L.cap + (s->have_final ? 1 : 0));
 }
 
+// Whether no cloth's sweeps end by a decision: none has a tolerance, or the
+// mode (reference-literal) does not look at it.
+int fixed_counts(const pdg_solver* s)
+{
+    if (s->mode == PDG_MODE_CONSISTENT)
+        for (const auto& c : s->cloths)
+            if (c.cfg.tolerance > 0.f) return 0;
+    return 1;
+}
+
 // Patches of at most pv vertices over these cloths.
 long long patch_count(const std::vector<ClothSetup>& cl, int pv)
 {
@@ -497,10 +507,7 @@ int pdg::create_solver(int n, const pdg_config* cfgs, const pdg_mesh* const* mes
             s->nt = rnt + 32;
             s->res_variant = variant;
             s->persist_grid = s->L.npatch;
-            // fixed sweep counts need no decisions
-            s->nbr_sync = 1;
-            for (const auto& c : s->cloths)
-                if (c.cfg.tolerance > 0.f) s->nbr_sync = 0;
+            s->nbr_sync = fixed_counts(s.get());
         } else if (c0.kernel == PDG_KERNEL_RESIDENT) {
             return set_error(PDG_ERR_ARG, "resident kernel does not fit this problem (%d patches of %d vertices)",
                              (int)patch_count(s->cloths, P), P);
@@ -1007,11 +1014,7 @@ int pdg_solver_set_tolerance(pdg_solver* s, int cloth, float tolerance)
                        s->stream));
     CK(cudaStreamSynchronize(s->stream));
     // the launch plan's choices that depend on the tolerance (as at creation)
-    if (s->kernel == PDG_KERNEL_RESIDENT) {
-        s->nbr_sync = 1;
-        for (const auto& c : s->cloths)
-            if (c.cfg.tolerance > 0.f) s->nbr_sync = 0;
-    }
+    if (s->kernel == PDG_KERNEL_RESIDENT) s->nbr_sync = fixed_counts(s);
     const pdg_config& f = s->cloths[0].cfg;
     const int hf = (s->mode == PDG_MODE_CONSISTENT) && (f.compute_final_residual || f.tolerance > 0.f);
     if (hf != s->have_final) {
