@@ -41,6 +41,7 @@
 #include <mutex>
 
 #include "../../include/pdg.h"
+#include "noalloc_wait.h"
 #include "pd_kernels.cuh"
 #include "pdg_host.h"
 
@@ -53,8 +54,7 @@ constexpr int kMaxIters = PDG_NOALLOC_MAX_ITERS;
 struct NaCtl {
     int active, used, status, pad;
     double res_y2, res0_2, resf_2;
-    unsigned bar;      // grid barrier: arrivals so far (cleared before each frame)
-    int err;           // a barrier wait gave up (cleared with them)
+    unsigned bar;      // grid barrier: arrivals so far, kNaGaveUp (cleared before each frame)
 };
 
 constexpr size_t kOffY = 0;
@@ -101,6 +101,25 @@ struct NaArgs {
     int cap, have_final, use_cheb, cheb_delay;
 };
 
+// The frame's barrier word (noalloc_wait.h) on the device.
+struct NaBarWord {
+    unsigned* p;
+    long long t0;
+    __device__ __forceinline__ void arrive()
+    {
+        asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "r"(1u) : "memory");
+    }
+    __device__ __forceinline__ unsigned look()
+    {
+        unsigned v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(__cvta_generic_to_global(p)) : "memory");
+        return v;
+    }
+    __device__ __forceinline__ void start() { t0 = clock64(); }
+    __device__ __forceinline__ bool late() { return clock64() - t0 > kNaWaitCycles; }
+    __device__ __forceinline__ void replace(unsigned v, unsigned to) { atomicCAS(p, v, to); }
+};
+
 // Barrier `phase` (1, 2, ...) of the frame over the grid: one arrival per
 // block on a count that only grows, polled until all blocks of the phase are
 // in.  False once a wait, here or in another block, gave up.  na_wait is the
@@ -109,18 +128,8 @@ struct NaArgs {
 // 129x129 cloth took 156 us instead of 150).
 __device__ __forceinline__ bool na_wait(NaCtl* c, unsigned phase)
 {
-    const unsigned want = phase * gridDim.x;
-    unsigned v;
-    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(__cvta_generic_to_global(&c->bar)), "r"(1u) : "memory");
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(__cvta_generic_to_global(&c->bar)) : "memory");
-    if (v < want) {
-        const long long t0 = clock64();
-        do {
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(__cvta_generic_to_global(&c->bar)) : "memory");
-            if (clock64() - t0 > kNaWaitCycles) { atomicCAS(&c->err, 0, 1); break; }
-        } while (v < want);
-    }
-    return v >= want;
+    NaBarWord w{&c->bar, 0};
+    return na_wait_on(w, phase * gridDim.x);
 }
 __device__ __forceinline__ bool na_barrier(NaCtl* c, unsigned& phase)
 {
@@ -622,7 +631,8 @@ extern "C" int pdg_step_noalloc(const pdg_config* cfg, int N, float* d_pos, floa
         NaCtl c;
         NA_CK(cudaMemcpyAsync(&c, a.s.ctl, sizeof(NaCtl), cudaMemcpyDeviceToHost, st));
         NA_CK(cudaStreamSynchronize(st));
-        if (c.err) return set_error(PDG_ERR_TIMEOUT, "pdg_step_noalloc: bounded wait ran out (grid barrier)");
+        if (c.bar & kNaGaveUp)
+            return set_error(PDG_ERR_TIMEOUT, "pdg_step_noalloc: bounded wait ran out (grid barrier)");
         stats->iterations = c.used;
         stats->warm_start_used = 0;
         stats->status = c.status;

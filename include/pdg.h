@@ -431,8 +431,8 @@ void pdg_warmstart_destroy(pdg_warmstart* w);
  * it is reported only through stats->status (PDG_ERR_NUMERIC): the call
  * itself returns PDG_OK, since without stats it does not wait for the GPU.
  * The frame is one cooperative launch whose grid barriers are bounded (about
- * 2 s); a wait that runs out is reported as PDG_ERR_TIMEOUT when stats are
- * asked for, and x and v are then undefined. */
+ * 2 s).  When a wait runs out the frame is given up as a whole: x and v stay
+ * as they were, and PDG_ERR_TIMEOUT is reported when stats are asked for. */
 #define PDG_NOALLOC_MAX_VERTS 131072
 #define PDG_NOALLOC_MAX_ITERS 4096
 int  pdg_step_noalloc(const pdg_config* cfg, int N, float* d_pos, float* d_vel, const float* d_mass,
