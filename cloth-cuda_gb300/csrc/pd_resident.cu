@@ -327,9 +327,9 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
     // The per-sweep sums and arrivals of a whole frame come in two sets: a
     // frame uses the one that p.frame's parity names and clears the other, so
     // that no block needs to wait for the clearing.  Frames with fixed sweep
-    // counts have no arrivals but clear them too: the frame that uses the set
-    // next may have a tolerance.  (A range uses the sums that the frame's
-    // first launch cleared.)
+    // counts have no arrivals but clear them too (in the spare warp, below):
+    // the frame that uses the set next may have a tolerance.  (A range uses
+    // the sums that the frame's first launch cleared.)
     const unsigned par = RANGE ? 0u : __ldcg(p.frame) & 1u;
     const size_t set = (size_t)a.ncloth * a.acc_stride;
     double* acc = a.acc + (RANGE ? 0 : par * set) + (size_t)c * a.acc_stride;
@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
         }
         for (int k = tid; k < a.acc_stride; k += NTT) {
             if (!RANGE) a.acc[(par ^ 1u) * set + (size_t)c * a.acc_stride + k] = 0.0;
-            p.cnt[(RANGE ? 0u : par ^ 1u) * set + (size_t)c * a.acc_stride + k] = 0;
+            if (TOL) p.cnt[(RANGE ? 0u : par ^ 1u) * set + (size_t)c * a.acc_stride + k] = 0;
         }
     }
     if (TOL && tid == 0) { gone = 0; stopped = 0; }
@@ -616,6 +616,8 @@ __global__ void __launch_bounds__(NT + 32, 512 / (NT + 32)) k_resident(PersistAr
         const int kq = max_iter() + (a.have_final ? 1 : 0);
         if (RANGE && first && lane == 0 && !ended && kend > k0 && kq < nsweep && complete(kend - 1))
             cloth_done(a, c, kq, true, true);
+    } else if (first) {
+        for (int k = tid - NT; k < a.acc_stride; k += 32) p.cnt[(par ^ 1u) * set + (size_t)c * a.acc_stride + k] = 0;
     }
     if (RANGE) return;
     // every per-sweep sum is complete after this barrier, and every block has
