@@ -247,12 +247,29 @@ int upload_graph(pdg_warmstart* w, int N, const int* ptr, int E, const int* adj,
 }
 
 // Waits for upload_graph's checks; nothing may read the graph before.
-int graph_ok(pdg_warmstart* w, cudaStream_t st)
+// backward_lists: some list ends before it begins (caller graphs; with one of
+// those an entry may belong to several lists, or the graph may also be bad).
+int graph_ok(pdg_warmstart* w, cudaStream_t st, bool* backward_lists = nullptr)
 {
     int bad = 0;
     GK(cudaMemcpyAsync(&bad, w->bad.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     GK(cudaStreamSynchronize(st));
-    return bad ? set_error(PDG_ERR_ARG, "warm start: adjacency is not symmetric") : PDG_OK;
+    if (backward_lists) *backward_lists = bad == 2;
+    return bad && !(backward_lists && bad == 2) ? set_error(PDG_ERR_ARG, "warm start: adjacency is not symmetric") : PDG_OK;
+}
+
+// The same graph with every list of its own, one after another: ptr, and of
+// each entry its place in the caller's arrays.  False where a list leaves them.
+bool plain_lists(int N, const int* ptr, int E, std::vector<int>& p, std::vector<int>& from)
+{
+    p.assign(1, 0);
+    for (int i = 0; i < N; ++i) {
+        if (ptr[i] < 0 || ptr[i] > E || ptr[i + 1] < 0 || ptr[i + 1] > E) return false;
+        for (int e = ptr[i]; e < ptr[i + 1]; ++e) from.push_back(e);
+        if (from.size() > 0x7fffffffu) return false;
+        p.push_back((int)from.size());
+    }
+    return true;
 }
 
 }  // namespace
@@ -387,8 +404,27 @@ int pdg_warmstart_eval(pdg_warmstart* w, int N, const float* x, const int* ptr, 
     GK(cudaMemcpyAsync(w->target.p, target, sizeof(float) * 3 * N, cudaMemcpyHostToDevice, st));
     GK(cudaMemcpyAsync(w->freew.p, freew, sizeof(float) * N, cudaMemcpyHostToDevice, st));
     if (ew && E) GK(cudaMemcpyAsync(w->ew.p, ew, sizeof(float) * E, cudaMemcpyHostToDevice, st));
-    rc = graph_ok(w, st);
+    bool backward_lists = false;
+    rc = graph_ok(w, st, &backward_lists);
     if (rc) return rc;
+    if (backward_lists) {   // the kernels keep one sign mask per entry: no entry may belong to two lists
+        try {
+            std::vector<int> p, from;
+            if (!plain_lists(N, ptr, E, p, from)) return set_error(PDG_ERR_ARG, "pdg_warmstart_eval: bad adjacency");
+            std::vector<int> a(from.size());
+            std::vector<float4> f(from.size());
+            std::vector<float> q(ew ? from.size() : 0);
+            for (size_t i = 0; i < from.size(); ++i) {
+                a[i] = adj[from[i]];
+                std::memcpy(&f[i], ef + 4 * (size_t)from[i], sizeof(float4));
+                if (ew) q[i] = ew[from[i]];
+            }
+            return pdg_warmstart_eval(w, N, x, p.data(), a.data(), f.empty() ? nullptr : &f[0].x, target, freew,
+                                      q.empty() ? nullptr : q.data(), out, loss, grads);
+        } catch (const std::bad_alloc&) {
+            return set_error(PDG_ERR_ALLOC, "host allocation failed");
+        }
+    }
     double cnt = 0.0;
     for (int i = 0; i < N; ++i) cnt += freew[i] > 0.f ? 3.0 : 0.0;
     rc = forward(w, st);

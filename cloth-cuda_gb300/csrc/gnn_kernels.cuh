@@ -1014,24 +1014,26 @@ __global__ void k_adam(int n, float* __restrict__ p, const float* g, float* __re
 
 // ---- caller graphs ---------------------------------------------------------
 // Per node its inverse degree, per directed edge (i <- adj[e]) the index of its
-// reverse.  *bad is set where the lists leave the arrays or an edge has no
-// reverse; the rest of the node's entries are then left unset.
+// reverse.  *bad becomes 1 where the lists leave the arrays or an edge has no
+// reverse (the rest of the node's entries are then left unset), 2 where a list
+// ends before it begins: it is empty, but lists may share entries then.
 __global__ void k_graph(int N, int E, const int* __restrict__ ptr, const int* __restrict__ adj, int* __restrict__ rev,
                         float* __restrict__ deg_inv, int* __restrict__ bad)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
     const int e0 = ptr[i], e1 = ptr[i + 1];
-    if (e0 < 0 || e1 < e0 || e1 > E) { *bad = 1; return; }
+    if (e0 < 0 || e0 > E || e1 < 0 || e1 > E) { *bad = 1; return; }
+    if (e1 < e0) *bad = 2;
     deg_inv[i] = e1 > e0 ? __fdiv_rn(1.f, (float)(e1 - e0)) : 0.f;
     for (int e = e0; e < e1; ++e) {
         const int j = adj[e];
         if (j < 0 || j >= N) { *bad = 1; return; }
         const int f0 = ptr[j], f1 = ptr[j + 1];
-        if (f0 < 0 || f1 < f0 || f1 > E) { *bad = 1; return; }
+        if (f0 < 0 || f0 > E || f1 < 0 || f1 > E) { *bad = 1; return; }
         int f = f0;
         while (f < f1 && adj[f] != i) ++f;
-        if (f == f1) { *bad = 1; return; }
+        if (f >= f1) { *bad = 1; return; }
         rev[e] = f;
     }
 }
