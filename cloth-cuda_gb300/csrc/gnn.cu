@@ -26,7 +26,7 @@ struct pdg_warmstart {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     DevBuf<float> p, g, m, v, bdp;
-    DevBuf<float> part;   // per-block partial weight gradients (summed in a fixed order)
+    DevBuf<float> part;   // per-block partial weight gradients (summed in a fixed order), from the first backward pass on
     DevBuf<bf16> wbuf;
     Bf16Weights W{};
     // graph and activations
@@ -71,9 +71,6 @@ int alloc_params(pdg_warmstart* w)
 {
     const int n = w->lay.total;
     GK(w->p.alloc(n)); GK(w->g.alloc(n)); GK(w->m.alloc(n)); GK(w->v.alloc(n)); GK(w->bdp.alloc(16));
-    // the partial sums of every gradient (they are added up in one launch)
-    GK(w->part.alloc((size_t)kWgradBlocks * ((NO * H + NO) + (H * NF + H) + L * ((2 * H * H + H) + (2 * H * H + 2 * H))) +
-                     (size_t)kMsgBwdBlocks * L * H * (EF + 1)));
     // bf16 copies: We 64x16, per layer AB 128x64, ABt 64x128, U 64x128, Ut 128x64, Wd 16x64, Wdt 64x16
     const size_t sizes[] = {(size_t)H * NFP, 2u * H * H, 2u * H * H, 2u * H * H, 2u * H * H, 16u * H, (size_t)H * 16};
     size_t total = sizes[0] + L * (sizes[1] + sizes[2] + sizes[3] + sizes[4]) + sizes[5] + sizes[6];
@@ -149,6 +146,15 @@ int forward(pdg_warmstart* w, cudaStream_t st)
 }
 
 int wgrad_grid(int M) { return std::max(1, std::min(kWgradBlocks, nb(M, kWgradRows))); }
+int msg_bwd_grid(int N) { return std::max(1, std::min(kMsgBwdBlocks, nb(N, 16))); }
+
+// Floats of the partial sums of every gradient over N nodes (they are added up
+// in one launch): 40 MB at most, which a network that only infers never needs.
+size_t part_floats(int N)
+{
+    return (size_t)wgrad_grid(N) * ((NO * H + NO) + (H * NF + H) + L * ((2 * H * H + H) + (2 * H * H + 2 * H))) +
+           (size_t)msg_bwd_grid(N) * L * H * (EF + 1);
+}
 
 // The partial sums of a backward pass: wgrad and the message backward append
 // a segment each, `run` adds all of them up.
@@ -192,6 +198,7 @@ int backward(pdg_warmstart* w, float inv_cnt, const float* ew, cudaStream_t st)
     const Layout& y = w->lay;
     const float* p = w->p.p;
     float* g = w->g.p;
+    GK(w->part.reserve(part_floats(N)));   // (grows only with the graph, whose upload waits for earlier passes)
     GradSums gs(w->part.p);
     launch_after(k_loss, nb(N, 256), 256, 0, st, N, w->out.p, w->target.p, w->freew.p, w->ptr.p, w->adj.p, ew, w->smooth,
                                        inv_cnt, w->dout.p, w->loss.p);
@@ -202,7 +209,7 @@ int backward(pdg_warmstart* w, float inv_cnt, const float* ew, cudaStream_t st)
         wgrad<H, 2 * H, true>(gs, dh, H, H, w->uo[l].p, H, w->cat[l].p, 2 * H, 2 * H, N, g + y.U[l], g + y.u[l], st);
         gemm<float, H, 2 * H, EPI_MASKA | EPI_SPLIT>(st, dh, H, N, w->W.Ut[l], nullptr, w->uo[l].p, H, nullptr, 0,
                                                      nullptr, 0, dn, H, w->da.p, H, w->deg_inv.p);
-        const int gm = std::max(1, std::min(kMsgBwdBlocks, nb(N, 16)));
+        const int gm = msg_bwd_grid(N);
         float* part = gs.add(gm, H * EF, H, g + y.C[l], g + y.c[l]);
         launch_after(k_msg_bwd, gm, 256, 0, st, N, w->ptr.p, w->adj.p, w->rev.p, w->ef.p, w->mask[l].p, w->da.p, w->dpq.p, part);
         wgrad<2 * H, H, false>(gs, w->dpq.p, 2 * H, 2 * H, nullptr, 0, w->cat[l].p, 2 * H, H, N, g + y.A[l], nullptr, st);
