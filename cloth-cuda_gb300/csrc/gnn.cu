@@ -196,7 +196,6 @@ int backward(pdg_warmstart* w, float inv_cnt, const float* ew, cudaStream_t st)
 {
     const int N = w->N;
     const Layout& y = w->lay;
-    const float* p = w->p.p;
     float* g = w->g.p;
     GK(w->part.reserve(part_floats(N)));   // (grows only with the graph, whose upload waits for earlier passes)
     GradSums gs(w->part.p);

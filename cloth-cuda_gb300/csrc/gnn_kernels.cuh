@@ -62,8 +62,7 @@ void launch_after(void (*kern)(P...), int grid, int block, size_t smem, cudaStre
     cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
-enum { EPI_RELU = 1, EPI_STORE1 = 2, EPI_RESID2 = 4, EPI_STOREF = 8, EPI_ACCF = 16, EPI_RESIDA = 32,
-       EPI_MASKA = 64, EPI_SPLIT = 128 };
+enum { EPI_RELU = 1, EPI_STORE1 = 2, EPI_STOREF = 4, EPI_ACCF = 8, EPI_RESIDA = 16, EPI_MASKA = 32, EPI_SPLIT = 64 };
 
 __device__ __forceinline__ uint32_t ld_pair(const bf16* p) { return *reinterpret_cast<const uint32_t*>(p); }
 __device__ __forceinline__ uint32_t ld_pair(const float* p)
@@ -97,8 +96,8 @@ __device__ __forceinline__ void mma_bf16(float* c, uint32_t a0, uint32_t a1, uin
 // loads are bank-conflict free) and the bias in shared memory once, in
 // 16-byte pieces, and its warps then walk 16-row tiles with a grid stride
 // (gemm_grid sizes the grid to the resident blocks).
-// Epilogue: optional ReLU; Y1 <- bf16(v); Y2 <- bf16(R + v) (R read, or taken
-// from the A fragments when it is X's first NOUT columns); Yf <- v or += v.
+// Epilogue: optional ReLU; Y1 <- bf16(v); Y2 <- bf16(r + v), r X's first NOUT
+// columns, taken from the A fragments; Yf <- v or += v.
 // The backward pass also has EPI_MASKA: X (fp32) counts as zero where R
 // [M][K] is not positive, and EPI_SPLIT (K = NOUT / 2): Yf <- X + v for the
 // first K columns of v, Yg <- v rs[row] for the others.
@@ -184,16 +183,11 @@ __global__ void __launch_bounds__(128) k_gemm(const TA* X, int ldx, int M, const
                 if (EPI & EPI_RELU) { v0 = fmaxf(v0, 0.f); v1 = fmaxf(v1, 0.f); }
                 if (EPI & EPI_STORE1)
                     *reinterpret_cast<__nv_bfloat162*>(Y1 + (size_t)row * ld1 + col) = __floats2bfloat162_rn(v0, v1);
-                if (EPI & (EPI_RESID2 | EPI_RESIDA)) {
-                    // EPI_RESIDA: the residual is the A operand's first NOUT
-                    // columns, already in this thread's fragments
-                    __nv_bfloat162 r;
-                    if (EPI & EPI_RESIDA) {
-                        const uint32_t u = a[n >> 1][(n & 1) * 2 + hf];
-                        r = *reinterpret_cast<const __nv_bfloat162*>(&u);
-                    } else {
-                        r = *reinterpret_cast<const __nv_bfloat162*>(R + (size_t)row * ldr + col);
-                    }
+                if constexpr ((EPI & EPI_RESIDA) != 0) {
+                    // the residual is the A operand's first NOUT columns,
+                    // already in this thread's fragments
+                    const uint32_t u = a[n >> 1][(n & 1) * 2 + hf];
+                    const __nv_bfloat162 r = *reinterpret_cast<const __nv_bfloat162*>(&u);
                     *reinterpret_cast<__nv_bfloat162*>(Y2 + (size_t)row * ld2 + col) =
                         __floats2bfloat162_rn(__bfloat162float(r.x) + v0, __bfloat162float(r.y) + v1);
                 }
@@ -498,9 +492,6 @@ void fused(cudaStream_t st, const bf16* X, int ldx, int M, const bf16* W1, const
     const int grid = resident_grid<k_fused<MODE>>(128, smem, ((((long long)M + 15) >> 4) + 3) / 4);
     launch_after(k_fused<MODE>, grid, 128, smem, st, X, ldx, M, W1, b1, W2, b2, hout, ldh, pq, A, Dp, warm);
 }
-
-__device__ __forceinline__ float tofloat(float v) { return v; }
-__device__ __forceinline__ float tofloat(bf16 v) { return __bfloat162float(v); }
 
 // Per-block partial weight gradients: block b writes
 //   part[b][n*K + k] = sum over its rows of dY[r][n] X[r][k]   (n < nout, k < K)
