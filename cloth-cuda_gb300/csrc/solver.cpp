@@ -296,21 +296,32 @@ long long patch_count(const std::vector<ClothSetup>& cl, int pv)
 
 // Patch size of the streaming plan on 256 threads when the caller leaves it
 // open: 256 vertices, or 192 where these fill the last wave of blocks better.
-// A wave holds 3 blocks per SM.  A 256-vertex patch (335 cells, two rounds of
-// the threads) took about 6.1 us, a 192-vertex one (255 cells, one round) 4.85
-// us; a part-filled last wave counts half of what it leaves empty, because the
-// next sweep's blocks start in it.  The rule picks the measured best on
-// 300x300 (256: 8.1 against 9.1 us per sweep), 333x500 (192: 11.7 against
-// 13.6), 400x400 (192: 12.2 against 13.6), 700x700 (256: 27.8 against 30.6),
-// 1025x1025 (256: 55.0 against 58.8) and a batch of 96 cloths (256: 30.7
-// against 34.4); 513x513 keeps 256 (17.6 against 17.2).
+// A wave holds 3 blocks per SM.  A sweep takes 2.25 us and per wave 5.75 us with
+// 256-vertex patches (335 cells, two rounds of the threads), 4.75 us with 192
+// (255 cells, one round).  A last wave with the share f of its blocks counts
+// 1.6 f of one and, because so few blocks have little to overlap their waits
+// with, up to half a wave more: the less, the more full ones (n) came before it,
+// whose blocks end at different times.  On 80 sheets and batches of 80,000 to
+// 1.2 million vertices that is within 8 % of the measured time, but for a part
+// wave after a single full one, which takes 0.45 + 1.6 f on sheets and longer on
+// uneven batches; with 0.65, 192 is 3 to 5 % slower than 256 on sheets of 349 to
+// 360 vertices a side and 5 to 9 % faster on 20 and 22 cloths of 17 to 129.
+// 192 is taken where it comes out faster by more than 1.5 % (us per sweep):
+// 333x500 (11.7 against 13.5), 400x400 (12.0 against 13.5), 500x500 (16.3
+// against 16.5), 24 cloths of 139,131 vertices (11.7 against 12.9); 256 on
+// 485x485 (15.05 against 16.2), 640x640 (25.2 against 25.7), 769x769 (31.9
+// against 35.8), 96 cloths of 590,807 vertices (32.6 against 34.4), 1025x1025
+// (54.9 against 58.5).  (Half of what the last wave leaves empty, however many
+// full ones came before, took 192 on 768x768: 37.0 against 32.0.)
 int stream_patch_verts(const std::vector<ClothSetup>& cl, int nsm)
 {
-    auto cost = [&](int pv, double us) {
-        const double w = (double)patch_count(cl, pv) / (3.0 * nsm);
-        return us * (w <= 1.0 ? 1.0 : 0.5 * (std::ceil(w) + w));
+    auto sweep = [&](int pv, double wave) {
+        const double w = (double)patch_count(cl, pv) / (3.0 * nsm), n = std::floor(w), f = w - n;
+        if (w <= 1.0) return 2.25 + wave;
+        const double alone = n < 2.0 ? 0.65 : std::max(0.0, 0.5 - 0.08 * n);
+        return 2.25 + wave * (n + (f > 0.0 ? std::min(1.0, alone + 1.6 * f) : 0.0));
     };
-    return cost(192, 4.85) < cost(256, 6.1) ? 192 : 256;
+    return sweep(192, 4.75) < 0.985 * sweep(256, 5.75) ? 192 : 256;
 }
 
 // Smallest patch size (first, first + step, ... most) with at most `blocks`
