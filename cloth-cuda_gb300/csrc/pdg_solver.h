@@ -45,8 +45,9 @@ struct HostLayout {
     std::vector<int> nbr_ptr, nbr;  // patches owning each patch's halo vertices
 };
 
-// layout.cpp: perm_global of build_layout alone
-void vertex_order(const std::vector<ClothSetup>& cl, int patch_verts, std::vector<int>& perm_global);
+// layout.cpp
+// perm_global of the layout in patches of patch_verts, from one in patches of any size
+void vertex_order(const std::vector<ClothSetup>& cl, const HostLayout& L, int patch_verts, std::vector<int>& perm_global);
 bool build_layout(const std::vector<ClothSetup>& cl, int patch_verts, HostLayout& L, std::string& err);
 // The properties the sweep kernels rely on (partition, halo, neighbour lists,
 // boundary-first order, each contribution slot written once, every incident

@@ -410,7 +410,7 @@ namespace pdg {
 const std::vector<int>& usual_order(pdg_solver* s)
 {
     if (!s->open_verts) return s->L.perm_global;
-    if (s->usual.empty()) vertex_order(s->cloths, s->open_verts, s->usual);
+    if (s->usual.empty()) vertex_order(s->cloths, s->L, s->open_verts, s->usual);
     return s->usual;
 }
 
