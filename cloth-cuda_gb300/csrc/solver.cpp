@@ -306,13 +306,14 @@ long long patch_count(const std::vector<ClothSetup>& cl, int pv)
 // wave after a single full one, which takes 0.45 + 1.6 f on sheets and longer on
 // uneven batches; with 0.65, 192 is 3 to 5 % slower than 256 on sheets of 349 to
 // 360 vertices a side and 5 to 9 % faster on 20 and 22 cloths of 17 to 129.
-// 192 is taken where it comes out faster by more than 1.5 % (us per sweep):
+// 192 is taken where it comes out faster by more than 2 % (us per sweep):
 // 333x500 (11.7 against 13.5), 400x400 (12.0 against 13.5), 500x500 (16.3
 // against 16.5), 24 cloths of 139,131 vertices (11.7 against 12.9); 256 on
-// 485x485 (15.05 against 16.2), 640x640 (25.2 against 25.7), 769x769 (31.9
-// against 35.8), 96 cloths of 590,807 vertices (32.6 against 34.4), 1025x1025
-// (54.9 against 58.5).  (Half of what the last wave leaves empty, however many
-// full ones came before, took 192 on 768x768: 37.0 against 32.0.)
+// 485x485 (15.05 against 16.2), 513x513 (17.4 against 17.0), 640x640 (25.2
+// against 25.7), 769x769 (31.9 against 35.8), 96 cloths of 590,807 vertices
+// (32.6 against 34.4), 1025x1025 (54.9 against 58.5).  (Half of what the last
+// wave leaves empty, however many full ones came before, took 192 on 768x768:
+// 37.0 against 32.0.)
 int stream_patch_verts(const std::vector<ClothSetup>& cl, int nsm)
 {
     auto sweep = [&](int pv, double wave) {
@@ -321,7 +322,7 @@ int stream_patch_verts(const std::vector<ClothSetup>& cl, int nsm)
         const double alone = n < 2.0 ? 0.65 : std::max(0.0, 0.5 - 0.08 * n);
         return 2.25 + wave * (n + (f > 0.0 ? std::min(1.0, alone + 1.6 * f) : 0.0));
     };
-    return sweep(192, 4.75) < 0.985 * sweep(256, 5.75) ? 192 : 256;
+    return sweep(192, 4.75) < 0.98 * sweep(256, 5.75) ? 192 : 256;
 }
 
 // Smallest patch size (first, first + step, ... most) with at most `blocks`
