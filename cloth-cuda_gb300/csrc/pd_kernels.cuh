@@ -18,9 +18,9 @@ __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b)
 __device__ __forceinline__ float fsub(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ float ffma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdiv_rn(a, b); }
-// Reciprocal square root of a normal number: one instruction.  rsqrtf also
-// handles subnormal inputs (four instructions, the same bits for normal ones);
-// every caller's argument is bounded below by 1e-30.
+// Reciprocal square root of a normal number: one PTX instruction.  rsqrtf also
+// handles subnormal inputs; every caller's argument is bounded below by 1e-30
+// (the iterates are bitwise those with rsqrtf).
 __device__ __forceinline__ float frsqrt(float a)
 {
     float r;

@@ -70,8 +70,8 @@ extern "C" {
                                     run in one cooperative launch instead.
                                     patch_verts and block_threads 0: patches
                                     small enough for that where two per SM
-                                    are, else 192 or 256 vertices, whichever
-                                    fills the last wave of blocks better     */
+                                    are, else 192 or 256 vertices, by the
+                                    time that their waves of blocks take     */
 
 /* Solver configuration.  Mirrors PDSolverConfig (include/pd_solver.h:4-15);
  * fields after `damping` extend it. */
